@@ -835,22 +835,22 @@ int upload_operators(rtfmm_fmm* f) {
     cudaError_t e = cudaMemcpy(stage, o.cc8.data(), sizeof(double) * o.cc8.size(), cudaMemcpyHostToDevice);
     if (f->m2l32) {
       float* gp = nullptr;
-      int rc = dalloc(f, &gp, o.cc8.size(), &f->d_G8);
+      int rc = dalloc(f, &gp, g8_layout_size(Nf, f->m2l32), &f->d_G8);
       if (rc) {
         cudaFree(stage);
         return rc;
       }
       f->d_G8 = gp;
-      if (e == cudaSuccess) e = launch_g8_layout<float>(stage, Nf, gp, f->s0);
+      if (e == cudaSuccess) e = launch_g8_layout(stage, Nf, gp, f->s0);
     } else {
       double* gp = nullptr;
-      int rc = dalloc(f, &gp, o.cc8.size(), &f->d_G8);
+      int rc = dalloc(f, &gp, g8_layout_size(Nf, f->m2l32), &f->d_G8);
       if (rc) {
         cudaFree(stage);
         return rc;
       }
       f->d_G8 = gp;
-      if (e == cudaSuccess) e = launch_g8_layout<double>(stage, Nf, gp, f->s0);
+      if (e == cudaSuccess) e = launch_g8_layout(stage, Nf, gp, f->s0);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(f->s0);
     cudaFree(stage);
@@ -1133,10 +1133,10 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
     f->launches += (nup8 > 0) + (nup27 > 0);
     CK(cudaEventRecord(f->ev_st[ST_UP], s0));
     if (f->m2l32) {
-      CK(launch_m2l_hadamard8<float>((const float*)f->d_Q8, (const float*)f->d_G8, f->d_tsrc8, f->nT8, f->nS8,
+      CK(launch_m2l_hadamard8((const float*)f->d_Q8, (const float*)f->d_G8, f->d_tsrc8, f->nT8, f->nS8,
                                      Nf, (float*)f->d_Pk8, s0));
     } else {
-      CK(launch_m2l_hadamard8<double>((const double*)f->d_Q8, (const double*)f->d_G8, f->d_tsrc8, f->nT8,
+      CK(launch_m2l_hadamard8((const double*)f->d_Q8, (const double*)f->d_G8, f->d_tsrc8, f->nT8,
                                       f->nS8, Nf, (double*)f->d_Pk8, s0));
     }
     CK(launch_m2l_hadamard27(f->d_Q27, f->d_G27, f->d_tsrc27, f->nT27, f->nS27, Nf, f->d_Pk27, s0));

@@ -1401,10 +1401,6 @@ template <> struct HadCfg<float> {
   static constexpr int TT = HAD_TT, DF = HAD_DF, THREADS = 256 / HAD_TT, MINB = HAD_MINB;
   static constexpr bool ACC_SMEM = HAD_ACC_SMEM;
 };
-template <> struct HadCfg<double> {
-  static constexpr int TT = 1, DF = 1, THREADS = 256, MINB = 1;
-  static constexpr bool ACC_SMEM = false;
-};
 
 template <typename T>
 __device__ __forceinline__ void load_row8(const T* qrow, typename Cplx<T>::type (&q)[8]) {
@@ -1640,18 +1636,166 @@ __global__ void __launch_bounds__(HadCfg<T>::THREADS, HadCfg<T>::MINB)
   }
 }
 
+// ---------------------------------------------------------------------------
+// Hadamard 8x8 in FP64, on the FP64 tensor path.
+//
+// The 8x8 block of a direction depends on a child pair only through its
+// offset, so along x it is a 2x2 Toeplitz matrix of 4x4 blocks (a on the
+// diagonal, b for source x = 1 and target x = 0, c for the converse), and
+//   y0 = a (x0 + x1) + (b - a) x1,   y1 = a (x0 + x1) + (c - a) x0
+// takes three 4x4 products instead of four.  The sum over the directions is
+// linear, so the three products are accumulated on their own and combined
+// once at the end.  Each is a real 8x8 matrix (4 complex slots) applied to 8
+// targets: two mma.sync.m8n8k4 (real parts, then imaginary parts of the four
+// source slots).  Against the product in full this does 192 instead of 256
+// multiply-adds per (target, direction, frequency), and a coefficient read
+// feeds 32 targets instead of one, which is what bounded the FP64 form on the
+// FMA pipe (every multiply-add waited for its share of a shared-memory
+// broadcast).  The rounding error of the spectra against 80-bit sums is
+// 0.6-1.1 times that of the full product (P = 4-10).
+//
+// A block takes one frequency and 96 targets, a warp 24 of them as three
+// tiles of 8; lane 4 r + q holds source slot q (and q + 4) of target row r.
+// A tile none of whose targets has a source in a direction skips it.
+// Three tiles a warp leave room for four blocks an SM (128 registers): 1.79 ms
+// at N = 2^20, P = 8, ncrit = 256 against 1.87 with four tiles and three
+// blocks and 1.97 with two and five; 3.58 ms for the product in full on the
+// FMA pipe.  The FP64 tensor pipe is 70% busy (27 of DGEMM's 35 TFLOP/s,
+// counting the 40% of the (target, direction) slots that are empty there).
+// ---------------------------------------------------------------------------
+constexpr int kHad64Tiles = 3, kHad64Threads = 128, kHad64Blocks = 4;
+
+// Coefficients of a frequency: [direction][product][source slot][target slot]
+constexpr int kG64PerDir = 3 * 16;
+
+__device__ __forceinline__ double2 ld_nc_f64x2(const double* p) {
+  double2 v;
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+
+__global__ void __launch_bounds__(kHad64Threads, kHad64Blocks)
+    k_m2l_hadamard8_f64(const double* __restrict__ Q, const double2* __restrict__ G, const int* __restrict__ tsrcT,
+                        int ntar, int nsrc, double* __restrict__ Pk) {
+  constexpr int MT = kHad64Tiles;
+  // B fragments of both mma of a product, per lane
+  __shared__ __align__(16) double2 Bs[26 * 3 * 32];
+  const int f = blockIdx.y;
+  const double2* Gf = G + (size_t)f * 26 * kG64PerDir;
+  for (int e = threadIdx.x; e < 26 * 3 * 32; e += kHad64Threads) {
+    // lane 8 t + 4 c + s: source slot s, column 2 t + c (part c of target slot t)
+    const double2 g = Gf[(e >> 5) * 16 + (e & 3) * 4 + ((e >> 3) & 3)];
+    Bs[e] = e & 4 ? make_double2(g.y, g.x) : make_double2(g.x, -g.y);
+  }
+  const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+  const int t0 = blockIdx.x * (8 * MT * (kHad64Threads / 32)) + (threadIdx.x >> 5) * (8 * MT) + r;
+  // slot q of the x = 0 children; the x = 1 children are two chunks on
+  const double* q0 = Q + ((size_t)f * 4 + (q >> 1)) * nsrc * 4 + (q & 1) * 2;
+  const double* q1 = q0 + (size_t)nsrc * 8;
+  auto index = [&](int d, int (&sd)[MT]) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const int t = t0 + 8 * m;
+      sd[m] = t < ntar ? tsrcT[d * ntar + t] : -1;
+    }
+  };
+  auto rows = [&](const int (&sd)[MT], double2 (&x0)[MT], double2 (&x1)[MT]) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      x0[m] = x1[m] = make_double2(0.0, 0.0);
+      if (sd[m] >= 0) {
+        x0[m] = ld_nc_f64x2(q0 + (size_t)sd[m] * 4);
+        x1[m] = ld_nc_f64x2(q1 + (size_t)sd[m] * 4);
+      }
+    }
+  };
+  double acc[3][MT][2];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int m = 0; m < MT; ++m) acc[k][m][0] = acc[k][m][1] = 0.0;
+  auto mac = [&](int d, const int (&sd)[MT], const double2 (&x0)[MT], const double2 (&x1)[MT]) {
+    const double2 b0 = Bs[(3 * d + 0) * 32 + lane], b1 = Bs[(3 * d + 1) * 32 + lane], b2 = Bs[(3 * d + 2) * 32 + lane];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      if (!__any_sync(0xffffffffu, sd[m] >= 0)) continue;
+      const double sr = x0[m].x + x1[m].x, si = x0[m].y + x1[m].y;
+      dmma8x8x4(acc[0][m], x1[m].x, b0.x);
+      dmma8x8x4(acc[1][m], sr, b1.x);
+      dmma8x8x4(acc[2][m], x0[m].x, b2.x);
+      dmma8x8x4(acc[0][m], x1[m].y, b0.y);
+      dmma8x8x4(acc[1][m], si, b1.y);
+      dmma8x8x4(acc[2][m], x0[m].y, b2.y);
+    }
+  };
+  // two-stage pipeline over the directions: the source rows of direction d+1
+  // are in flight while direction d is multiplied, the row indices run one
+  // direction further ahead
+  int ia[MT], ib[MT];
+  double2 xa0[MT], xa1[MT], xb0[MT], xb1[MT];
+  index(0, ia);
+  rows(ia, xa0, xa1);
+  index(1, ib);
+  __syncthreads();
+  if (t0 - r >= ntar) return;  // warp-uniform
+#pragma unroll 1
+  for (int d = 0; d < 26; d += 2) {
+    int ja[MT], jb[MT];
+    rows(ib, xb0, xb1);
+    if (d + 2 < 26) index(d + 2, ja);
+    mac(d, ia, xa0, xa1);
+    if (d + 2 < 26) {
+      rows(ja, xa0, xa1);
+      index(d + 3, jb);
+    }
+    mac(d + 1, ib, xb0, xb1);
+    if (d + 2 < 26) {
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        ia[m] = ja[m];
+        ib[m] = jb[m];
+      }
+    }
+  }
+  // accumulator columns 2 q, 2 q + 1: target slot q, real and imaginary part
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    const int t = t0 + 8 * m;
+    if (t >= ntar) break;
+    double2* out = reinterpret_cast<double2*>(Pk) + ((size_t)f * ntar + t) * 8 + q;
+    out[0] = make_double2(acc[1][m][0] + acc[0][m][0], acc[1][m][1] + acc[0][m][1]);
+    out[4] = make_double2(acc[1][m][0] + acc[2][m][0], acc[1][m][1] + acc[2][m][1]);
+  }
+}
+
 // The 8x8 kernel spectra re-laid frequency-major for the Hadamard:
-// G[(f * 26 + d) * 64 + pair] = cc8[(d * 64 + pair) * Nf + f] (complex), in the
-// pass's precision (FP32 by round to nearest).
-template <typename T>
-__global__ void k_g8_layout(const double2* __restrict__ cc8, int Nf, T* __restrict__ G) {
+// G[(f * 26 + d) * 64 + pair] = cc8[(d * 64 + pair) * Nf + f] (complex), in
+// FP32 by round to nearest.
+__global__ void k_g8_layout(const double2* __restrict__ cc8, int Nf, float2* __restrict__ G) {
   const size_t total = (size_t)26 * 64 * Nf;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
     const int pr = (int)(e % 64), d = (int)((e / 64) % 26);
     const size_t f = e / (64 * 26);
     const double2 v = cc8[((size_t)d * 64 + pr) * Nf + f];
-    G[2 * e] = (T)v.x;
-    G[2 * e + 1] = (T)v.y;
+    G[e] = make_float2((float)v.x, (float)v.y);
+  }
+}
+
+// The same for the FP64 form: the coefficients of its three products,
+// G[((f * 26 + d) * 3 + k) * 16 + 4 s + t] = b - a, a, c - a (k = 0, 1, 2) of
+// source slot s and target slot t (y and z octant bits).
+__global__ void k_g8_layout64(const double2* __restrict__ cc8, int Nf, double2* __restrict__ G) {
+  const size_t total = (size_t)26 * kG64PerDir * Nf;
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+    const int t = (int)(e % 4), s = (int)(e / 4 % 4), k = (int)(e / 16 % 3), d = (int)(e / 48 % 26);
+    const size_t f = e / (48 * 26);
+    auto at = [&](int isrc, int itar) { return cc8[((size_t)d * 64 + isrc * 8 + itar) * Nf + f]; };
+    double2 v = at(s, t);
+    if (k != 1) {
+      const double2 o = k == 0 ? at(s + 4, t) : at(s, t + 4);
+      v = make_double2(o.x - v.x, o.y - v.y);
+    }
+    G[e] = v;
   }
 }
 
@@ -2085,27 +2229,43 @@ cudaError_t launch_m2l_up(const double* q_equiv, const int* items, int nitems, c
   }
 }
 
-template <typename T>
-cudaError_t launch_m2l_hadamard8(const T* Q, const T* G, const int* tsrcT, int ntar, int nsrc, int Nf, T* Pk,
-                                 cudaStream_t st) {
+cudaError_t launch_m2l_hadamard8(const float* Q, const float* G, const int* tsrcT, int ntar, int nsrc, int Nf,
+                                 float* Pk, cudaStream_t st) {
   if (ntar > 0) {
-    constexpr int NT = HadCfg<T>::THREADS, TT = HadCfg<T>::TT;
+    constexpr int NT = HadCfg<float>::THREADS, TT = HadCfg<float>::TT;
     dim3 grid(cdiv(ntar, NT * TT), Nf);
-    k_m2l_hadamard8<T><<<grid, NT, 0, st>>>(Q, G, tsrcT, ntar, nsrc, Nf, Pk);
+    k_m2l_hadamard8<float><<<grid, NT, 0, st>>>(Q, G, tsrcT, ntar, nsrc, Nf, Pk);
   }
   return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_g8_layout(const double* cc8, int Nf, T* G, cudaStream_t st) {
-  const size_t total = (size_t)26 * 64 * Nf;
-  if (total > 0)
-    k_g8_layout<T><<<(int)std::min<size_t>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
-        reinterpret_cast<const double2*>(cc8), Nf, G);
+cudaError_t launch_m2l_hadamard8(const double* Q, const double* G, const int* tsrcT, int ntar, int nsrc, int Nf,
+                                 double* Pk, cudaStream_t st) {
+  if (ntar > 0) {
+    dim3 grid(cdiv(ntar, 8 * kHad64Tiles * (kHad64Threads / 32)), Nf);
+    k_m2l_hadamard8_f64<<<grid, kHad64Threads, 0, st>>>(Q, reinterpret_cast<const double2*>(G), tsrcT, ntar, nsrc,
+                                                        Pk);
+  }
   return cudaGetLastError();
 }
-template cudaError_t launch_g8_layout<float>(const double*, int, float*, cudaStream_t);
-template cudaError_t launch_g8_layout<double>(const double*, int, double*, cudaStream_t);
+
+size_t g8_layout_size(int Nf, bool fp32) { return (size_t)26 * (fp32 ? 64 : kG64PerDir) * Nf * 2; }
+
+cudaError_t launch_g8_layout(const double* cc8, int Nf, float* G, cudaStream_t st) {
+  const size_t total = (size_t)26 * 64 * Nf;
+  if (total > 0)
+    k_g8_layout<<<(int)std::min<size_t>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
+        reinterpret_cast<const double2*>(cc8), Nf, reinterpret_cast<float2*>(G));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_g8_layout(const double* cc8, int Nf, double* G, cudaStream_t st) {
+  const size_t total = (size_t)26 * kG64PerDir * Nf;
+  if (total > 0)
+    k_g8_layout64<<<(int)std::min<size_t>((total + 255) / 256, 148 * 16), 256, 0, st>>>(
+        reinterpret_cast<const double2*>(cc8), Nf, reinterpret_cast<double2*>(G));
+  return cudaGetLastError();
+}
 
 cudaError_t launch_body_leaf(const LeafInfo* leaves, int nleaf, int n, int* body_leaf, cudaStream_t st) {
   if (nleaf > 0) k_body_leaf<<<nleaf, 128, 0, st>>>(leaves, nleaf, n, body_leaf);
@@ -2224,10 +2384,6 @@ template cudaError_t launch_m2l_up<float>(const double*, const int*, int, const 
                                           int, int, float*, cudaStream_t);
 template cudaError_t launch_m2l_up<double>(const double*, const int*, int, const int*, const double*, int, int,
                                            int, int, double*, cudaStream_t);
-template cudaError_t launch_m2l_hadamard8<float>(const float*, const float*, const int*, int, int, int, float*,
-                                                 cudaStream_t);
-template cudaError_t launch_m2l_hadamard8<double>(const double*, const double*, const int*, int, int, int,
-                                                  double*, cudaStream_t);
 template cudaError_t launch_m2l_down<float>(const float*, const int*, const double*, int, const int*,
                                             const double*, int, int, int, int, double*, cudaStream_t);
 template cudaError_t launch_m2l_down<double>(const double*, const int*, const double*, int, const int*,

@@ -89,8 +89,8 @@ cudaError_t launch_apply(const ApplyBatch& b, cudaStream_t st);
 // (parent, coff, cnum) triplets
 cudaError_t launch_sum_children(const int* list, int nparents, const double* Y, int ns, double* q,
                                 cudaStream_t st);
-// FFT-M2L spectra are frequency-major: Q[f][src][slot], Pk[f][tar][slot],
-// G[f][d][isrc*8+itar] (complex, interleaved re/im).
+// FFT-M2L spectra are frequency-major: Q[f][src][slot], Pk[f][tar][slot]
+// (complex, interleaved re/im).
 // items hold 10 ints per block: parent, first slot, child cell of each of the
 // sp slots of the group (-1 = absent); sp from m2l_up_slots / m2l_down_slots.
 template <typename T>
@@ -100,12 +100,15 @@ int m2l_down_slots(int P);
 template <typename T>
 cudaError_t launch_m2l_up(const double* q_equiv, const int* items, int nitems, const int* surf_ijk,
                           const double* twiddle, int P, int ns, int nsrc, int sp, T* Q, cudaStream_t st);
-template <typename T>
-cudaError_t launch_m2l_hadamard8(const T* Q, const T* G, const int* tsrcT /*[26][ntar]*/, int ntar, int nsrc,
-                                 int Nf, T* Pk, cudaStream_t st);
-// G (frequency-major, the Hadamard's layout) from cc8 [d][pair][f] (device)
-template <typename T>
-cudaError_t launch_g8_layout(const double* cc8, int Nf, T* G, cudaStream_t st);
+cudaError_t launch_m2l_hadamard8(const float* Q, const float* G, const int* tsrcT /*[26][ntar]*/, int ntar, int nsrc,
+                                 int Nf, float* Pk, cudaStream_t st);
+cudaError_t launch_m2l_hadamard8(const double* Q, const double* G, const int* tsrcT, int ntar, int nsrc, int Nf,
+                                 double* Pk, cudaStream_t st);
+// G (frequency-major, the layout of that precision's Hadamard, g8_layout_size
+// values) from cc8 [d][pair][f] (device)
+size_t g8_layout_size(int Nf, bool fp32);
+cudaError_t launch_g8_layout(const double* cc8, int Nf, float* G, cudaStream_t st);
+cudaError_t launch_g8_layout(const double* cc8, int Nf, double* G, cudaStream_t st);
 cudaError_t launch_m2l_hadamard27(const double* Q, const double* G27 /*[d][f]*/, const int* tsrc /*[ntar][26]*/,
                                   int ntar, int nsrc, int Nf, double* Pk, cudaStream_t st);
 template <typename T>

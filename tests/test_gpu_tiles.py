@@ -1,0 +1,50 @@
+"""The pass at the edges of its kernels' tiles, against the oracle and the
+host build.
+
+Tolerances are those of the parity tests: FP64 1e-9 on the gradient (1e-7
+from P = 9, where the equivalent densities are as ill-conditioned as FP64
+holds and two FP64 implementations agree to that), FP32-mixed 1e-5.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def uniform01(n, seed):
+    rng = np.random.default_rng(seed)
+    x = rng.random((n, 3))
+    q = rng.random(n) * 2 - 1
+    return x, q - q.mean()
+
+
+def l2(a, b):
+    return float(np.linalg.norm(np.asarray(a) - np.asarray(b)) / np.linalg.norm(np.asarray(b)))
+
+
+def args(pkg, P, ncrit, images, precision, stages=None):
+    return pkg.Argument(P=P, ncrit=ncrit, images=images, cycle=1.0, x=(0.5, 0.5, 0.5), dipole_correction=0,
+                        divide_4pi=1, precision=precision, stages=pkg.STAGE_ALL if stages is None else stages)
+
+
+# far field at every order with its own transform kernels and at two without
+# (2, 11), with 9 and with 73 target parents (the Hadamard's tiles hold 8, 24
+# and 96), periodic and free
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("P,n,ncrit,images", [(2, 900, 24, 1), (4, 900, 24, 2), (5, 700, 12, 0), (6, 2500, 8, 1),
+                                              (7, 900, 24, 3), (8, 900, 24, 0), (9, 900, 24, 2), (10, 2500, 8, 1),
+                                              (11, 600, 24, 1)])
+def test_far_field_at_every_order(pkg, oracle, P, n, ncrit, images, precision):
+    x, q = uniform01(n, 100 + P)
+    # from P = 9 the two pseudo-inverses (two SVDs, cut at 4e-16) differ by up
+    # to 1e-7 of the whole field, of which the far part is a tenth here
+    stages = "far" if P < 9 else "all"
+    f = pkg.LaplaceFMM(x, q, args(pkg, P, ncrit, images, precision, pkg.STAGE_FAR if P < 9 else pkg.STAGE_ALL))
+    phi, grad = f.solve()
+    f.close()
+    rphi, rgrad = oracle.FMM(x, q, P, ncrit, images, 1.0, center=(0.5, 0.5, 0.5), divide_4pi=1).solve(stages=stages)
+    tol = 1e-5 if precision else 1e-9 if P < 9 else 1e-7
+    assert l2(grad, rgrad) < tol
+    assert l2(phi - phi.mean(), rphi - rphi.mean()) < max(tol, 1e-8)

@@ -132,6 +132,29 @@ def test_kernel_spectra_match_oracle(pkg, oracle, P):
     assert np.abs(got - ref).max() / scale < 1e-13
 
 
+@pytest.mark.parametrize("P", [4, 7])
+def test_m2l_blocks_are_toeplitz(pkg, P):
+    """The 8x8 block of a direction depends on a child pair through its offset
+    only, so that each direction takes three 4x4 products along x instead of
+    four: a (x0 + x1) + (b - a) x1 and a (x0 + x1) + (c - a) x0."""
+    x, q = uniform(100, 1)
+    f = pkg.LaplaceFMM(x, q, pkg.Argument(P=P, ncrit=10, images=2, cycle=1.0))
+    f.setup()
+    Nf = (2 * P - 1) ** 2 * P
+    g = f.operator(3, 26 * 64 * Nf * 2).reshape(26, 2, 4, 2, 4, Nf, 2)
+    g = g[..., 0] + 1j * g[..., 1]  # direction, source x, source yz, target x, target yz
+    assert np.array_equal(g[:, 0, :, 0], g[:, 1, :, 1])
+    rng = np.random.default_rng(2)
+    v = rng.standard_normal((2, 4, Nf)) + 1j * rng.standard_normal((2, 4, Nf))
+    a, b, c = g[:, 0, :, 0], g[:, 1, :, 0], g[:, 0, :, 1]
+    mul = lambda m, u: np.einsum("dstf,sf->dtf", m, u)  # noqa: E731
+    mid = mul(a, v[0] + v[1])
+    want = np.einsum("dxsytf,xsf->dytf", g, v)
+    got = np.stack([mid + mul(b - a, v[1]), mid + mul(c - a, v[0])], 1)
+    assert np.abs(got - want).max() <= 1e-14 * np.abs(want).max() * 8  # eight terms of rounding 1e-16
+    f.close()
+
+
 @pytest.mark.parametrize("P", [4, 6, 8, 10])
 def test_m2m_reproduces_child_potential(pkg, oracle, P):
     """The parent equivalent density from M2M reproduces the child's field on
