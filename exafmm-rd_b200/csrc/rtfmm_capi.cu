@@ -106,9 +106,10 @@ struct rtfmm_fmm {
   // host plan tables
   std::vector<LeafInfo> leaves;
   std::vector<int> body_leaf;
-  std::vector<P2PItem32> items2; // P2P work items (target groups), both precisions
+  std::vector<P2PItem> items2;    // P2P work items (target groups x list parts), both precisions
   std::vector<int> list_off;
   int n_items2 = 0;               // work items (host or device built)
+  int n_slots = 0;                // slots of the items whose list is cut into parts
   int64_t p2p_pairs = 0;          // body pairs of the P2P lists
   // the P2P lists, offsets and items were built on the GPU (device set-up):
   // the host vectors above are empty
@@ -160,7 +161,9 @@ struct rtfmm_fmm {
   double *d_qeq = nullptr, *d_pchk = nullptr, *d_leafvec = nullptr, *d_leafvec2 = nullptr, *d_y = nullptr;
   double *d_far_phi = nullptr, *d_far_grad = nullptr, *d_near_phi = nullptr, *d_near_grad = nullptr;
   double *d_out_phi = nullptr, *d_out_grad = nullptr;
-  P2PItem32* d_items2 = nullptr;
+  P2PItem* d_items2 = nullptr;
+  double4* d_part = nullptr;  // sums of a list part: 32 per slot
+  int* d_part_done = nullptr;
   int* d_list_off = nullptr;
   P2PSrc32* d_list32 = nullptr;
   P2PSrc64* d_list64 = nullptr;
@@ -446,8 +449,9 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
     return k;
   };
   f->list_off.assign(nlf + 1, 0);
-  std::vector<int> item_off(nlf + 1, 0);
-#pragma omp parallel for schedule(dynamic, 64)
+  std::vector<int> item_off(nlf + 1, 0), bodies(nlf, 0);
+  unsigned long long work = 0;
+#pragma omp parallel for schedule(dynamic, 64) reduction(+ : work)
   for (int l = 0; l < nlf; ++l) {
     int path[kMaxPath];
     const int np = path_lists(f->leaves[l].cell, path);
@@ -457,19 +461,26 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
         int lo, hi;
         leaf_run(e.src, &lo, &hi);
         cnt += hi - lo;
+        bodies[l] += p.cells[e.src].bnum;
       }
     f->list_off[l + 1] = (int)cnt;
-    item_off[l + 1] = (f->leaves[l].bnum + 31) / 32;
+    work += (unsigned long long)bodies[l] * ((f->leaves[l].bnum + 31) / 32);
   }
+  // long lists are cut into parts of about `part` bodies
+  const int part = p2p_part_bodies(work);
+  std::vector<int> slot_off(nlf + 1, 0);
   for (int l = 0; l < nlf; ++l) {
+    const int groups = (f->leaves[l].bnum + 31) / 32, nparts = std::max(1, (bodies[l] + part - 1) / part);
     f->list_off[l + 1] += f->list_off[l];
-    item_off[l + 1] += item_off[l];
+    item_off[l + 1] = item_off[l] + groups * nparts;
+    slot_off[l + 1] = slot_off[l] + (nparts > 1 ? groups * nparts : 0);
   }
+  f->n_slots = slot_off[nlf];
   // the list form of the handle's precision only
   const bool mixed = f->args.precision == RTFMM_FP32_MIXED;
   f->list32.assign(mixed ? f->list_off[nlf] : 0, P2PSrc32{});
   f->list64.assign(mixed ? 0 : f->list_off[nlf], P2PSrc64{});
-  f->items2.assign(item_off[nlf], P2PItem32{});
+  f->items2.assign(item_off[nlf], P2PItem{});
   f->n_items2 = item_off[nlf];
   int64_t pairs = 0;
 #pragma omp parallel for schedule(dynamic, 64) reduction(+ : pairs)
@@ -479,12 +490,32 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
     int path[kMaxPath];
     const int np = path_lists(c, path);
     int k = f->list_off[l];
+    // work items: 32 targets each (the last <= 16 targets of a leaf take a
+    // narrower group, W = 16, 8 or 4 lanes, and split the sources 32/W ways)
+    // times the parts of the list: part p starts at the first entry with
+    // p/nparts of the bodies before it
+    const int groups = (T.bnum + 31) / 32, nparts = groups ? (item_off[l + 1] - item_off[l]) / groups : 0;
+    int before = 0, next = 0;  // bodies of the entries so far, parts begun
+    auto begin_parts = [&](int entry, bool end) {
+      for (; next < nparts && (end || before >= (int64_t)next * bodies[l] / nparts); ++next)
+        for (int g = 0; g < groups; ++g) {
+          const int rem = std::min(32, T.bnum - 32 * g);
+          int lw = 5;
+          while (lw > 2 && rem <= (1 << (lw - 1))) --lw;
+          P2PItem* it = &f->items2[item_off[l] + next * groups + g];
+          *it = {l, T.boff + 32 * g, (short)rem, (short)lw, entry, f->list_off[l + 1], next, nparts,
+                 slot_off[l] + g * nparts};
+          if (next > 0) (it - groups)->e1 = entry;
+        }
+    };
     for (int i = 0; i < np; ++i)
       for (const P2PEntry& e : p.p2p.at(path[i])) {
         int lo, hi;
         leaf_run(e.src, &lo, &hi);
         for (int r = lo; r < hi; ++r) {
           const int sl = dfs[r];
+          begin_parts(k, false);
+          before += f->leaves[sl].bnum;
           const Cell& S = p.cells[f->leaves[sl].cell];
           P2PSrc32 a;
           a.dx = (float)(S.x[0] + e.off[0] - T.x[0]);
@@ -512,22 +543,14 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
           ++k;
         }
       }
-    // FP32 items: 32 targets each; the last <= 16 targets of a leaf take a
-    // narrower group (W = 16, 8 or 4 lanes) and split the sources 32/W ways
-    int j = item_off[l];
-    for (int t0 = 0; t0 < f->leaves[l].bnum; t0 += 32, ++j) {
-      const int rem = std::min(32, f->leaves[l].bnum - t0);
-      int lw = 5;
-      while (lw > 2 && rem <= (1 << (lw - 1))) --lw;
-      f->items2[j] = {l, f->leaves[l].boff + t0, rem, lw};
-    }
+    begin_parts(k, true);
   }
   f->p2p_pairs = pairs;
   if (f->shard_n > 1) {  // this rank's targets only
-    std::vector<P2PItem32> mine;
+    std::vector<P2PItem> mine;
     std::vector<char> own(nlf, 0);
     for (int l : f->own_leaves) own[l] = 1;
-    for (const P2PItem32& it : f->items2)
+    for (const P2PItem& it : f->items2)
       if (own[it.leaf]) mine.push_back(it);
     f->items2.swap(mine);
     f->n_items2 = (int)f->items2.size();
@@ -862,6 +885,15 @@ int upload_operators(rtfmm_fmm* f) {
   return RTFMM_OK;
 }
 
+// The slots of the P2P list parts, their counters zero.
+int alloc_parts(rtfmm_fmm* f) {
+  int rc = 0;
+  if ((rc = dalloc(f, &f->d_part, 32 * (size_t)f->n_slots)) || (rc = dalloc(f, &f->d_part_done, (size_t)f->n_slots)))
+    return rc;
+  CK(cudaMemsetAsync(f->d_part_done, 0, sizeof(int) * std::max(1, f->n_slots), f->s0));
+  return RTFMM_OK;
+}
+
 // Upload the plan (everything but the per-pass body values) to the device.
 int upload_plan(rtfmm_fmm* f) {
   const double t0 = wall_s();
@@ -925,6 +957,7 @@ int upload_plan(rtfmm_fmm* f) {
   if (!f->p2p_on_device) {  // else device_p2p_tables writes them
     RC(dupload(f, &f->d_items2, f->items2));
     RC(dupload(f, &f->d_list_off, f->list_off));
+    RC(alloc_parts(f));
     if (mixed)
       RC(dupload(f, &f->d_list32, f->list32));
     else
@@ -1066,7 +1099,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
     }
     CK(cudaEventRecord(f->ev_near0, s1));
     if (mixed) {
-      CK(launch_p2p32(f->d_body32, f->d_items2, f->n_items2, f->d_list_off, f->d_list32,
+      CK(launch_p2p32(f->d_body32, f->d_items2, f->n_items2, f->d_list32, f->d_part, f->d_part_done,
                       f->d_near_phi, f->d_near_grad, s1));
       f->launches += 1;
       if (f->n_close > 0) {
@@ -1075,7 +1108,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
         f->launches += 1;
       }
     } else {
-      CK(launch_p2p64(f->d_body64, f->d_items2, f->n_items2, f->d_list_off, f->d_list64,
+      CK(launch_p2p64(f->d_body64, f->d_items2, f->n_items2, f->d_list64, f->d_part, f->d_part_done,
                       f->d_near_phi, f->d_near_grad, s1));
       f->launches += 1;
     }
@@ -1511,8 +1544,9 @@ int device_tables(rtfmm_fmm* f, const TreeScratchFn& scratch) {
   if (device_p2p_tables(f->dwalk, in, mixed, f->s0, scratch, kTableSlots, alloc, &out, msg) != kTreeOk)
     return fail(RTFMM_ECUDA, msg);
   f->n_items2 = out.nitems;
+  f->n_slots = out.nslots;
   f->p2p_pairs = out.pairs;
-  return RTFMM_OK;
+  return alloc_parts(f);
 }
 
 void begin_setup(rtfmm_fmm* f, int64_t n) {

@@ -39,14 +39,11 @@
 #ifndef P2P_MINB
 #define P2P_MINB 20
 #endif
-#ifndef P2P_PACKED
-#define P2P_PACKED 1
-#endif
 #ifndef P2P_WARPS
 #define P2P_WARPS 1
 #endif
-#ifndef P2P_TILE
-#define P2P_TILE 32
+#ifndef P2P_FLUSH
+#define P2P_FLUSH 4
 #endif
 // register-blocked FFT-M2L up: resident blocks per SM (FP32; FP64 keeps 2)
 #ifndef UP_RB_MINB
@@ -190,36 +187,99 @@ __global__ void k_body_leaf(const LeafInfo* __restrict__ leaves, int nleaf, int 
 }
 
 // ---------------------------------------------------------------------------
-// P2P: one warp per work item (up to 32 targets of one leaf); sources staged
-// 32 at a time in a per-warp shared-memory slot and read as broadcasts, the
-// next tile's bodies and the next list entry loaded while the current tile is
-// computed.  FP32 partial sums per source leaf are accumulated into FP64.
+// P2P: one warp per work item, up to 32 targets of one leaf against a part of
+// the leaf's source list (entries e0..e1).  The bodies of the list's entries
+// are taken as one sequence and staged 32 at a time in a per-warp
+// shared-memory slot, so a tile is full whatever the sizes of the source
+// leaves; the next tile's bodies and the next 32 entries load while the
+// current tile is computed.
+//
+// A clustered tree has leaves whose lists hold forty times the mean number of
+// bodies (a large leaf beside many small ones): such a list is cut into parts
+// (p2p_part_bodies), each part leaves its sums in a slot of its own, and the
+// last part to finish adds the slots up in order, so that the result does not
+// depend on which one that is.  Measured: 150001 bodies in blobs (longest list
+// 60593 bodies, mean 1435), FP64, 3.98 -> 0.50 ms; 30011 in blobs, FP32,
+// 0.36 -> 0.052; 2^22 in blobs, FP32, 13.0 -> 8.2; uniform 2^20, ncrit = 256:
+// FP32 3.13 -> 3.07, FP64 9.28 -> 8.14 (24 -> 18 FP64 operations a pair).
+// FP32: bound by the FMA pipe (65% busy, 13 operations and one rsqrt a pair).
 // ---------------------------------------------------------------------------
 constexpr int kP2PWarps = P2P_WARPS;
 constexpr int kP2PUnroll = P2P_UNROLL;
-constexpr int kP2PTile = P2P_TILE;  // sources staged per tile (32 or 64)
+constexpr int kP2PFlush = P2P_FLUSH;  // tiles summed in FP32 before they go into FP64
 
-// Lanes of group `k0` (of G groups) take the tile's sources k0, k0+G, ...
-template <int G, bool MASK>
-__device__ __forceinline__ void p2p32_tile(const float4* __restrict__ s, int k0, int cnt, float px, float py,
-                                           float pz, float& p, float& fx, float& fy, float& fz) {
-#pragma unroll kP2PUnroll
-  for (int k = k0; k < cnt; k += G) {
-    const float4 b = s[k];
-    const float dx = px - b.x, dy = py - b.y, dz = pz - b.z;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    float ir = rsqrt_approx(r2);
-    if (MASK) ir = r2 > 0.f ? ir : 0.f;
-    const float qir = b.w * ir;
-    p += qir;
-    const float q3 = qir * ir * ir;
-    fx = fmaf(q3, dx, fx);
-    fy = fmaf(q3, dy, fy);
-    fz = fmaf(q3, dz, fz);
+// A chunk of up to 32 list entries, one per lane: `start` is the lane's
+// entry's first body in the chunk's sequence, `src` + position the body in
+// tree order.
+struct P2PChunk {
+  int start, src, total, nent;
+};
+__device__ __forceinline__ P2PChunk p2p_chunk(int boff, int bnum, int nent, int lane) {
+  P2PChunk c;
+  int s = bnum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += v;
+  }
+  c.start = s - bnum;
+  c.src = boff - c.start;
+  c.total = __shfl_sync(0xffffffffu, s, 31);
+  c.nent = nent;
+  return c;
+}
+// The entry (lane number) that holds the sequence's body base + lane: leaves
+// hold at least one body, so the starts are distinct and their bits count the
+// entries begun.
+__device__ __forceinline__ int p2p_entry(const P2PChunk& c, int base, int lane) {
+  const int rel = c.start - base;
+  const bool valid = lane < c.nent;
+  const unsigned before = __ballot_sync(0xffffffffu, valid && rel < 0);
+  const unsigned bit = valid && rel >= 0 && rel < 32 ? 1u << rel : 0u;
+  const unsigned begun = __reduce_or_sync(0xffffffffu, bit);
+  return __popc(before) + __popc(begun & (0xffffffffu >> (31 - lane))) - 1;
+}
+
+// The sums of a work item: written, or left in the item's slot when its list
+// is cut into parts.
+__device__ __forceinline__ void p2p_store(const P2PItem& it, bool writer, int ti, double P, double Gx, double Gy,
+                                          double Gz, double4* __restrict__ part, int* __restrict__ done,
+                                          double* __restrict__ phi, double* __restrict__ grad) {
+  if (it.nparts > 1) {
+    if (writer) part[(size_t)(it.slot + it.part) * 32 + ti] = make_double4(P, Gx, Gy, Gz);
+    __threadfence();
+    __syncwarp();
+    int last = 0;
+    if ((threadIdx.x & 31) == 0) last = atomicInc((unsigned*)done + it.slot, it.nparts - 1) == it.nparts - 1;
+    last = __shfl_sync(0xffffffffu, last, 0);
+    if (!last) return;
+    __threadfence();
+    if (writer) {
+      P = Gx = Gy = Gz = 0.0;
+      for (int k = 0; k < it.nparts; ++k) {
+        const double2* v = reinterpret_cast<const double2*>(part + (size_t)(it.slot + k) * 32 + ti);
+        const double2 a = __ldcg(v), b = __ldcg(v + 1);
+        P += a.x;
+        Gx += a.y;
+        Gy += b.x;
+        Gz += b.y;
+      }
+    }
+  }
+  if (writer) {
+    const int b = it.boff + ti;
+    phi[b] = P;
+    grad[3 * b + 0] = -Gx;
+    grad[3 * b + 1] = -Gy;
+    grad[3 * b + 2] = -Gz;
   }
 }
 
-// One source pair k of a packed tile (layout below) against this lane's target.
+// One source pair k of a tile against this lane's target, in packed FP32x2
+// arithmetic (sm_100 FADD2/FMUL2/FFMA2): the tile is held as 16 pairs, pair k
+// at s[2k] = (-x, -x', -y, -y') and s[2k+1] = (-z, -z', q, q'); the sums run
+// in two interleaved halves.  All 16 pairs of a tile are written (padding
+// carries no charge and sits far away).
 template <bool MASK>
 __device__ __forceinline__ void p2p32_pair2(const float4* __restrict__ s, int k, float2 px, float2 py, float2 pz,
                                             float2& p, float2& fx, float2& fy, float2& fz) {
@@ -243,118 +303,95 @@ __device__ __forceinline__ void p2p32_pair2(const float4* __restrict__ s, int k,
   fz = __ffma2_rn(q3, dz, fz);
 }
 
-// The same over source pairs with packed FP32x2 arithmetic (sm_100
-// FADD2/FMUL2/FFMA2): the tile is held as 16 pairs, pair k at s[2k] =
-// (-x, -x', -y, -y') and s[2k+1] = (-z, -z', q, q'); lanes of group k0 take
-// pairs k0, k0+G, ...  Per pair the arithmetic and its rounding are those of
-// p2p32_tile; only the sum over sources is split into two interleaved halves.
-// All 16 pairs of a tile are written (padding carries no charge and sits far
-// away); running the padding too, in fixed blocks, was measured slower.
-template <int G, bool MASK>
-__device__ __forceinline__ void p2p32_tile2(const float4* __restrict__ s, int k0, int npair, float2 px, float2 py,
-                                            float2 pz, float2& p, float2& fx, float2& fy, float2& fz) {
+// Lanes of group k0 (of G groups) take the tile's source pairs k0, k0+G, ...;
+// a full tile has a constant bound.
+template <int G, bool MASK, bool FULL>
+__device__ __forceinline__ void p2p32_tile(const float4* __restrict__ s, int k0, int npair, float2 px, float2 py,
+                                           float2 pz, float2& p, float2& fx, float2& fy, float2& fz) {
+  const int n = FULL ? 16 : npair;
 #pragma unroll kP2PUnroll
-  for (int k = k0; k < npair; k += G) p2p32_pair2<MASK>(s, k, px, py, pz, p, fx, fy, fz);
+  for (int k = k0; k < n; k += G) p2p32_pair2<MASK>(s, k, px, py, pz, p, fx, fy, fz);
 }
 
 // One work item: W = 32/G lanes per target group, G groups per warp.
 template <int G>
-__device__ __forceinline__ void p2p32_item(const float4* __restrict__ body32, const P2PItem32& it,
-                                           const int* __restrict__ list_off, const P2PSrc32* __restrict__ list,
-                                           float4* __restrict__ sw, int lane, double* __restrict__ phi,
-                                           double* __restrict__ grad) {
+__device__ __forceinline__ void p2p32_item(const float4* __restrict__ body32, const P2PItem& it,
+                                           const P2PSrc32* __restrict__ list, float4* __restrict__ sw, int lane,
+                                           double4* __restrict__ part, int* __restrict__ done,
+                                           double* __restrict__ phi, double* __restrict__ grad) {
   constexpr int W = 32 / G;
   const int grp = lane / W, ti = lane % W;
   const bool active = ti < it.nt;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   // tile padding: no charge, far from every target (finite 1/r)
   const float4 pad = make_float4(1e18f, 1e18f, 1e18f, 0.f);
-  const float4 xt = active ? body32[it.boff + ti] : zero;
+  const float4 xt = active ? body32[it.boff + ti] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float2 px = make_float2(xt.x, xt.x), py = make_float2(xt.y, xt.y), pz = make_float2(xt.z, xt.z);
   double P = 0.0, Gx = 0.0, Gy = 0.0, Gz = 0.0;
-  int e = list_off[it.leaf];
-  const int e1 = list_off[it.leaf + 1];
-  P2PSrc32 cur{}, nxt{};
-  // this lane stages sources c0 + lane + 32 h of the tile, h < kP2PTile / 32
-  constexpr int NH = kP2PTile / 32;
-  float4 stage[NH];
-#pragma unroll
-  for (int h = 0; h < NH; ++h) stage[h] = pad;
-  if (e < e1) {
-    cur = list[e];
-#pragma unroll
-    for (int h = 0; h < NH; ++h)
-      if (lane + 32 * h < cur.bnum) stage[h] = body32[cur.boff + lane + 32 * h];
-  }
-  if (e + 1 < e1) nxt = list[e + 1];
-  int c0 = 0;
-#if P2P_PACKED
   float2 p = make_float2(0.f, 0.f), fx = p, fy = p, fz = p;
+  auto entry = [&](int e) { return e < it.e1 ? list[e] : P2PSrc32{}; };
+  P2PSrc32 cur{}, nxt{};  // this lane's entry of the chunk and of the next one
+  P2PChunk c{};
+  int self0 = 0, self1 = 0;  // the target leaf's own bodies in the chunk's sequence
+  auto chunk = [&](int e0) {
+    c = p2p_chunk(cur.boff, cur.bnum, min(32, it.e1 - e0), lane);
+    const unsigned own = __ballot_sync(0xffffffffu, cur.self);
+    const int o = own ? __ffs(own) - 1 : 0;
+    self0 = own ? __shfl_sync(0xffffffffu, c.start, o) : 0;
+    self1 = own ? self0 + __shfl_sync(0xffffffffu, cur.bnum, o) : 0;
+  };
+  float4 b = pad;  // the next tile's body of this lane and its leaf's offset
+  float ox = 0.f, oy = 0.f, oz = 0.f;
+  auto stage = [&](int base) {
+    const int s = p2p_entry(c, base, lane), pos = base + lane;
+    const int i = __shfl_sync(0xffffffffu, c.src, s) + pos;
+    ox = __shfl_sync(0xffffffffu, cur.dx, s);
+    oy = __shfl_sync(0xffffffffu, cur.dy, s);
+    oz = __shfl_sync(0xffffffffu, cur.dz, s);
+    b = pos < c.total ? body32[i] : pad;
+  };
+  int e = it.e0, base = 0, tiles = 0;
+  bool more = e < it.e1;
+  if (more) {
+    cur = entry(e + lane);
+    nxt = entry(e + 32 + lane);
+    chunk(e);
+    stage(0);
+  }
   float* sf = reinterpret_cast<float*>(sw) + 8 * (lane >> 1) + (lane & 1);
-#else
-  static_assert(kP2PTile == 32, "the scalar P2P form stages 32 sources");
-  float p = 0.f, fx = 0.f, fy = 0.f, fz = 0.f;
-#endif
-  while (e < e1) {
-    const int cnt = min(kP2PTile, cur.bnum - c0);
+  while (more) {
+    const int cnt = min(32, c.total - base);
+    const bool mask = self0 < base + 32 && self1 > base;
     __syncwarp();
-#if P2P_PACKED
-#pragma unroll
-    for (int h = 0; h < NH; ++h) {
-      sf[128 * h + 0] = -stage[h].x;
-      sf[128 * h + 2] = -stage[h].y;
-      sf[128 * h + 4] = -stage[h].z;
-      sf[128 * h + 6] = stage[h].w;
-    }
-#else
-    sw[lane] = stage[0];
-#endif
+    sf[0] = -(b.x + ox);
+    sf[2] = -(b.y + oy);
+    sf[4] = -(b.z + oz);
+    sf[6] = b.w;
     __syncwarp();
-    // next tile: the rest of this source leaf, else the first of the next
-    const bool last = c0 + kP2PTile >= cur.bnum;
-#pragma unroll
-    for (int h = 0; h < NH; ++h) {
-      stage[h] = pad;
-      if (!last) {
-        if (lane + 32 * h < cur.bnum - c0 - kP2PTile) stage[h] = body32[cur.boff + c0 + kP2PTile + lane + 32 * h];
-      } else if (e + 1 < e1) {
-        if (lane + 32 * h < nxt.bnum) stage[h] = body32[nxt.boff + lane + 32 * h];
+    base += 32;
+    if (base >= c.total) {
+      e += 32;
+      base = 0;
+      more = e < it.e1;
+      if (more) {
+        cur = nxt;
+        nxt = entry(e + 32 + lane);
+        chunk(e);
       }
     }
-    const float px = xt.x - cur.dx, py = xt.y - cur.dy, pz = xt.z - cur.dz;
-#if P2P_PACKED
-    const int npair = (cnt + 1) >> 1;
-    if (cur.self)
-      p2p32_tile2<G, true>(sw, grp, npair, make_float2(px, px), make_float2(py, py), make_float2(pz, pz), p, fx,
-                           fy, fz);
+    if (more) stage(base);
+    if (mask)
+      p2p32_tile<G, true, false>(sw, grp, (cnt + 1) >> 1, px, py, pz, p, fx, fy, fz);
+    else if (cnt == 32)
+      p2p32_tile<G, false, true>(sw, grp, 16, px, py, pz, p, fx, fy, fz);
     else
-      p2p32_tile2<G, false>(sw, grp, npair, make_float2(px, px), make_float2(py, py), make_float2(pz, pz), p, fx,
-                            fy, fz);
-#else
-    if (cur.self)
-      p2p32_tile<G, true>(sw, grp, cnt, px, py, pz, p, fx, fy, fz);
-    else
-      p2p32_tile<G, false>(sw, grp, cnt, px, py, pz, p, fx, fy, fz);
-#endif
-    if (last) {
-#if P2P_PACKED
+      p2p32_tile<G, false, false>(sw, grp, (cnt + 1) >> 1, px, py, pz, p, fx, fy, fz);
+    if (++tiles == kP2PFlush || !more) {
+      tiles = 0;
       P += (double)p.x + (double)p.y;
       Gx += (double)fx.x + (double)fx.y;
       Gy += (double)fy.x + (double)fy.y;
       Gz += (double)fz.x + (double)fz.y;
       p = fx = fy = fz = make_float2(0.f, 0.f);
-#else
-      P += (double)p;
-      Gx += (double)fx;
-      Gy += (double)fy;
-      Gz += (double)fz;
-      p = fx = fy = fz = 0.f;
-#endif
-      ++e;
-      c0 = 0;
-      cur = nxt;
-      if (e + 1 < e1) nxt = list[e + 1];
-    } else {
-      c0 += kP2PTile;
     }
   }
   // sum the source groups (lanes ti, ti + W, ...)
@@ -365,89 +402,103 @@ __device__ __forceinline__ void p2p32_item(const float4* __restrict__ body32, co
     Gy += __shfl_xor_sync(0xffffffffu, Gy, o);
     Gz += __shfl_xor_sync(0xffffffffu, Gz, o);
   }
-  if (active && grp == 0) {
-    const int b = it.boff + ti;
-    phi[b] = P;
-    grad[3 * b + 0] = -Gx;
-    grad[3 * b + 1] = -Gy;
-    grad[3 * b + 2] = -Gz;
-  }
+  p2p_store(it, active && grp == 0, ti, P, Gx, Gy, Gz, part, done, phi, grad);
 }
 
 __global__ void __launch_bounds__(32 * kP2PWarps, P2P_MINB)
-    k_p2p32(const float4* __restrict__ body32, const P2PItem32* __restrict__ items, int nitems,
-            const int* __restrict__ list_off, const P2PSrc32* __restrict__ list, double* __restrict__ phi,
-            double* __restrict__ grad) {
-  __shared__ float4 sbuf[kP2PWarps][kP2PTile];
+    k_p2p32(const float4* __restrict__ body32, const P2PItem* __restrict__ items, int nitems,
+            const P2PSrc32* __restrict__ list, double4* __restrict__ part, int* __restrict__ done,
+            double* __restrict__ phi, double* __restrict__ grad) {
+  __shared__ float4 sbuf[kP2PWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = blockIdx.x * kP2PWarps + warp;
   if (item >= nitems) return;  // warp-uniform
-  const P2PItem32 it = items[item];
+  const P2PItem it = items[item];
   switch (it.lw) {
-    case 5: p2p32_item<1>(body32, it, list_off, list, sbuf[warp], lane, phi, grad); break;
-    case 4: p2p32_item<2>(body32, it, list_off, list, sbuf[warp], lane, phi, grad); break;
-    case 3: p2p32_item<4>(body32, it, list_off, list, sbuf[warp], lane, phi, grad); break;
-    default: p2p32_item<8>(body32, it, list_off, list, sbuf[warp], lane, phi, grad); break;
+    case 5: p2p32_item<1>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    case 4: p2p32_item<2>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    case 3: p2p32_item<4>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    default: p2p32_item<8>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
   }
 }
 
-// FP64 P2P, the same work items as the FP32 kernel (lane groups for a leaf's
-// last targets, next tile and list entry loaded during the current tile);
-// per pair the reference's arithmetic (dx = x_t - (x_s + offset),
-// kernel.cpp:283-290) in FP64 with the Newton-refined reciprocal square root.
+// 1/sqrt(x) in FP64 for the FP64 P2P: from the hardware seed y (9.1e-7
+// relative), with e = 1 - x y^2 the Taylor series of (1 - e)^(-1/2) to second
+// order, y (1 + e/2 + 3 e^2/8) (Householder's method of third order; the
+// remainder 5/16 e^3 is 2e-18), five operations.  Zero for x = 0, by the high
+// word on the integer pipe instead of a comparison on the FP64 pipe, which is
+// what bounds the kernel; other x must be normal.
+__device__ __forceinline__ double rsqrt_or_zero(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const int hi = __double2hiint(x);
+  y = __hiloint2double(hi ? __double2hiint(y) : 0, hi ? __double2loint(y) : 0);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// FP64 P2P, the same work items; per pair the reference's arithmetic
+// (dx = x_t - (x_s + offset), kernel.cpp:283-290) in FP64, 18 operations.
 template <int G>
-__device__ __forceinline__ void p2p64_item(const double4* __restrict__ body64, const P2PItem32& it,
-                                           const int* __restrict__ list_off, const P2PSrc64* __restrict__ list,
-                                           double4* __restrict__ sw, int lane, double* __restrict__ phi,
-                                           double* __restrict__ grad) {
+__device__ __forceinline__ void p2p64_item(const double4* __restrict__ body64, const P2PItem& it,
+                                           const P2PSrc64* __restrict__ list, double4* __restrict__ sw, int lane,
+                                           double4* __restrict__ part, int* __restrict__ done,
+                                           double* __restrict__ phi, double* __restrict__ grad) {
   constexpr int W = 32 / G;
   const int grp = lane / W, ti = lane % W;
   const bool active = ti < it.nt;
   const double4 zero = make_double4(0.0, 0.0, 0.0, 0.0);
   const double4 xt = active ? body64[it.boff + ti] : zero;
   double P = 0.0, Gx = 0.0, Gy = 0.0, Gz = 0.0;
-  int e = list_off[it.leaf];
-  const int e1 = list_off[it.leaf + 1];
+  auto entry = [&](int e) { return e < it.e1 ? list[e] : P2PSrc64{}; };
   P2PSrc64 cur{}, nxt{};
-  double4 stage = zero;
-  if (e < e1) {
-    cur = list[e];
-    if (lane < cur.bnum) stage = body64[cur.boff + lane];
+  P2PChunk c{};
+  double4 b = zero;
+  double ox = 0.0, oy = 0.0, oz = 0.0;
+  auto stage = [&](int base) {
+    const int s = p2p_entry(c, base, lane), pos = base + lane;
+    const int i = __shfl_sync(0xffffffffu, c.src, s) + pos;
+    ox = __shfl_sync(0xffffffffu, cur.ox, s);
+    oy = __shfl_sync(0xffffffffu, cur.oy, s);
+    oz = __shfl_sync(0xffffffffu, cur.oz, s);
+    b = pos < c.total ? body64[i] : zero;
+  };
+  int e = it.e0, base = 0;
+  bool more = e < it.e1;
+  if (more) {
+    cur = entry(e + lane);
+    nxt = entry(e + 32 + lane);
+    c = p2p_chunk(cur.boff, cur.bnum, min(32, it.e1 - e), lane);
+    stage(0);
   }
-  if (e + 1 < e1) nxt = list[e + 1];
-  int c0 = 0;
-  while (e < e1) {
-    const int cnt = min(32, cur.bnum - c0);
+  while (more) {
+    const int cnt = min(32, c.total - base);
     __syncwarp();
-    sw[lane] = stage;
+    sw[lane] = make_double4(b.x + ox, b.y + oy, b.z + oz, b.w);
     __syncwarp();
-    const bool last = c0 + 32 >= cur.bnum;
-    stage = zero;
-    if (!last) {
-      if (lane < cur.bnum - c0 - 32) stage = body64[cur.boff + c0 + 32 + lane];
-    } else if (e + 1 < e1) {
-      if (lane < nxt.bnum) stage = body64[nxt.boff + lane];
+    base += 32;
+    if (base >= c.total) {
+      e += 32;
+      base = 0;
+      more = e < it.e1;
+      if (more) {
+        cur = nxt;
+        nxt = entry(e + 32 + lane);
+        c = p2p_chunk(cur.boff, cur.bnum, min(32, it.e1 - e), lane);
+      }
     }
+    if (more) stage(base);
 #pragma unroll 4
     for (int k = grp; k < cnt; k += G) {
-      const double4 b = sw[k];
-      const double dx = xt.x - (b.x + cur.ox), dy = xt.y - (b.y + cur.oy), dz = xt.z - (b.z + cur.oz);
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      const double ir = r2 > 0.0 ? rsqrt_nr<2>(r2) : 0.0;
-      const double qir = b.w * ir;
+      const double4 s = sw[k];
+      const double dx = xt.x - s.x, dy = xt.y - s.y, dz = xt.z - s.z;
+      const double ir = rsqrt_or_zero(dx * dx + dy * dy + dz * dz);
+      const double qir = s.w * ir;
       P += qir;
       const double q3 = qir * ir * ir;
       Gx += q3 * dx;
       Gy += q3 * dy;
       Gz += q3 * dz;
-    }
-    if (last) {
-      ++e;
-      c0 = 0;
-      cur = nxt;
-      if (e + 1 < e1) nxt = list[e + 1];
-    } else {
-      c0 += 32;
     }
   }
 #pragma unroll
@@ -457,29 +508,23 @@ __device__ __forceinline__ void p2p64_item(const double4* __restrict__ body64, c
     Gy += __shfl_xor_sync(0xffffffffu, Gy, o);
     Gz += __shfl_xor_sync(0xffffffffu, Gz, o);
   }
-  if (active && grp == 0) {
-    const int bi = it.boff + ti;
-    phi[bi] = P;
-    grad[3 * bi + 0] = -Gx;
-    grad[3 * bi + 1] = -Gy;
-    grad[3 * bi + 2] = -Gz;
-  }
+  p2p_store(it, active && grp == 0, ti, P, Gx, Gy, Gz, part, done, phi, grad);
 }
 
 __global__ void __launch_bounds__(32 * kP2PWarps)
-    k_p2p64(const double4* __restrict__ body64, const P2PItem32* __restrict__ items, int nitems,
-            const int* __restrict__ list_off, const P2PSrc64* __restrict__ list, double* __restrict__ phi,
-            double* __restrict__ grad) {
+    k_p2p64(const double4* __restrict__ body64, const P2PItem* __restrict__ items, int nitems,
+            const P2PSrc64* __restrict__ list, double4* __restrict__ part, int* __restrict__ done,
+            double* __restrict__ phi, double* __restrict__ grad) {
   __shared__ double4 sbuf[kP2PWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = blockIdx.x * kP2PWarps + warp;
   if (item >= nitems) return;  // warp-uniform
-  const P2PItem32 it = items[item];
+  const P2PItem it = items[item];
   switch (it.lw) {
-    case 5: p2p64_item<1>(body64, it, list_off, list, sbuf[warp], lane, phi, grad); break;
-    case 4: p2p64_item<2>(body64, it, list_off, list, sbuf[warp], lane, phi, grad); break;
-    case 3: p2p64_item<4>(body64, it, list_off, list, sbuf[warp], lane, phi, grad); break;
-    default: p2p64_item<8>(body64, it, list_off, list, sbuf[warp], lane, phi, grad); break;
+    case 5: p2p64_item<1>(body64, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    case 4: p2p64_item<2>(body64, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    case 3: p2p64_item<4>(body64, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    default: p2p64_item<8>(body64, it, list, sbuf[warp], lane, part, done, phi, grad); break;
   }
 }
 
@@ -511,15 +556,15 @@ constexpr float kCloseFrac = CLOSE_FRAC;
 // (source body, list entry) of target t at pairs[off[t] ...], in list order.
 template <bool EMIT>
 __global__ void __launch_bounds__(256)
-    k_close_scan(const float4* __restrict__ body32, const P2PItem32* __restrict__ items, int nitems,
+    k_close_scan(const float4* __restrict__ body32, const P2PItem* __restrict__ items, int nitems,
                  const int* __restrict__ list_off, const P2PSrc32* __restrict__ list,
                  const LeafInfo* __restrict__ leaves, int* __restrict__ cnt, const int* __restrict__ off,
                  int2* __restrict__ pairs) {
   const int item = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (item >= nitems) return;
-  const P2PItem32 it = items[item];
-  if (lane >= it.nt) return;
+  const P2PItem it = items[item];
+  if (it.part > 0 || lane >= it.nt) return;  // a cut list's first item scans all of it
   const int t = it.boff + lane;
   const float4 xt = body32[t];
   const float rt = (float)leaves[it.leaf].r;
@@ -542,7 +587,7 @@ __global__ void __launch_bounds__(256)
     if (!__any_sync(mask, bx * bx + by * by + bz * bz < rc2)) continue;
     for (int k = 0; k < s.bnum; ++k) {
       const float4 b = body32[s.boff + k];
-      const float dx = px - b.x, dy = py - b.y, dz = pz - b.z;
+      const float dx = xt.x - (b.x + s.dx), dy = xt.y - (b.y + s.dy), dz = xt.z - (b.z + s.dz);
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
       if (r2 < rc2 && !(s.self && s.boff + k == t)) {
         if (EMIT) {
@@ -574,8 +619,8 @@ __global__ void k_close_fix(const double4* __restrict__ body64, const float4* __
     const P2PSrc32 s = list[pr.y];
     // the FP32 terms exactly as k_p2p32 formed them
     const float4 b = body32[pr.x];
-    const float px = xt.x - s.dx, py = xt.y - s.dy, pz = xt.z - s.dz;
-    const float dx = __fadd_rn(px, -b.x), dy = __fadd_rn(py, -b.y), dz = __fadd_rn(pz, -b.z);
+    const float dx = __fadd_rn(xt.x, -__fadd_rn(b.x, s.dx)), dy = __fadd_rn(xt.y, -__fadd_rn(b.y, s.dy)),
+                dz = __fadd_rn(xt.z, -__fadd_rn(b.z, s.dz));
     float r2 = __fmul_rn(dz, dz);
     r2 = __fmaf_rn(dy, dy, r2);
     r2 = __fmaf_rn(dx, dx, r2);
@@ -2054,23 +2099,21 @@ cudaError_t launch_prep32(const double4* body64, const int* body_leaf, const Lea
   return cudaGetLastError();
 }
 
-cudaError_t launch_p2p32(const float4* body32, const P2PItem32* items, int nitems, const int* list_off,
-                         const P2PSrc32* list, double* phi, double* grad, cudaStream_t st) {
+cudaError_t launch_p2p32(const float4* body32, const P2PItem* items, int nitems, const P2PSrc32* list, double4* part,
+                         int* done, double* phi, double* grad, cudaStream_t st) {
   if (nitems > 0)
-    k_p2p32<<<cdiv(nitems, kP2PWarps), 32 * kP2PWarps, 0, st>>>(body32, items, nitems, list_off, list, phi,
-                                                               grad);
+    k_p2p32<<<cdiv(nitems, kP2PWarps), 32 * kP2PWarps, 0, st>>>(body32, items, nitems, list, part, done, phi, grad);
   return cudaGetLastError();
 }
 
-cudaError_t launch_p2p64(const double4* body64, const P2PItem32* items, int nitems, const int* list_off,
-                         const P2PSrc64* list, double* phi, double* grad, cudaStream_t st) {
+cudaError_t launch_p2p64(const double4* body64, const P2PItem* items, int nitems, const P2PSrc64* list, double4* part,
+                         int* done, double* phi, double* grad, cudaStream_t st) {
   if (nitems > 0)
-    k_p2p64<<<cdiv(nitems, kP2PWarps), 32 * kP2PWarps, 0, st>>>(body64, items, nitems, list_off, list, phi,
-                                                               grad);
+    k_p2p64<<<cdiv(nitems, kP2PWarps), 32 * kP2PWarps, 0, st>>>(body64, items, nitems, list, part, done, phi, grad);
   return cudaGetLastError();
 }
 
-cudaError_t launch_close_count(const float4* body32, const P2PItem32* items, int nitems, const int* list_off,
+cudaError_t launch_close_count(const float4* body32, const P2PItem* items, int nitems, const int* list_off,
                                const P2PSrc32* list, const LeafInfo* leaves, int* cnt, cudaStream_t st) {
   if (nitems > 0)
     k_close_scan<false><<<cdiv(nitems, 8), 256, 0, st>>>(body32, items, nitems, list_off, list, leaves, cnt,
@@ -2078,7 +2121,7 @@ cudaError_t launch_close_count(const float4* body32, const P2PItem32* items, int
   return cudaGetLastError();
 }
 
-cudaError_t launch_close_emit(const float4* body32, const P2PItem32* items, int nitems, const int* list_off,
+cudaError_t launch_close_emit(const float4* body32, const P2PItem* items, int nitems, const int* list_off,
                               const P2PSrc32* list, const LeafInfo* leaves, const int* off, int2* pairs,
                               cudaStream_t st) {
   if (nitems > 0)

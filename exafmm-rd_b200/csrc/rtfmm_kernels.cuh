@@ -19,12 +19,28 @@ struct LeafInfo {
 // P2P work item: nt <= W targets of one leaf, W = 1 << lw
 // lanes per target group; the 32/W groups of a warp split every source tile
 // between them, so a leaf's last few targets do not leave most lanes idle.
-struct P2PItem32 {
-  int leaf;   // leaf-table index of the target leaf (its source list)
-  int boff;   // first target body (tree order)
-  int nt;     // targets in this item (1..W)
-  int lw;     // log2 W, W in {4, 8, 16, 32}
+// `e0`..`e1` is the item's part of the leaf's source list: a list of more than
+// p2p_part_bodies bodies is cut into `nparts` items of the same targets, whose
+// sums meet in slots `slot`..`slot + nparts - 1`.
+struct P2PItem {
+  int leaf;      // leaf-table index of the target leaf
+  int boff;      // first target body (tree order)
+  short nt, lw;  // targets in this item (1..W); log2 W, W in {4, 8, 16, 32}
+  int e0, e1;    // source-list entries
+  int part, nparts, slot;
 };
+// Bodies of a source list from which it is cut, for a plan with `work` =
+// sum over leaves of list bodies x target groups of 32.  A part is at most
+// about an eighth of what each of the 20 warps an SM holds (148 SMs) has to
+// do, so that no warp is left running alone for long, and at least 256 bodies,
+// below which a part's fixed cost shows.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int p2p_part_bodies(unsigned long long work) {
+  const unsigned long long s = work / (148 * 20 * 8);
+  return s < 256 ? 256 : s > (1 << 20) ? 1 << 20 : (int)s;
+}
 
 // One P2P list entry (source leaf) of a target leaf, FP32 form.  Both forms
 // carry the source's body range so that the kernels read bodies with one
@@ -61,17 +77,21 @@ struct ApplyBatch {
 cudaError_t launch_body_leaf(const LeafInfo* leaves, int nleaf, int n, int* body_leaf, cudaStream_t st);
 cudaError_t launch_prep32(const double4* body64, const int* body_leaf, const LeafInfo* leaves,
                           float4* body32, int n, cudaStream_t st);
-cudaError_t launch_p2p32(const float4* body32, const P2PItem32* items, int nitems, const int* list_off,
-                         const P2PSrc32* list, double* phi, double* grad, cudaStream_t st);
-cudaError_t launch_p2p64(const double4* body64, const P2PItem32* items, int nitems, const int* list_off,
-                         const P2PSrc64* list, double* phi, double* grad, cudaStream_t st);
+// part: 32 double4 per slot of the items, done: one counter per slot, zero
+// before the first pass (every pass leaves them zero)
+cudaError_t launch_p2p32(const float4* body32, const P2PItem* items, int nitems,
+                         const P2PSrc32* list, double4* part, int* done, double* phi, double* grad,
+                         cudaStream_t st);
+cudaError_t launch_p2p64(const double4* body64, const P2PItem* items, int nitems,
+                         const P2PSrc64* list, double4* part, int* done, double* phi, double* grad,
+                         cudaStream_t st);
 // Close-pair refinement of the FP32 P2P: per-target counts of the pairs
 // closer than a fraction of their leaves (cnt[t], tree order), their list
 // (source body, list entry) at pairs[off[t]...], and the per-pass fix that
 // replaces their FP32 terms in phi / grad (P2P outputs) by FP64 ones.
-cudaError_t launch_close_count(const float4* body32, const P2PItem32* items, int nitems, const int* list_off,
+cudaError_t launch_close_count(const float4* body32, const P2PItem* items, int nitems, const int* list_off,
                                const P2PSrc32* list, const LeafInfo* leaves, int* cnt, cudaStream_t st);
-cudaError_t launch_close_emit(const float4* body32, const P2PItem32* items, int nitems, const int* list_off,
+cudaError_t launch_close_emit(const float4* body32, const P2PItem* items, int nitems, const int* list_off,
                               const P2PSrc32* list, const LeafInfo* leaves, const int* off, int2* pairs,
                               cudaStream_t st);
 // cycle > 0: periodic (nearest image); 0: free space

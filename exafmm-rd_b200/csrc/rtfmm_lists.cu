@@ -434,26 +434,41 @@ __device__ __forceinline__ void leaf_run(const LeafTables& T, int c, int* lo, in
   *hi = T.dfs_pos[T.body_leaf[b0 + nb - 1]] + 1;
 }
 
-__global__ void k_leaf_list_count(LeafTables T, int* __restrict__ cnt, int* __restrict__ icnt) {
+// cnt: list entries of leaf l; bodies: bodies of those entries; work: their
+// sum over the leaves, times the leaf's target groups.
+__global__ void k_leaf_list_count(LeafTables T, int* __restrict__ cnt, int* __restrict__ bodies,
+                                  unsigned long long* __restrict__ work) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= T.nlf) return;
   int path[kMaxPathLen];
   const int np = leaf_path(T, T.leaves[l].cell, path);
-  int c = 0;
+  int c = 0, nb = 0;
   for (int i = 0; i < np; ++i)
     for (int e = T.cstart[path[i]]; e < T.cend[path[i]]; ++e) {
       const int sc = (int)((T.pairs[e] >> 5) & ((1ull << kCellBits) - 1));
       int lo, hi;
       leaf_run(T, sc, &lo, &hi);
       c += hi - lo;
+      nb += T.cbnum[sc];
     }
   cnt[l] = c;
-  icnt[l] = (T.leaves[l].bnum + 31) / 32;
+  bodies[l] = nb;
+  atomicAdd(work, (unsigned long long)nb * ((T.leaves[l].bnum + 31) / 32));
 }
 
-__global__ void k_leaf_list_fill(LeafTables T, const int* __restrict__ off, const int* __restrict__ ioff, int mixed,
-                                 P2PSrc32* __restrict__ l32, P2PSrc64* __restrict__ l64,
-                                 P2PItem32* __restrict__ items, unsigned long long* __restrict__ pair_total) {
+// Work items of leaf l: its target groups of 32 times the parts of its list.
+__global__ void k_leaf_item_count(LeafTables T, const int* __restrict__ bodies,
+                                  const unsigned long long* __restrict__ work, int* __restrict__ icnt) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= T.nlf) return;
+  const int S = p2p_part_bodies(*work);
+  icnt[l] = (T.leaves[l].bnum + 31) / 32 * max(1, (bodies[l] + S - 1) / S);
+}
+
+__global__ void k_leaf_list_fill(LeafTables T, const int* __restrict__ off, const int* __restrict__ ioff,
+                                 const int* __restrict__ bodies, int mixed, P2PSrc32* __restrict__ l32,
+                                 P2PSrc64* __restrict__ l64, P2PItem* __restrict__ items,
+                                 unsigned long long* __restrict__ pair_total, int* __restrict__ nslots) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= T.nlf) return;
   const LeafInfo Tl = T.leaves[l];
@@ -461,6 +476,24 @@ __global__ void k_leaf_list_fill(LeafTables T, const int* __restrict__ off, cons
   const int np = leaf_path(T, Tl.cell, path);
   int k = off[l];
   unsigned long long pairs = 0;
+  // work items: 32 targets each (the last <= 16 targets of a leaf take a
+  // narrower lane group: 16, 8 or 4 lanes) times the parts of the list: part
+  // p starts at the first entry with p/nparts of the bodies before it
+  const int groups = (Tl.bnum + 31) / 32, nparts = groups ? (ioff[l + 1] - ioff[l]) / groups : 0;
+  const int slot0 = nparts > 1 ? atomicAdd(nslots, groups * nparts) : 0;
+  int before = 0, next = 0;  // bodies of the entries so far, parts begun
+  auto begin_parts = [&](int entry, bool end) {
+    for (; next < nparts && (end || before >= (long long)next * bodies[l] / nparts); ++next)
+      for (int g = 0; g < groups; ++g) {
+        const int rem = min(32, Tl.bnum - 32 * g);
+        int lw = 5;
+        while (lw > 2 && rem <= (1 << (lw - 1))) --lw;
+        P2PItem* it = items + ioff[l] + next * groups + g;
+        *it = P2PItem{l, Tl.boff + 32 * g, (short)rem, (short)lw, entry, off[l + 1], next, nparts,
+                      slot0 + g * nparts};
+        if (next > 0) (it - groups)->e1 = entry;
+      }
+  };
   for (int i = 0; i < np; ++i)
     for (int e = T.cstart[path[i]]; e < T.cend[path[i]]; ++e) {
       const unsigned long long v = T.pairs[e];
@@ -472,6 +505,8 @@ __global__ void k_leaf_list_fill(LeafTables T, const int* __restrict__ off, cons
         const int sl = T.dfs[r];
         const LeafInfo Sl = T.leaves[sl];
         const int self = (Sl.cell == Tl.cell && o[0] == 0 && o[1] == 0 && o[2] == 0) ? 1 : 0;
+        begin_parts(k, false);
+        before += Sl.bnum;
         if (mixed) {
           P2PSrc32 a;
           // the host build's expression: (c_src + offset) - c_tar in FP64, then FP32
@@ -500,15 +535,7 @@ __global__ void k_leaf_list_fill(LeafTables T, const int* __restrict__ off, cons
       }
     }
   atomicAdd(pair_total, pairs);
-  // work items: 32 targets each; the last <= 16 targets of a leaf take a
-  // narrower lane group (16, 8 or 4 lanes)
-  int j = ioff[l];
-  for (int t0 = 0; t0 < Tl.bnum; t0 += 32, ++j) {
-    const int rem = min(32, Tl.bnum - t0);
-    int lw = 5;
-    while (lw > 2 && rem <= (1 << (lw - 1))) --lw;
-    items[j] = P2PItem32{l, Tl.boff + t0, rem, lw};
-  }
+  begin_parts(k, true);
 }
 
 }  // namespace
@@ -518,26 +545,28 @@ int device_p2p_tables(const DeviceWalk& w, const DeviceLeafInput& in, bool mixed
                       std::string& msg) {
   Scratch S{scratch, slot_base};
   const int nlf = in.nlf;
-  int *cstart, *cend, *cnt, *icnt, *off, *ioff;
-  unsigned long long* total;
+  int *cstart, *cend, *cnt, *icnt, *off, *ioff, *bodies;
+  unsigned long long* total;  // body pairs, work, slots
   LCK(S.get(0, &cstart, w.ncell));
   LCK(S.get(1, &cend, w.ncell));
   LCK(S.get(2, &cnt, nlf + 1));
   LCK(S.get(3, &icnt, nlf + 1));
   LCK(S.get(4, &ioff, nlf + 1));
-  LCK(S.get(5, &total, 1));
+  LCK(S.get(5, &total, 3));
+  LCK(S.get(7, &bodies, nlf));
   LCK(cudaMemsetAsync(cstart, 0, sizeof(int) * w.ncell, st));
   LCK(cudaMemsetAsync(cend, 0, sizeof(int) * w.ncell, st));
   LCK(cudaMemsetAsync(cnt + nlf, 0, sizeof(int), st));
   LCK(cudaMemsetAsync(icnt + nlf, 0, sizeof(int), st));
-  LCK(cudaMemsetAsync(total, 0, sizeof(unsigned long long), st));
+  LCK(cudaMemsetAsync(total, 0, 3 * sizeof(unsigned long long), st));
   if (w.npairs > 0) {
     k_pair_bounds<<<cdiv(w.npairs, 256), 256, 0, st>>>(w.pairs, w.npairs, cstart, cend);
     LCK(cudaGetLastError());
   }
   LeafTables T{in.leaves, nlf, in.parent, w.cboff, w.cbnum, in.body_leaf, in.dfs, in.dfs_pos, cstart, cend,
                w.pairs, w.offs};
-  k_leaf_list_count<<<cdiv(nlf, 128), 128, 0, st>>>(T, cnt, icnt);
+  k_leaf_list_count<<<cdiv(nlf, 128), 128, 0, st>>>(T, cnt, bodies, total + 1);
+  k_leaf_item_count<<<cdiv(nlf, 128), 128, 0, st>>>(T, bodies, total + 1, icnt);
   LCK(cudaGetLastError());
   off = alloc.list_off(nlf + 1);
   if (!off) {
@@ -560,19 +589,21 @@ int device_p2p_tables(const DeviceWalk& w, const DeviceLeafInput& in, bool mixed
     l32 = alloc.list32(tot[0]);
   else
     l64 = alloc.list64(tot[0]);
-  P2PItem32* items = alloc.items(tot[1]);
+  P2PItem* items = alloc.items(tot[1]);
   if ((mixed && !l32) || (!mixed && !l64) || !items) {
     msg = "device allocation of the P2P lists failed";
     return kTreeError;
   }
-  k_leaf_list_fill<<<cdiv(nlf, 128), 128, 0, st>>>(T, off, ioff, mixed ? 1 : 0, l32, l64, items, total);
+  k_leaf_list_fill<<<cdiv(nlf, 128), 128, 0, st>>>(T, off, ioff, bodies, mixed ? 1 : 0, l32, l64, items, total,
+                                                   reinterpret_cast<int*>(total + 2));
   LCK(cudaGetLastError());
-  unsigned long long pairs = 0;
-  LCK(cudaMemcpyAsync(&pairs, total, sizeof(pairs), cudaMemcpyDeviceToHost, st));
+  unsigned long long sums[3];
+  LCK(cudaMemcpyAsync(sums, total, sizeof(sums), cudaMemcpyDeviceToHost, st));
   LCK(cudaStreamSynchronize(st));
   out->nlist = tot[0];
   out->nitems = tot[1];
-  out->pairs = (int64_t)pairs;
+  out->nslots = (int)(unsigned)sums[2];
+  out->pairs = (int64_t)sums[0];
   return kTreeOk;
 }
 

@@ -71,10 +71,10 @@ struct P2PTableAlloc {
   std::function<int*(int)> list_off;
   std::function<P2PSrc32*(int)> list32;
   std::function<P2PSrc64*(int)> list64;
-  std::function<P2PItem32*(int)> items;
+  std::function<P2PItem*(int)> items;
 };
 struct P2PTablesOut {
-  int nlist = 0, nitems = 0;
+  int nlist = 0, nitems = 0, nslots = 0;
   int64_t pairs = 0;  // body pairs: sum over entries of n_target * n_source
 };
 int device_p2p_tables(const DeviceWalk& w, const DeviceLeafInput& in, bool mixed, cudaStream_t st,

@@ -48,3 +48,33 @@ def test_far_field_at_every_order(pkg, oracle, P, n, ncrit, images, precision):
     tol = 1e-5 if precision else 1e-9 if P < 9 else 1e-7
     assert l2(grad, rgrad) < tol
     assert l2(phi - phi.mean(), rphi - rphi.mean()) < max(tol, 1e-8)
+
+
+# near field where source lists are cut into parts: a leaf of 200 bodies
+# beside leaves of one to eight, and lists of many tiny leaves (more than 32
+# entries); target groups of 1, 4, 5, 16, 17, 32 and 33 bodies
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("images", [0, 1])
+def test_near_field_with_long_lists(pkg, oracle, images, precision):
+    rng = np.random.default_rng(7)
+    sizes = [200, 33, 32, 17, 16, 5, 4, 1]
+    corners = np.array([[i, j, k] for i in (0, 1) for j in (0, 1) for k in (0, 1)])
+    parts = [(c + rng.random((m, 3))) * 0.25 for c, m in zip(corners, sizes)]  # eight leaves of edge 1/4
+    parts.append(0.5 + 0.02 * rng.standard_normal((1500, 3)))  # a dense cluster at their corner
+    x = np.clip(np.concatenate(parts), 1e-6, 1 - 1e-6)
+    q = rng.standard_normal(len(x))
+    q -= q.mean()
+    f = pkg.LaplaceFMM(x, q, args(pkg, 4, 8 if images else 200, images, precision, pkg.STAGE_NEAR))
+    phi, grad = f.solve()
+    f.setup()
+    lo, src, _ = f.leaf_lists()
+    ints, _ = f.cells()
+    leaf = ints[:f.info()["ncell"]]
+    bnum = leaf[(leaf[:, 3] == 0) & (leaf[:, 5] > 0), 5][:f.info()["nleaf"]]
+    bodies = np.add.reduceat(bnum[src], lo[:-1])
+    assert bodies.max() > 512, "a list long enough to be cut"
+    f.close()
+    rphi, rgrad = oracle.FMM(x, q, 4, 8 if images else 200, images, 1.0, center=(0.5, 0.5, 0.5),
+                             divide_4pi=1).solve(stages="near")
+    tol = 1e-5 if precision else 1e-12  # FP64: a sum of 2000 terms, ~1e-15 each
+    assert l2(grad, rgrad) < tol and l2(phi, rphi) < tol
