@@ -55,7 +55,7 @@ enum Stage { ST_PREP = 0, ST_P2M, ST_M2M, ST_UP, ST_HAD, ST_DOWN, ST_L2L, ST_L2P
 enum BufId { BUF_QEQ = 0, BUF_PCHK, BUF_LEAF, BUF_LEAF2, BUF_Y, BUF_NUM };
 
 struct ApplyCall {
-  int groups, S, rows_max;
+  int groups, rows_max;
   size_t inrow_off, outrow_off, scale_off, goff_off;  // offsets into the index / scale pools
   int bsel;        // which operator stack
   int abuf, cbuf;  // BufId of A and C
@@ -65,7 +65,7 @@ struct ApplyCall {
   int nsum = 0;
 };
 
-// Operator stacks, each in the [s][j][n] layout of k_apply_f64:
+// Operator stacks, each in the [j][n] layout of k_apply_f64_tc:
 //   P2M  (p2m_precompute, kernel.cpp:369-370): y = U^T p, q = scale * V S^-1 y
 //   L2P  (l2p_precompute, kernel.cpp:1465-1467): y = V^T p, q = scale * U S^-1 y
 //   M2M per octant (transposed), L2L = M2M^T per octant, image sum / image 13
@@ -568,12 +568,11 @@ void build_pass_tables(rtfmm_fmm* f) {
   // batched operator applications
   f->idx_pool.clear();
   f->scale_pool.clear();
-  auto add_call = [&](std::vector<ApplyCall>& dst, int S, const std::vector<std::vector<int>>& in_by_group,
+  auto add_call = [&](std::vector<ApplyCall>& dst, const std::vector<std::vector<int>>& in_by_group,
                       const std::vector<std::vector<int>>& out_by_group, const std::vector<double>* scale,
                       int bsel, int abuf, int cbuf, int beta) {
     ApplyCall ac;
     ac.groups = (int)out_by_group.size();
-    ac.S = S;
     ac.rows_max = 0;
     ac.bsel = bsel;
     ac.abuf = abuf;
@@ -610,10 +609,10 @@ void build_pass_tables(rtfmm_fmm* f) {
     }
     std::vector<int> lid(f->leaves_own.size());
     for (int l = 0; l < (int)lid.size(); ++l) lid[l] = l;
-    add_call(f->p2m_call, 1, {lid}, {lid}, nullptr, B_P2M1, BUF_LEAF, BUF_LEAF2, 0);
-    add_call(f->p2m_call, 1, {lid}, {out}, &sc, B_P2M2, BUF_LEAF2, BUF_QEQ, 0);
-    add_call(f->l2p_call, 1, {out}, {lid}, nullptr, B_L2P1, BUF_PCHK, BUF_LEAF, 0);
-    add_call(f->l2p_call, 1, {lid}, {lid}, &sc, B_L2P2, BUF_LEAF, BUF_LEAF2, 0);
+    add_call(f->p2m_call, {lid}, {lid}, nullptr, B_P2M1, BUF_LEAF, BUF_LEAF2, 0);
+    add_call(f->p2m_call, {lid}, {out}, &sc, B_P2M2, BUF_LEAF2, BUF_QEQ, 0);
+    add_call(f->l2p_call, {out}, {lid}, nullptr, B_L2P1, BUF_PCHK, BUF_LEAF, 0);
+    add_call(f->l2p_call, {lid}, {lid}, &sc, B_L2P2, BUF_LEAF, BUF_LEAF2, 0);
   }
   // the non-leaf cells of each depth, in cell order
   std::vector<std::vector<int>> by_depth(p.dmax - p.dmin + 1);
@@ -643,12 +642,12 @@ void build_pass_tables(rtfmm_fmm* f) {
       }
     }
     if (depth >= 0 && !sums.empty()) {
-      add_call(f->m2m_calls, 1, in, out, nullptr, B_M2MT, BUF_QEQ, BUF_Y, 0);
+      add_call(f->m2m_calls, in, out, nullptr, B_M2MT, BUF_QEQ, BUF_Y, 0);
       f->m2m_calls.back().sum_off = f->idx_pool.size();
       f->m2m_calls.back().nsum = (int)sums.size() / 3;
       f->idx_pool.insert(f->idx_pool.end(), sums.begin(), sums.end());
     } else if (depth < 0 && !out1.empty()) {
-      add_call(f->m2m_calls, 1, {in1}, {out1}, nullptr, B_IMGSUMT, BUF_QEQ, BUF_QEQ, 0);
+      add_call(f->m2m_calls, {in1}, {out1}, nullptr, B_IMGSUMT, BUF_QEQ, BUF_QEQ, 0);
     }
   }
   // L2L top-down (fmm.cpp:195-229): depth = dmin .. dmax-1
@@ -672,9 +671,9 @@ void build_pass_tables(rtfmm_fmm* f) {
     if (depth >= 0) {
       bool any = false;
       for (auto& g : out) any |= !g.empty();
-      if (any) add_call(f->l2l_calls, 1, in, out, nullptr, B_M2M, BUF_PCHK, BUF_PCHK, 1);
+      if (any) add_call(f->l2l_calls, in, out, nullptr, B_M2M, BUF_PCHK, BUF_PCHK, 1);
     } else if (!out1.empty()) {
-      add_call(f->l2l_calls, 1, {in1}, {out1}, nullptr, B_IMG13, BUF_PCHK, BUF_PCHK, 1);
+      add_call(f->l2l_calls, {in1}, {out1}, nullptr, B_IMG13, BUF_PCHK, BUF_PCHK, 1);
     }
   }
 
@@ -815,7 +814,7 @@ int upload_operators(rtfmm_fmm* f) {
     tw[2 * m + 1] = -std::sin(2.0 * M_PI * m / o.N);
   }
   RC(dupload(f, &f->d_twiddle, tw));
-  // operator stacks in the [s][j][n] layout of k_apply_f64
+  // operator stacks in the [j][n] layout of k_apply_f64_tc
   const size_t nn = (size_t)ns * ns;
   std::vector<double> b;
   b = o.U;  // y[n] = sum_j U^T[n][j] p[j]
@@ -1044,7 +1043,6 @@ int run_apply(rtfmm_fmm* f, const ApplyCall& c, bool adjoint = false) {
   if (adjoint && bsel == B_IMG13) bsel = B_ADJ_IMG_DOWN;
   b.B = f->d_B[bsel];
   b.groups = c.groups;
-  b.S = c.S;
   b.ns = f->ops.ns;
   b.beta = c.beta;
   b.max_rows = c.rows_max;

@@ -8,7 +8,7 @@
 //     hadamard_8x8 / 1x27 (kernel.cpp:1012-1138)          k_m2l_hadamard27, k_m2l_down
 //   l2l_precompute / img  (kernel.cpp:1419-1435)          k_apply_f64_tc per level
 //   l2p_precompute        (kernel.cpp:1458-1511)          k_apply_f64_tc + k_l2p_eval
-// (k_apply_f64 is the SIMT form of the operator GEMM, built with APPLY_TC=0.)
+// (k_apply_f64_small is the operator GEMM in small tiles.)
 // The adjoint adds k_swap_charges, k_restore_charges, k_adj_combine; the
 // device-buffer forward k_set_charges.
 //   dipole_correction, scale_bodies, sort_bodies_by_idx
@@ -75,18 +75,6 @@
 // FP32 Hadamard: packed FP32x2 FMAs (1) or scalar FMAs (0)
 #ifndef HAD_F2
 #define HAD_F2 1
-#endif
-// FP64 operator application: output rows per block (64 or 128), FP64
-// tensor-core (mma.sync) inner product
-#ifndef APPLY_TM
-#define APPLY_TM 64
-#endif
-#ifndef APPLY_MMA
-#define APPLY_MMA 0
-#endif
-// FP64 operator application on the cp.async + mma.sync kernel
-#ifndef APPLY_TC
-#define APPLY_TC 1
 #endif
 
 namespace rtfmm_b200 {
@@ -778,158 +766,8 @@ __global__ void __launch_bounds__(kSurfThreads)
 
 // ---------------------------------------------------------------------------
 // Batched FP64 operator application:
-//   C[outrow[r]][n] = beta*C + scale[r] * sum_s sum_j A[inrow[r*S+s]][j] B[g][s][j][n]
-// 128x64 output tiles, 16-deep K steps, 8x4 outputs per thread; the next K
-// step's A rows (gathered through inrow) and B panel are loaded into
-// registers while the current step is multiplied out of shared memory.
-// ---------------------------------------------------------------------------
-constexpr int kTM = APPLY_TM, kTN = 64, kTK = 16;
-constexpr int kRPT = kTM / 16;  // output rows per thread
-
-__global__ void __launch_bounds__(256, 2) k_apply_f64(ApplyBatch b) {
-  __shared__ double As[kTK][kTM + 1];
-  __shared__ double Bs[kTK][kTN];
-  const int g = blockIdx.z;
-  const int rbeg = b.group_off[g], rend = b.group_off[g + 1];
-  const int r0 = rbeg + blockIdx.y * kTM;
-  const int c0 = blockIdx.x * kTN;
-  if (r0 >= rend) return;  // block-uniform
-  const int ns = b.ns, S = b.S;
-  const double* Bg = b.B + (size_t)g * S * ns * ns;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int nkt = (ns + kTK - 1) / kTK, total = S * nkt;
-  // this thread loads A rows ty + 16u (the rows it also writes) at k = tx,
-  // and B elements tid + 256u of the 16x64 panel
-  int src[kRPT];
-  double ra[kRPT], rb[4];
-  int s_cur = 0;
-  auto load_src = [&](int s) {
-#pragma unroll
-    for (int u = 0; u < kRPT; ++u) {
-      const int row = r0 + ty + 16 * u;
-      src[u] = row < rend ? b.inrow[(size_t)row * S + s] : -1;
-    }
-  };
-  auto fetch = [&](int kt) {
-    const int s = kt / nkt, j0 = (kt - s * nkt) * kTK;
-    const int j = j0 + tx;
-#pragma unroll
-    for (int u = 0; u < kRPT; ++u) ra[u] = (src[u] >= 0 && j < ns) ? b.A[(size_t)src[u] * ns + j] : 0.0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e = tid + 256 * u;
-      const int jj = j0 + (e >> 6), n = c0 + (e & 63);
-      rb[u] = (jj < ns && n < ns) ? Bg[((size_t)s * ns + jj) * ns + n] : 0.0;
-    }
-  };
-#if APPLY_MMA
-  static_assert(kTM == 64, "the tensor-core path tiles 64 rows as 2 x 4 warps");
-  const int lane = tid & 31, wm = (tid >> 5) & 1, wn = tid >> 6;
-  double dacc[4][2][2];
-#pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) dacc[mt][nt][0] = dacc[mt][nt][1] = 0.0;
-#else
-  double acc[kRPT][4];
-#pragma unroll
-  for (int i = 0; i < kRPT; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-#endif
-  load_src(0);
-  fetch(0);
-  for (int kt = 0; kt < total; ++kt) {
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < kRPT; ++u) As[tx][ty + 16 * u] = ra[u];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e = tid + 256 * u;
-      Bs[e >> 6][e & 63] = rb[u];
-    }
-    __syncthreads();
-    if (kt + 1 < total) {
-      const int s_next = (kt + 1) / nkt;
-      if (s_next != s_cur) {
-        s_cur = s_next;
-        load_src(s_next);
-      }
-      fetch(kt + 1);
-    }
-#if APPLY_MMA
-    // FP64 tensor-core steps: mma.sync m8n8k4 over this warp's 32x16 block
-    // (4 x 2 tiles of 8x8).  Fragments: A[m][k] at m = lane/4, k = lane%4;
-    // B[k][n] at k = lane%4, n = lane/4; D[m][n] at m = lane/4,
-    // n = 2 (lane%4) + {0, 1}.
-#pragma unroll
-    for (int k4 = 0; k4 < kTK; k4 += 4) {
-      double fa[4], fb[2];
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt) fa[mt] = As[k4 + (lane & 3)][wm * 32 + mt * 8 + (lane >> 2)];
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) fb[nt] = Bs[k4 + (lane & 3)][wn * 16 + nt * 8 + (lane >> 2)];
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-          asm volatile(
-              "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-              : "+d"(dacc[mt][nt][0]), "+d"(dacc[mt][nt][1])
-              : "d"(fa[mt]), "d"(fb[nt]));
-    }
-  }
-#pragma unroll
-  for (int mt = 0; mt < 4; ++mt) {
-    const int row = r0 + wm * 32 + mt * 8 + (lane >> 2);
-    if (row >= rend) continue;
-    const int o = b.outrow[row];
-    const double sc = b.scale ? b.scale[row] : 1.0;
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int n = c0 + wn * 16 + nt * 8 + 2 * (lane & 3) + i;
-        if (n >= ns) continue;
-        double* cp = b.C + (size_t)o * ns + n;
-        *cp = b.beta ? *cp + sc * dacc[mt][nt][i] : sc * dacc[mt][nt][i];
-      }
-  }
-}
-#else
-#pragma unroll
-    for (int k = 0; k < kTK; ++k) {
-      double a[kRPT], bb[4];
-#pragma unroll
-      for (int i = 0; i < kRPT; ++i) a[i] = As[k][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bb[j] = Bs[k][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < kRPT; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < kRPT; ++i) {
-    const int row = r0 + ty + 16 * i;
-    if (row >= rend) continue;
-    const int o = b.outrow[row];
-    const double sc = b.scale ? b.scale[row] : 1.0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = c0 + tx + 16 * j;
-      if (n >= ns) continue;
-      double* cp = b.C + (size_t)o * ns + n;
-      *cp = b.beta ? *cp + sc * acc[i][j] : sc * acc[i][j];
-    }
-  }
-}
-#endif
-
-// ---------------------------------------------------------------------------
-// The same batched application on the FP64 tensor path: 64x64 output tiles
-// per 128-thread block (2 x 2 warps of 32x32, each 4 x 4 mma.sync m8n8k4
+//   C[outrow[r]][n] = beta*C + scale[r] * sum_j A[inrow[r]][j] B[g][j][n]
+// on the FP64 tensor path: 64x64 output tiles per 128-thread block (2 x 2 warps of 32x32, each 4 x 4 mma.sync m8n8k4
 // f64 tiles), A rows (gathered through inrow) and the B panel moved into
 // shared memory by cp.async through a three-stage ring, so that the loads of
 // K step t+2 are in flight while step t is multiplied.  Products and sums
@@ -968,25 +806,21 @@ __global__ void __launch_bounds__(kGThreads) k_apply_f64_tc(ApplyBatch b) {
   const int r0 = rbeg + blockIdx.y * kGM;
   const int c0 = blockIdx.x * kGN;
   if (r0 >= rend) return;  // block-uniform
-  const int ns = b.ns, S = b.S;
-  const double* Bg = b.B + (size_t)g * S * ns * ns;
+  const int ns = b.ns;
+  const double* Bg = b.B + (size_t)g * ns * ns;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp & 1, wn = warp >> 1;
-  const int nkt = (ns + kGK - 1) / kGK, total = S * nkt;
+  const int total = (ns + kGK - 1) / kGK;
   // copies of this thread: A chunk e = tid + 128u -> row e/8, doubles 2(e%8)..+1;
   // B chunk e -> K row e/32, columns 2(e%32)..+1
   int srow[4];
-  int s_cur = -1;
-  auto issue = [&](int kt) {
-    const int s = kt / nkt, j0 = (kt - s * nkt) * kGK;
-    if (s != s_cur) {
-      s_cur = s;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int row = r0 + ((tid + kGThreads * u) >> 3);
-        srow[u] = row < rend ? b.inrow[(size_t)row * S + s] : -1;
-      }
-    }
+  for (int u = 0; u < 4; ++u) {
+    const int row = r0 + ((tid + kGThreads * u) >> 3);
+    srow[u] = row < rend ? b.inrow[row] : -1;
+  }
+  auto issue = [&](int kt) {
+    const int j0 = kt * kGK;
     double* as = As + (kt % kGStages) * kAStage;
     double* bs = Bs + (kt % kGStages) * kBStage;
 #pragma unroll
@@ -1001,7 +835,7 @@ __global__ void __launch_bounds__(kGThreads) k_apply_f64_tc(ApplyBatch b) {
       const int e = tid + kGThreads * u;
       const int kr = e >> 5, ch = e & 31, jj = j0 + kr, n = c0 + 2 * ch;
       const bool ok = jj < ns && n < ns;
-      cp_async16(bs + kr * kBPitch + 2 * ch, ok ? Bg + ((size_t)s * ns + jj) * ns + n : Bg, ok);
+      cp_async16(bs + kr * kBPitch + 2 * ch, ok ? Bg + (size_t)jj * ns + n : Bg, ok);
     }
   };
   double acc[4][4][2];
@@ -1055,6 +889,100 @@ __global__ void __launch_bounds__(kGThreads) k_apply_f64_tc(ApplyBatch b) {
       }
       *cp = v;
     }
+  }
+}
+
+// The same product in 16 x 32 tiles, for batches that leave the 64 x 64 tiles
+// on a few SMs (the upper tree levels, the image levels with one row, small
+// body sets): a 64 x 64 tile alone takes ns/16 steps of 1024 tensor cycles on
+// one SM whatever its rows hold (5 us at ns = 152, 17 us at ns = 488), a
+// 16 x 32 tile a sixteenth of the cycles and a chain of ns/4 dependent mma.
+// Each output sums its products in the same order as above, so the choice of
+// the tile does not change a result.
+constexpr int kSM = 16, kSN = 32, kSK = 32, kSStages = 4;
+constexpr int kSAPitch = kSK + 4, kSBPitch = kSN + 4;
+constexpr int kSAStage = kSM * kSAPitch, kSBStage = kSK * kSBPitch;
+#ifndef APPLY_SMALL
+#define APPLY_SMALL 296
+#endif
+constexpr int kApplySmallBelow = APPLY_SMALL;
+constexpr size_t kSSmem = sizeof(double) * kSStages * (kSAStage + kSBStage);
+
+__global__ void __launch_bounds__(128) k_apply_f64_small(ApplyBatch b) {
+  extern __shared__ __align__(16) double gsm[];
+  double* As = gsm;
+  double* Bs = gsm + kSStages * kSAStage;
+  const int g = blockIdx.z;
+  const int rbeg = b.group_off[g], rend = b.group_off[g + 1];
+  const int r0 = rbeg + blockIdx.y * kSM;
+  const int c0 = blockIdx.x * kSN;
+  if (r0 >= rend) return;  // block-uniform
+  const int ns = b.ns;
+  const double* Bg = b.B + (size_t)g * ns * ns;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = warp & 1, wn = warp >> 1;
+  const int total = (ns + kSK - 1) / kSK;
+  // copies of this thread: A chunks tid, tid + 128 -> row e/16, doubles
+  // 2(e%16)..+1; B chunks tid + 128u -> K row e/16, columns 2(e%16)..+1
+  int srow[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int row = r0 + ((tid + 128 * u) >> 4);
+    srow[u] = row < rend ? b.inrow[row] : -1;
+  }
+  const int ch = 2 * (tid & 15);
+  auto issue = [&](int kt) {
+    const int j0 = kt * kSK;
+    double* as = As + (kt % kSStages) * kSAStage;
+    double* bs = Bs + (kt % kSStages) * kSBStage;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int kr = (tid + 128 * u) >> 4, jj = j0 + kr, n = c0 + ch;
+      const bool ok = jj < ns && n < ns;
+      cp_async16(bs + kr * kSBPitch + ch, ok ? Bg + (size_t)jj * ns + n : Bg, ok);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int j = j0 + ch;
+      const bool ok = srow[u] >= 0 && j < ns;
+      cp_async16(as + ((tid + 128 * u) >> 4) * kSAPitch + ch, ok ? b.A + (size_t)srow[u] * ns + j : b.A, ok);
+    }
+  };
+  double acc[2][2] = {};
+#pragma unroll
+  for (int st = 0; st < kSStages - 1; ++st) {
+    if (st < total) issue(st);
+    cp_async_commit();
+  }
+  for (int kt = 0; kt < total; ++kt) {
+    cp_async_wait<kSStages - 2>();
+    __syncthreads();  // step kt is in shared memory; step kt-1's buffer is free
+    if (kt + kSStages - 1 < total) issue(kt + kSStages - 1);
+    cp_async_commit();
+    const double* as = As + (kt % kSStages) * kSAStage + (wm * 8 + (lane >> 2)) * kSAPitch + (lane & 3);
+    const double* bs = Bs + (kt % kSStages) * kSBStage + (lane & 3) * kSBPitch + wn * 16 + (lane >> 2);
+#pragma unroll
+    for (int k4 = 0; k4 < kSK; k4 += 4)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) dmma8x8x4(acc[nt], as[k4], bs[k4 * kSBPitch + nt * 8]);
+  }
+  cp_async_wait<0>();
+  const int row = r0 + wm * 8 + (lane >> 2);
+  if (row >= rend) return;
+  const int o = b.outrow[row];
+  const double sc = b.scale ? b.scale[row] : 1.0;
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt) {
+    const int n = c0 + wn * 16 + nt * 8 + 2 * (lane & 3);
+    if (n >= ns) continue;
+    double2* cp = reinterpret_cast<double2*>(b.C + (size_t)o * ns + n);
+    double2 v = make_double2(sc * acc[nt][0], sc * acc[nt][1]);
+    if (b.beta) {
+      const double2 c = *cp;
+      v.x += c.x;
+      v.y += c.y;
+    }
+    *cp = v;
   }
 }
 
@@ -2175,7 +2103,6 @@ cudaError_t launch_l2p_eval(const double4* body64, const LeafInfo* leaves, int n
 
 cudaError_t launch_apply(const ApplyBatch& b, cudaStream_t st) {
   if (b.max_rows > 0 && b.groups > 0) {
-#if APPLY_TC
     if (b.ns % 2 != 0) return cudaErrorInvalidValue;  // 16-byte copies need an even ns
     // the shared-memory opt-in is per function and device; set once per
     // device, safely when several host threads make their first call at once
@@ -2185,15 +2112,24 @@ cudaError_t launch_apply(const ApplyBatch& b, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
       e = cudaFuncSetAttribute(k_apply_f64_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGSmem);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_apply_f64_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSSmem);
       if (e != cudaSuccess) return e;
       if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    dim3 grid(cdiv(b.ns, kGN), cdiv(b.max_rows, kGM), b.groups);
-    k_apply_f64_tc<<<grid, kGThreads, kGSmem, st>>>(b);
-#else
-    dim3 grid(cdiv(b.ns, kTN), cdiv(b.max_rows, kTM), b.groups);
-    k_apply_f64<<<grid, 256, 0, st>>>(b);
-#endif
+    // small tiles while there are fewer large ones than two an SM: the chip is
+    // then part idle, and a large tile's ns/16 steps are the kernel's length.
+    // M2M + L2L of 8192 bodies at P = 6: 0.174 ms in large tiles, 0.084 here;
+    // of 2^20 at P = 8: 0.639 and 0.455; with the line at one large tile an SM
+    // 0.127 against 0.119 (200003 bodies, P = 6), at four the same as at two.
+    const int64_t large = (int64_t)cdiv(b.ns, kGN) * cdiv(b.max_rows, kGM) * b.groups;
+    if (large < kApplySmallBelow) {
+      dim3 grid(cdiv(b.ns, kSN), cdiv(b.max_rows, kSM), b.groups);
+      k_apply_f64_small<<<grid, 128, kSSmem, st>>>(b);
+    } else {
+      dim3 grid(cdiv(b.ns, kGN), cdiv(b.max_rows, kGM), b.groups);
+      k_apply_f64_tc<<<grid, kGThreads, kGSmem, st>>>(b);
+    }
   }
   return cudaGetLastError();
 }

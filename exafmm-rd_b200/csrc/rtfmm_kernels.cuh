@@ -59,16 +59,16 @@ struct P2PSrc64 {
   int boff, bnum;     // source bodies (tree order)
 };
 
-// Batched FP64 operator application (see k_apply_f64).
+// Batched FP64 operator application (see k_apply_f64_tc).
 struct ApplyBatch {
   const double* A;      // input vectors, row stride ns
-  const int* inrow;     // rows*S input row indices (-1 = zero vector)
-  const double* B;      // groups x S x ns x ns operator stack, row-major [s][j][n]
+  const int* inrow;     // input row indices (-1 = zero vector)
+  const double* B;      // groups x ns x ns operator stack, row-major [j][n]
   const int* outrow;    // output row indices
   const double* scale;  // per-row scale (nullptr = 1)
   const int* group_off; // groups+1 row offsets
   double* C;            // output vectors, row stride ns
-  int groups, S, ns, beta;
+  int groups, ns, beta;
   int max_rows;         // rows of the largest group (grid sizing)
 };
 

@@ -152,7 +152,6 @@ extern "C" int rtfmm_b200_p2m_noalloc(int P, int64_t nleaf, const rtfmm_leaf* d_
     return fail(RTFMM_ECUDA, "p2m_noalloc: check-surface launch failed");
   ApplyBatch b;
   b.groups = 1;
-  b.S = 1;
   b.ns = ns;
   b.beta = 0;
   b.max_rows = nl;
