@@ -1121,7 +1121,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
   if (far && phase == 0) CK(cudaMemsetAsync(f->d_pchk, 0, sizeof(double) * p.cells.size() * ns, s0));
   if (far && up) {
     CK(launch_p2m_check(f->d_body64, f->d_leaves_own, nleaf, f->d_surf_unit, ns, f->d_leafvec, s0,
-                        mixed ? 1 : 2));
+                        !mixed));
     f->launches++;
     for (auto& c : f->p2m_call) {
       int rc = run_apply(f, c);
@@ -1194,7 +1194,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
       if (rc) return rc;
     }
     CK(launch_l2p_eval(f->d_body64, f->d_leaves_own, nleaf, f->d_surf_unit, ns, f->d_leafvec2, f->d_far_phi,
-                       f->d_far_grad, s0, mixed ? 1 : 2));
+                       f->d_far_grad, s0, !mixed));
     f->launches++;
     CK(cudaEventRecord(f->ev_st[ST_L2P], s0));
   } else {

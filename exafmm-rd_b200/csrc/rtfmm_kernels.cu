@@ -24,11 +24,6 @@
 
 #include <cub/cub.cuh>
 
-// FP64 pair kernels: seed the reciprocal square root with the FP64 (1) or
-// FP32 (0) hardware approximation
-#ifndef RSQ_SEED64
-#define RSQ_SEED64 1
-#endif
 // FP32 P2P: inner unroll and resident blocks per SM.  A block is one warp
 // (P2P_WARPS): work items differ in cost several-fold, and a block of four
 // held the slots of its finished warps until its slowest one was done
@@ -120,27 +115,38 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   return y;
 }
 
-// 1/sqrt(x) in FP64 by Newton-Raphson, y <- y (3/2 - x y^2 / 2), from a
-// hardware seed.  The PTX FP64 approximation (rsqrt.approx.ftz.f64, one
-// special-function op) is good to 9.1e-7 relative; one step gives 1.3e-12 and
-// two give 3.3e-16 (maxima measured against CUDA's rsqrt over 1e-30..1e30).
-// The FP32 approximation (1.5e-7, but two conversions on the same pipe as the
-// seed) gives 3.2e-14 and 3.3e-16, for arguments in the normal FP32 range.
-// x must be positive and normal (pairs closer than 1e-154 are not supported).
-template <int NR>
-__device__ __forceinline__ double rsqrt_nr(double x) {
-#if RSQ_SEED64
+// 1/sqrt(x) in FP64 from the hardware seed (one special-function op, 9.1e-7
+// relative), and zero for x = 0; other x must be normal (pairs closer than
+// 1e-154 are not supported).  The zero is made by the seed's words on the
+// integer pipe: a comparison would take the FP64 pipe, which bounds every
+// kernel that calls this.
+__device__ __forceinline__ double rsqrt_seed(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-#else
-  const float xf = (float)x;
-  if (!(xf >= 1.2e-38f && xf <= 3.0e38f)) return rsqrt(x);
-  double y = (double)rsqrt_approx(xf);
-#endif
-  const double h = 0.5 * x;
-#pragma unroll
-  for (int i = 0; i < NR; ++i) y = y * fma(-h * y, y, 1.5);
-  return y;
+  const int hi = __double2hiint(x);
+  return __hiloint2double(hi ? __double2hiint(y) : 0, hi ? __double2loint(y) : 0);
+}
+// To full precision: with e = 1 - x y^2 the Taylor series of (1 - e)^(-1/2) to
+// second order, y (1 + e/2 + 3 e^2/8) (Householder's method of third order;
+// the remainder 5/16 e^3 is 2e-18): five operations, where two Newton steps
+// take seven.
+__device__ __forceinline__ double rsqrt_or_zero(double x) {
+  const double y = rsqrt_seed(x);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+// Twice 1/sqrt(x) to 1.3e-12 (maximum against CUDA's rsqrt over 1e-30..1e30):
+// one Newton step y (3 - x y^2), whose factor 1/2 the callers put into the
+// charges, three operations instead of four.
+__device__ __forceinline__ double rsqrt_twice(double x) {
+  const double y = rsqrt_seed(x);
+  return y * fma(-(x * y), y, 3.0);
+}
+// What the surface kernels use: FULL 1/sqrt(x), else 2/sqrt(x) with charges
+// halved (kHalf, exact).
+template <bool FULL>
+__device__ __forceinline__ double rsqrt_surf(double x) {
+  return FULL ? rsqrt_or_zero(x) : rsqrt_twice(x);
 }
 
 // ---------------------------------------------------------------------------
@@ -410,21 +416,6 @@ __global__ void __launch_bounds__(32 * kP2PWarps, P2P_MINB)
   }
 }
 
-// 1/sqrt(x) in FP64 for the FP64 P2P: from the hardware seed y (9.1e-7
-// relative), with e = 1 - x y^2 the Taylor series of (1 - e)^(-1/2) to second
-// order, y (1 + e/2 + 3 e^2/8) (Householder's method of third order; the
-// remainder 5/16 e^3 is 2e-18), five operations.  Zero for x = 0, by the high
-// word on the integer pipe instead of a comparison on the FP64 pipe, which is
-// what bounds the kernel; other x must be normal.
-__device__ __forceinline__ double rsqrt_or_zero(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const int hi = __double2hiint(x);
-  y = __hiloint2double(hi ? __double2hiint(y) : 0, hi ? __double2loint(y) : 0);
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // FP64 P2P, the same work items; per pair the reference's arithmetic
 // (dx = x_t - (x_s + offset), kernel.cpp:283-290) in FP64, 18 operations.
 template <int G>
@@ -625,7 +616,7 @@ __global__ void k_close_fix(const double4* __restrict__ body64, const float4* __
       ez -= cycle * rint(ez / cycle);
     }
     const double rr = ex * ex + ey * ey + ez * ez;
-    const double jr = rr > 0.0 ? rsqrt_nr<2>(rr) : 0.0;
+    const double jr = rsqrt_or_zero(rr);
     const double qjr = y.w * jr;
     const double q3d = qjr * jr * jr;
     P += qjr - (double)qir;
@@ -649,7 +640,7 @@ constexpr int kSurfThreads = 128;
 constexpr int kCheckMaxThreads = 256;
 constexpr int kCheckPer = 2;
 
-template <int NR>
+template <bool FULL>
 __global__ void __launch_bounds__(kCheckMaxThreads)
     k_p2m_check(const double4* __restrict__ body64, const LeafInfo* __restrict__ leaves,
                 const double* __restrict__ surf_unit, int ns, double* __restrict__ out) {
@@ -671,7 +662,11 @@ __global__ void __launch_bounds__(kCheckMaxThreads)
     for (int b0 = 0; b0 < L.bnum; b0 += nt) {
       const int cnt = min(nt, L.bnum - b0);
       __syncthreads();
-      if (tid < cnt) sb[tid] = body64[L.boff + b0 + tid];
+      if (tid < cnt) {
+        double4 b = body64[L.boff + b0 + tid];
+        if (!FULL) b.w *= 0.5;
+        sb[tid] = b;
+      }
       __syncthreads();
 #pragma unroll 2
       for (int j = 0; j < cnt; ++j) {
@@ -679,9 +674,7 @@ __global__ void __launch_bounds__(kCheckMaxThreads)
 #pragma unroll
         for (int k = 0; k < kCheckPer; ++k) {
           const double dx = yx[k] - b.x, dy = yy[k] - b.y, dz = yz[k] - b.z;
-          const double r2 = dx * dx + dy * dy + dz * dz;
-          const double ir = r2 > 0.0 ? rsqrt_nr<NR>(r2) : 0.0;
-          acc[k] += b.w * ir;
+          acc[k] += b.w * rsqrt_surf<FULL>(dx * dx + dy * dy + dz * dz);
         }
       }
     }
@@ -701,7 +694,7 @@ __global__ void __launch_bounds__(kCheckMaxThreads)
 // takes points g, g+G, ...) and sums the groups in shared memory, so that a
 // 34-body leaf keeps 102 of 128 threads busy instead of 34.
 // ---------------------------------------------------------------------------
-template <int NR>
+template <bool FULL>
 __global__ void __launch_bounds__(kSurfThreads)
     k_l2p_eval(const double4* __restrict__ body64, const LeafInfo* __restrict__ leaves,
                const double* __restrict__ surf_unit, int ns, const double* __restrict__ q_down,
@@ -712,7 +705,7 @@ __global__ void __launch_bounds__(kSurfThreads)
   const double R = L.r * 2.95;
   for (int i = threadIdx.x; i < ns; i += blockDim.x)
     sy[i] = make_double4(surf_unit[3 * i] * R + L.cx, surf_unit[3 * i + 1] * R + L.cy,
-                         surf_unit[3 * i + 2] * R + L.cz, q_down[(size_t)blockIdx.x * ns + i]);
+                         surf_unit[3 * i + 2] * R + L.cz, (FULL ? 1.0 : 0.5) * q_down[(size_t)blockIdx.x * ns + i]);
   __syncthreads();
   const int bnum = L.bnum;
   if (bnum <= 0) return;  // block-uniform
@@ -727,8 +720,7 @@ __global__ void __launch_bounds__(kSurfThreads)
       for (int i = grp; i < ns; i += G) {
         const double4 y = sy[i];
         const double dx = x.x - y.x, dy = x.y - y.y, dz = x.z - y.z;
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        const double ir = r2 > 0.0 ? rsqrt_nr<NR>(r2) : 0.0;
+        const double ir = rsqrt_surf<FULL>(dx * dx + dy * dy + dz * dz);
         const double qir = y.w * ir;
         p += qir;
         const double q3 = qir * ir * ir;
@@ -756,10 +748,11 @@ __global__ void __launch_bounds__(kSurfThreads)
     }
     if (grp == 0 && t < bnum) {
       const int b = L.boff + t;
+      const double sg = FULL ? -1.0 : -0.25;  // (2/r)^3 against halved charges
       phi[b] = p;
-      grad[3 * b + 0] = -gx;
-      grad[3 * b + 1] = -gy;
-      grad[3 * b + 2] = -gz;
+      grad[3 * b + 0] = sg * gx;
+      grad[3 * b + 1] = sg * gy;
+      grad[3 * b + 2] = sg * gz;
     }
   }
 }
@@ -2069,36 +2062,36 @@ cudaError_t launch_count_scan(const int* cnt, int* off, int n, void* tmp, size_t
 }
 
 cudaError_t launch_p2m_check(const double4* body64, const LeafInfo* leaves, int nleaf,
-                             const double* surf_unit, int ns, double* out, cudaStream_t st, int newton) {
+                             const double* surf_unit, int ns, double* out, cudaStream_t st, bool full) {
   if (nleaf > 0) {
     const int per = cdiv(ns, kCheckPer);
     const int nt = per >= kCheckMaxThreads ? kCheckMaxThreads : cdiv(per, 32) * 32;
-    if (newton == 1)
-      k_p2m_check<1><<<nleaf, nt, 0, st>>>(body64, leaves, surf_unit, ns, out);
+    if (full)
+      k_p2m_check<true><<<nleaf, nt, 0, st>>>(body64, leaves, surf_unit, ns, out);
     else
-      k_p2m_check<2><<<nleaf, nt, 0, st>>>(body64, leaves, surf_unit, ns, out);
+      k_p2m_check<false><<<nleaf, nt, 0, st>>>(body64, leaves, surf_unit, ns, out);
   }
   return cudaGetLastError();
 }
 
-template <int NR>
-static cudaError_t l2p_nr(const double4* body64, const LeafInfo* leaves, int nleaf, const double* surf_unit, int ns,
+template <bool FULL>
+static cudaError_t l2p_eval(const double4* body64, const LeafInfo* leaves, int nleaf, const double* surf_unit, int ns,
                           const double* q_down, double* phi, double* grad, cudaStream_t st) {
   const size_t sm = sizeof(double4) * ns;
   if (sm > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_l2p_eval<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = cudaFuncSetAttribute(k_l2p_eval<FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
   }
-  k_l2p_eval<NR><<<nleaf, kSurfThreads, sm, st>>>(body64, leaves, surf_unit, ns, q_down, phi, grad);
+  k_l2p_eval<FULL><<<nleaf, kSurfThreads, sm, st>>>(body64, leaves, surf_unit, ns, q_down, phi, grad);
   return cudaGetLastError();
 }
 
 cudaError_t launch_l2p_eval(const double4* body64, const LeafInfo* leaves, int nleaf,
                             const double* surf_unit, int ns, const double* q_down, double* phi,
-                            double* grad, cudaStream_t st, int newton) {
+                            double* grad, cudaStream_t st, bool full) {
   if (nleaf <= 0) return cudaGetLastError();
-  return newton == 1 ? l2p_nr<1>(body64, leaves, nleaf, surf_unit, ns, q_down, phi, grad, st)
-                     : l2p_nr<2>(body64, leaves, nleaf, surf_unit, ns, q_down, phi, grad, st);
+  return full ? l2p_eval<true>(body64, leaves, nleaf, surf_unit, ns, q_down, phi, grad, st)
+              : l2p_eval<false>(body64, leaves, nleaf, surf_unit, ns, q_down, phi, grad, st);
 }
 
 cudaError_t launch_apply(const ApplyBatch& b, cudaStream_t st) {

@@ -100,10 +100,9 @@ cudaError_t launch_close_fix(const double4* body64, const float4* body32, const 
 // off = exclusive prefix sum of cnt (n values); tmp == nullptr: *tmp_bytes
 // = the scratch it needs
 cudaError_t launch_count_scan(const int* cnt, int* off, int n, void* tmp, size_t* tmp_bytes, cudaStream_t st);
-// newton: Newton steps of the FP64 reciprocal square root (1: ~1e-13, for
-// the FP32-mixed form; 2: full FP64)
+// full: reciprocal square roots to full precision, else to 1.3e-12 (mixed form)
 cudaError_t launch_p2m_check(const double4* body64, const LeafInfo* leaves, int nleaf,
-                             const double* surf_unit, int ns, double* out, cudaStream_t st, int newton = 2);
+                             const double* surf_unit, int ns, double* out, cudaStream_t st, bool full = true);
 cudaError_t launch_apply(const ApplyBatch& b, cudaStream_t st);
 // q[parent] = sum of Y[child] over the parent's children; `list` holds
 // (parent, coff, cnum) triplets
@@ -137,7 +136,7 @@ cudaError_t launch_m2l_down(const T* Pk, const int* items, const double* tscale,
                             double* p_check, cudaStream_t st);
 cudaError_t launch_l2p_eval(const double4* body64, const LeafInfo* leaves, int nleaf,
                             const double* surf_unit, int ns, const double* q_down, double* phi,
-                            double* grad, cudaStream_t st, int newton = 2);
+                            double* grad, cudaStream_t st, bool full = true);
 // sums of q x, q y, q z and q into partial[4 * kDipoleBlocks + 0..3]; partial
 // holds kDipoleScratch doubles (per-block sums, then the totals)
 constexpr int kDipoleBlocks = 256;
