@@ -21,6 +21,8 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cmath>
+#include <type_traits>
 
 #include <cub/cub.cuh>
 
@@ -39,10 +41,6 @@
 #endif
 #ifndef P2P_FLUSH
 #define P2P_FLUSH 4
-#endif
-// register-blocked FFT-M2L up: resident blocks per SM (FP32; FP64 keeps 2)
-#ifndef UP_RB_MINB
-#define UP_RB_MINB 3
 #endif
 // FP32 Hadamard: targets per thread, directions per FP32 partial sum,
 // resident blocks per SM
@@ -1013,14 +1011,11 @@ __device__ __forceinline__ void cmad(T& re, T& im, T ar, T ai, T br, T bi) {
 // together so that each frequency's sp values are written contiguously into
 // the frequency-major spectrum Q[f][src][slot].
 // items: 10 ints per block = src, first slot, child cell per slot (-1 = none).
-// PP > 0 fixes P at compile time (cheap index arithmetic); PP = 0 takes it
-// from the argument.
-template <typename T, int PP>
+template <typename T>
 __global__ void __launch_bounds__(256)
     k_m2l_up(const double* __restrict__ q_equiv, const int* __restrict__ items,
-             const int* __restrict__ surf_ijk, const double* __restrict__ twiddle, int P_, int ns, int nsrc,
+             const int* __restrict__ surf_ijk, const double* __restrict__ twiddle, int P, int ns, int nsrc,
              int sp, T* __restrict__ Q) {
-  const int P = PP > 0 ? PP : P_;
   extern __shared__ unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
   const int N = 2 * P - 1;
@@ -1108,249 +1103,276 @@ __global__ void __launch_bounds__(256)
 }
 
 // The up and down kernels above with register blocking, for the orders P
-// fixed at compile time: the sp children of a block go through each DFT pass
-// together, and a thread keeps one input line of the pass (the values along
-// the transformed axis) in registers and forms every output of that line, the
-// twiddles read as shared-memory broadcasts.  Each output sums its terms in
-// the same order as k_m2l_up / k_m2l_down, so the results are the same bit
-// for bit; the shared-memory traffic per multiply-add falls from two loads
-// to about one broadcast.
-template <typename T, int PP>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? UP_RB_MINB : 2)
-    k_m2l_up_rb(const double* __restrict__ q_equiv, const int* __restrict__ items, const int* __restrict__ surf_ijk,
-                const double* __restrict__ twiddle, int ns, int nsrc, int sp, T* __restrict__ Q) {
-  constexpr int P = PP, N = 2 * P - 1, P3 = P * P * P, PNP = P * N * P;
-  // the last pass: a thread per (pair of slots, ky, kx, range of kz)
-  constexpr int KC = (128 / (N * P)) < 1 ? 1 : ((128 / (N * P)) > N ? N : 128 / (N * P));
-  constexpr int KH = (N + KC - 1) / KC;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // the twiddle table padded to 8 values, so that A and the cube (read as
-  // 16-byte vectors) start on 16-byte boundaries
-  constexpr int WSZ = (2 * N * N + 7) / 8 * 8;
-  T* W = reinterpret_cast<T*>(smem_raw);  // N*N complex: W[k][n] = w^(k n mod N)
-  T* A = W + WSZ;                         // sp * P^3 complex: [slot][z][y][kx]
-  T* cube = A + 2 * (size_t)sp * P3;      // sp * P^3, read by the first pass only
-  T* Bm = cube;                           // sp * P*N*P complex: [slot][z][ky][kx], after it
-  const int* it = items + 10 * blockIdx.x;
-  const int src = it[0], slot0 = it[1];
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int e = tid; e < N * N; e += nt) {
-    const int m = ((e / N) * (e % N)) % N;
-    W[2 * e] = (T)twiddle[2 * m];
-    W[2 * e + 1] = (T)twiddle[2 * m + 1];
-  }
-  for (int e = tid; e < sp * P3; e += nt) cube[e] = T(0);
-  __syncthreads();
-  for (int e = tid; e < sp * ns; e += nt) {
-    const int j = e / ns, i = e - j * ns;
-    const int child = it[2 + j];
-    if (child < 0) continue;  // an absent child: zero spectra
-    const int x = surf_ijk[3 * i], y = surf_ijk[3 * i + 1], z = surf_ijk[3 * i + 2];
-    cube[(size_t)j * P3 + (z * P + y) * P + x] = (T)q_equiv[(size_t)child * ns + i];
-  }
-  __syncthreads();
-  // x -> kx: a thread per (slot, z, y)
-  for (int e = tid; e < sp * P * P; e += nt) {
-    const int j = e / (P * P), zy = e - j * P * P;
-    const T* row = cube + (size_t)j * P3 + zy * P;
-    T r[P];
-    if constexpr (sizeof(T) == 4 && P % 4 == 0) {
+// fixed at compile time.  A thread takes one line of a pass (the values along
+// the transformed axis) for 16 bytes of child slots (two in FP32, one in
+// FP64) and forms every output of the line in registers.  Frequencies k and
+// N - k share their cosines and sines,
+//   X_k e^(it) + X_(N-k) e^(-it) = (X_k + X_(N-k)) cos t + i (X_k - X_(N-k)) sin t,
+// which halves the multiply-adds of a complex transform, and the twiddles,
+// indexed by constants after unrolling, are operands in the kernel's
+// parameter bank (the form before read each as a shared-memory broadcast, one
+// for two multiply-adds, which bounded it).  Shared memory holds one array
+// [z][ky][kx][slot]; every pass works in place on it, which leaves room for
+// two to seven blocks per SM.  Up and down at N = 2^20, P = 8 (FP32): 0.20 and
+// 0.34 -> 0.12 and 0.14 ms; at P = 10 (FP64, 10^6 bodies in blobs): 1.47 and
+// 2.38 -> 0.84 and 0.78 ms, 60% of the measured HBM rate for the spectra alone.
+template <typename T, int N>
+struct Twiddles {
+  T c[N], s[N];  // cos, sin (2 pi m / N)
+};
+template <typename T>
+struct DftSlots {
+  static constexpr int kPer = 16 / (2 * sizeof(T));  // child slots of a thread
+  static constexpr int kBlock = 2 * kPer;            // child slots of a block: one sector of spectrum
+};
+constexpr int dft_threads(int P) { return (2 * (2 * P - 1) * P + 31) / 32 * 32; }
+constexpr int dft_blocks(int P, int bytes) {  // resident blocks per SM the registers are sized for
+  const int t = dft_threads(P), regs = bytes == 4 ? 64 : P <= 7 ? 80 : 84;
+  return 65536 / (t * regs) < 1 ? 1 : 65536 / (t * regs) > 8 ? 8 : 65536 / (t * regs);
+}
+
+__device__ __forceinline__ void ld_slots(const float* p, float (&re)[2], float (&im)[2]) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  re[0] = v.x;
+  im[0] = v.y;
+  re[1] = v.z;
+  im[1] = v.w;
+}
+__device__ __forceinline__ void ld_slots(const double* p, double (&re)[1], double (&im)[1]) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  re[0] = v.x;
+  im[0] = v.y;
+}
+__device__ __forceinline__ void st_slots(float* p, const float (&re)[2], const float (&im)[2]) {
+  *reinterpret_cast<float4*>(p) = make_float4(re[0], im[0], re[1], im[1]);
+}
+__device__ __forceinline__ void st_slots(double* p, const double (&re)[1], const double (&im)[1]) {
+  *reinterpret_cast<double2*>(p) = make_double2(re[0], im[0]);
+}
+
+// N outputs X_k = sum_y x_y exp(-2 pi i k y / N) of P inputs `in[y * si]`,
+// given to put(k, re, im).
+template <typename T, int P, typename Put>
+__device__ __forceinline__ void dft_forward(const T* in, int si, const Twiddles<T, 2 * P - 1>& tw, Put put) {
+  constexpr int N = 2 * P - 1, U = DftSlots<T>::kPer;
+  T xr[P][U], xi[P][U];
 #pragma unroll
-      for (int x = 0; x < P; x += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(row + x);
-        r[x] = v.x;
-        r[x + 1] = v.y;
-        r[x + 2] = v.z;
-        r[x + 3] = v.w;
-      }
-    } else {
+  for (int y = 0; y < P; ++y) ld_slots(in + y * si, xr[y], xi[y]);
 #pragma unroll
-      for (int x = 0; x < P; ++x) r[x] = row[x];
+  for (int k = 0; k < P; ++k) {
+    T ar[U], ai[U], br[U], bi[U];  // sums of x cos and x sin
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      ar[u] = xr[0][u];
+      ai[u] = xi[0][u];
+      br[u] = bi[u] = T(0);
     }
-    T* a = A + 2 * ((size_t)j * P3 + zy * P);
 #pragma unroll
-    for (int kx = 0; kx < P; ++kx) {
-      const T* wk = W + 2 * kx * N;
-      T re = 0, im = 0;
+    for (int y = 1; y < P; ++y) {
+      const T c = tw.c[(k * y) % N], s = tw.s[(k * y) % N];
 #pragma unroll
-      for (int x = 0; x < P; ++x) {
-        re = fma(r[x], wk[2 * x], re);
-        im = fma(r[x], wk[2 * x + 1], im);
-      }
-      a[2 * kx] = re;
-      a[2 * kx + 1] = im;
-    }
-  }
-  __syncthreads();
-  // y -> ky: a thread per (slot, z, kx)
-  for (int e = tid; e < sp * P * P; e += nt) {
-    const int j = e / (P * P), z = (e / P) % P, kx = e % P;
-    T ar[P], ai[P];
-#pragma unroll
-    for (int y = 0; y < P; ++y) {
-      const T* q = A + 2 * ((size_t)j * P3 + (z * P + y) * P + kx);
-      ar[y] = q[0];
-      ai[y] = q[1];
-    }
-    T* b = Bm + 2 * ((size_t)j * PNP + z * N * P + kx);
-#pragma unroll
-    for (int ky = 0; ky < N; ++ky) {
-      const T* wk = W + 2 * ky * N;
-      T re = 0, im = 0;
-#pragma unroll
-      for (int y = 0; y < P; ++y) cmad(re, im, ar[y], ai[y], wk[2 * y], wk[2 * y + 1]);
-      b[2 * ky * P] = re;
-      b[2 * ky * P + 1] = im;
-    }
-  }
-  __syncthreads();
-  // z -> kz: a thread per (pair of slots, ky, kx, range of kz); the two
-  // slots of a pair written together as in k_m2l_up
-  using V2 = typename Cplx2<T>::type;
-  const int npair = (sp + 1) / 2;
-  for (int e = tid; e < npair * N * P * KC; e += nt) {
-    const int jp = e / (N * P * KC), c = (e / (N * P)) % KC, ky = (e / P) % N, kx = e % P;
-    const int j = 2 * jp;
-    const bool two = j + 1 < sp;
-    T br[2][P], bi[2][P];
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-      for (int z = 0; z < P; ++z) {
-        if (u == 0 || two) {
-          const T* q = Bm + 2 * ((size_t)(j + u) * PNP + (z * N + ky) * P + kx);
-          br[u][z] = q[0];
-          bi[u][z] = q[1];
-        } else {
-          br[u][z] = bi[u][z] = T(0);
+      for (int u = 0; u < U; ++u) {
+        ar[u] = fma(xr[y][u], c, ar[u]);
+        ai[u] = fma(xi[y][u], c, ai[u]);
+        if (k > 0) {
+          br[u] = fma(xr[y][u], s, br[u]);
+          bi[u] = fma(xi[y][u], s, bi[u]);
         }
       }
-    const int kz1 = (c + 1) * KH < N ? (c + 1) * KH : N;
-    for (int kz = c * KH; kz < kz1; ++kz) {
-      const T* wk = W + 2 * kz * N;
-      const int f = (kz * N + ky) * P + kx;
-      T* out = Q + 2 * q8_index<T>(f, src, slot0 + j, nsrc);
-      T re0 = 0, im0 = 0, re1 = 0, im1 = 0;
+    }
+    T re[U], im[U];
 #pragma unroll
-      for (int z = 0; z < P; ++z) {
-        cmad(re0, im0, br[0][z], bi[0][z], wk[2 * z], wk[2 * z + 1]);
-        if (two) cmad(re1, im1, br[1][z], bi[1][z], wk[2 * z], wk[2 * z + 1]);
+    for (int u = 0; u < U; ++u) {
+      re[u] = ar[u] + bi[u];
+      im[u] = ai[u] - br[u];
+    }
+    put(k, re, im);
+    if (k > 0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        re[u] = ar[u] - bi[u];
+        im[u] = ai[u] + br[u];
       }
-      if (two) {
-        V2 v;
-        v.x = re0;
-        v.y = im0;
-        v.z = re1;
-        v.w = im1;
-        *reinterpret_cast<V2*>(out) = v;
-      } else {
-        out[0] = re0;
-        out[1] = im0;
+      put(N - k, re, im);
+    }
+  }
+}
+
+// P outputs x_o = sum_k X_k exp(2 pi i k (P - 1 + o) / N) of N inputs
+// `in[k * si]`.
+template <typename T, int P>
+__device__ __forceinline__ void dft_inverse(const T* in, size_t si, const Twiddles<T, 2 * P - 1>& tw,
+                                            T (&re)[P][DftSlots<T>::kPer], T (&im)[P][DftSlots<T>::kPer]) {
+  constexpr int N = 2 * P - 1, U = DftSlots<T>::kPer;
+  {
+    T xr[U], xi[U];
+    ld_slots(in, xr, xi);
+#pragma unroll
+    for (int o = 0; o < P; ++o)
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        re[o][u] = xr[u];
+        im[o][u] = xi[u];
+      }
+  }
+#pragma unroll
+  for (int k = 1; k < P; ++k) {
+    T xr[U], xi[U], yr[U], yi[U];
+    ld_slots(in + k * si, xr, xi);
+    ld_slots(in + (N - k) * si, yr, yi);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const T sr = xr[u] + yr[u], sim = xi[u] + yi[u], dr = xr[u] - yr[u], di = xi[u] - yi[u];
+#pragma unroll
+      for (int o = 0; o < P; ++o) {
+        const T c = tw.c[(k * (P - 1 + o)) % N], s = tw.s[(k * (P - 1 + o)) % N];
+        re[o][u] = fma(sr, c, re[o][u]);
+        re[o][u] = fma(-di, s, re[o][u]);
+        im[o][u] = fma(sim, c, im[o][u]);
+        im[o][u] = fma(dr, s, im[o][u]);
       }
     }
   }
 }
 
-template <typename T, int PP>
-__global__ void __launch_bounds__(256)
-    k_m2l_down_rb(const T* __restrict__ Pk, const int* __restrict__ items, const double* __restrict__ tscale,
-                  const int* __restrict__ surf_ijk, const double* __restrict__ twiddle, int ns, int ntar, int sp,
-                  double* __restrict__ p_check) {
-  constexpr int P = PP, N = 2 * P - 1, P3 = P * P * P, PNP = P * N * P, Nf = N * N * P;
-  extern __shared__ unsigned char smem_raw[];
-  T* W = reinterpret_cast<T*>(smem_raw);  // P*N complex: W[o][k] = conj(w)^(k (P-1+o) mod N)
-  T* Y1 = W + 2 * P * N;                  // sp * P*N*P complex: [slot][zo][ky][kx]
-  T* X = Y1 + 2 * (size_t)sp * PNP;       // sp * Nf complex: [slot][f]; later Y2
-  T* Y2 = X;                              // sp * P^3 complex: [slot][zo][yo][kx]
+template <typename T, int P>
+__global__ void __launch_bounds__(dft_threads(P), dft_blocks(P, sizeof(T)))
+    k_m2l_up_rb(const double* __restrict__ q_equiv, const int* __restrict__ items, const int* __restrict__ surf_ijk,
+                const __grid_constant__ Twiddles<T, 2 * P - 1> tw, int nsrc, T* __restrict__ Q) {
+  constexpr int N = 2 * P - 1, U = DftSlots<T>::kPer, SP = DftSlots<T>::kBlock, ns = 6 * (P - 1) * (P - 1) + 2;
+  constexpr int NT = dft_threads(P);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* B = reinterpret_cast<T*>(smem_raw);  // complex [z][ky][kx][slot]
+  auto cell = [&](int z, int ky, int kx) { return B + 2 * SP * ((z * N + ky) * P + kx); };
+  // the [0,P)^3 corner of the grid, [z][y][x][slot], in the rows ky >= P of
+  // each z, which the first pass leaves alone and the second overwrites
+  auto corner = [&](int z, int y) { return cell(z, P, 0) + SP * (y * P); };
   const int* it = items + 10 * blockIdx.x;
-  const int tar = it[0], slot0 = it[1];
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int e = tid; e < P * N; e += nt) {
-    const int o = e / N, k = e % N;
-    const int m = (k * (P - 1 + o)) % N;
-    W[2 * e] = (T)twiddle[2 * m];
-    W[2 * e + 1] = -(T)twiddle[2 * m + 1];
+  const int src = it[0], slot0 = it[1], tid = threadIdx.x;
+  bool any = false;
+#pragma unroll
+  for (int j = 0; j < SP; ++j) any |= it[2 + j] >= 0;
+  if (!any) {  // no child here: zero spectra
+    const T zero[U] = {};
+    for (int e = tid; e < 2 * N * N * P; e += NT)
+      st_slots(Q + 2 * q8_index<T>(e >> 1, src, slot0 + (e & 1) * U, nsrc), zero, zero);
+    return;
   }
-  if (sp >= 2) {
-    using V2 = typename Cplx2<T>::type;
-    const int hp = sp / 2;
-    for (int e = tid; e < Nf * hp; e += nt) {
-      const int f = e / hp, j = 2 * (e % hp);
-      const V2 v = *reinterpret_cast<const V2*>(Pk + (((size_t)f * ntar + tar) * 8 + slot0 + j) * 2);
-      X[2 * ((size_t)j * Nf + f)] = v.x;
-      X[2 * ((size_t)j * Nf + f) + 1] = v.y;
-      X[2 * ((size_t)(j + 1) * Nf + f)] = v.z;
-      X[2 * ((size_t)(j + 1) * Nf + f) + 1] = v.w;
-    }
-  } else {
-    for (int f = tid; f < Nf; f += nt) {
-      const T* in = Pk + (((size_t)f * ntar + tar) * 8 + slot0) * 2;
-      X[2 * f] = in[0];
-      X[2 * f + 1] = in[1];
+  for (int e = tid; e < P * P * P * SP; e += NT) corner(e / (P * P * SP), 0)[e % (P * P * SP)] = T(0);
+  __syncthreads();
+  for (int e = tid; e < SP * ns; e += NT) {
+    const int j = e / ns, i = e - j * ns;
+    const int child = it[2 + j];
+    if (child < 0) continue;
+    const int x = surf_ijk[3 * i], y = surf_ijk[3 * i + 1], z = surf_ijk[3 * i + 2];
+    corner(z, y)[x * SP + j] = (T)q_equiv[(size_t)child * ns + i];
+  }
+  __syncthreads();
+  // x -> kx of the rows (z, y), real input
+  for (int e = tid; e < 2 * P * P; e += NT) {
+    const int g = e & 1, y = (e >> 1) % P, z = (e >> 1) / P;
+    const T* row = corner(z, y) + g * U;
+    T r[P][U];
+#pragma unroll
+    for (int x = 0; x < P; ++x)
+#pragma unroll
+      for (int u = 0; u < U; ++u) r[x][u] = row[x * SP + u];
+#pragma unroll
+    for (int kx = 0; kx < P; ++kx) {
+      T re[U], im[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        re[u] = r[0][u];
+        im[u] = T(0);
+#pragma unroll
+        for (int x = 1; x < P; ++x) {
+          re[u] = fma(r[x][u], tw.c[(x * kx) % N], re[u]);
+          im[u] = fma(-r[x][u], tw.s[(x * kx) % N], im[u]);
+        }
+      }
+      st_slots(cell(z, y, kx) + 2 * U * g, re, im);
     }
   }
   __syncthreads();
-  // kz -> zo (zo < P only): a thread per (slot, ky, kx)
-  for (int e = tid; e < sp * N * P; e += nt) {
-    const int j = e / (N * P), ky = (e / P) % N, kx = e % P;
-    T xr[N], xi[N];
-#pragma unroll
-    for (int kz = 0; kz < N; ++kz) {
-      const T* q = X + 2 * ((size_t)j * Nf + (kz * N + ky) * P + kx);
-      xr[kz] = q[0];
-      xi[kz] = q[1];
-    }
-#pragma unroll
-    for (int zo = 0; zo < P; ++zo) {
-      const T* wo = W + 2 * zo * N;
-      T re = 0, im = 0;
-#pragma unroll
-      for (int kz = 0; kz < N; ++kz) cmad(re, im, xr[kz], xi[kz], wo[2 * kz], wo[2 * kz + 1]);
-      T* y1 = Y1 + 2 * ((size_t)j * PNP + (zo * N + ky) * P + kx);
-      y1[0] = re;
-      y1[1] = im;
-    }
+  // y -> ky of the columns (z, kx)
+  for (int e = tid; e < 2 * P * P; e += NT) {
+    const int g = e & 1, kx = (e >> 1) % P, z = (e >> 1) / P;
+    T* col = cell(z, 0, kx) + 2 * U * g;
+    dft_forward<T, P>(col, 2 * SP * P, tw,
+                      [&](int ky, const T(&re)[U], const T(&im)[U]) { st_slots(col + ky * 2 * SP * P, re, im); });
   }
-  __syncthreads();  // X is read: its space becomes Y2
-  // ky -> yo (yo < P): a thread per (slot, zo, kx)
-  for (int e = tid; e < sp * P * P; e += nt) {
-    const int j = e / (P * P), zo = (e / P) % P, kx = e % P;
-    T yr[N], yi[N];
+  __syncthreads();
+  // z -> kz, into the spectra
+  for (int e = tid; e < 2 * N * P; e += NT) {
+    const int g = e & 1, l = e >> 1;  // l = ky * P + kx
+    T* out = Q + 2 * q8_index<T>(l, src, slot0 + g * U, nsrc);
+    const size_t so = 2 * (q8_index<T>(N * P, 0, 0, nsrc) - q8_index<T>(0, 0, 0, nsrc));
+    dft_forward<T, P>(B + 2 * SP * l + 2 * U * g, 2 * SP * N * P, tw,
+                      [&](int kz, const T(&re)[U], const T(&im)[U]) { st_slots(out + kz * so, re, im); });
+  }
+}
+
+template <typename T, int P>
+__global__ void __launch_bounds__(dft_threads(P), dft_blocks(P, sizeof(T)))
+    k_m2l_down_rb(const T* __restrict__ Pk, const int* __restrict__ items, const double* __restrict__ tscale,
+                  const int* __restrict__ surf_ijk, const __grid_constant__ Twiddles<T, 2 * P - 1> tw, int ntar,
+                  double* __restrict__ p_check) {
+  constexpr int N = 2 * P - 1, U = DftSlots<T>::kPer, SP = DftSlots<T>::kBlock, ns = 6 * (P - 1) * (P - 1) + 2;
+  constexpr int NT = dft_threads(P);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* Y = reinterpret_cast<T*>(smem_raw);  // complex [zo][ky][kx][slot]
+  auto cell = [&](int z, int ky, int kx) { return Y + 2 * SP * ((z * N + ky) * P + kx); };
+  const int* it = items + 10 * blockIdx.x;
+  const int tar = it[0], slot0 = it[1], tid = threadIdx.x;
+  T re[P][U], im[P][U];
+  // kz -> zo, from the spectra
+  for (int e = tid; e < 2 * N * P; e += NT) {
+    const int g = e & 1, l = e >> 1;  // l = ky * P + kx
+    dft_inverse<T, P>(Pk + (((size_t)l * ntar + tar) * 8 + slot0 + g * U) * 2, (size_t)N * P * ntar * 16, tw, re, im);
 #pragma unroll
-    for (int ky = 0; ky < N; ++ky) {
-      const T* q = Y1 + 2 * ((size_t)j * PNP + (zo * N + ky) * P + kx);
-      yr[ky] = q[0];
-      yi[ky] = q[1];
-    }
+    for (int zo = 0; zo < P; ++zo) st_slots(Y + 2 * SP * (zo * N * P + l) + 2 * U * g, re[zo], im[zo]);
+  }
+  __syncthreads();
+  // ky -> yo of the columns (zo, kx)
+  for (int e = tid; e < 2 * P * P; e += NT) {
+    const int g = e & 1, kx = (e >> 1) % P, zo = (e >> 1) / P;
+    T* col = cell(zo, 0, kx) + 2 * U * g;
+    dft_inverse<T, P>(col, 2 * SP * P, tw, re, im);
 #pragma unroll
-    for (int yo = 0; yo < P; ++yo) {
-      const T* wo = W + 2 * yo * N;
-      T re = 0, im = 0;
+    for (int yo = 0; yo < P; ++yo) st_slots(col + yo * 2 * SP * P, re[yo], im[yo]);
+  }
+  __syncthreads();
+  // kx -> xo of the rows (zo, yo): real output, the half kx >= 1 doubled; an
+  // inner row meets the check surface at its ends only
+  for (int e = tid; e < 2 * P * P; e += NT) {
+    const int g = e & 1, yo = (e >> 1) % P, zo = (e >> 1) / P;
+    const bool face = yo == 0 || yo == P - 1 || zo == 0 || zo == P - 1;
+    T* row = cell(zo, yo, 0) + 2 * U * g;
 #pragma unroll
-      for (int ky = 0; ky < N; ++ky) cmad(re, im, yr[ky], yi[ky], wo[2 * ky], wo[2 * ky + 1]);
-      T* y2 = Y2 + 2 * ((size_t)j * P3 + (zo * P + yo) * P + kx);
-      y2[0] = re;
-      y2[1] = im;
+    for (int kx = 0; kx < P; ++kx) ld_slots(row + kx * 2 * SP, re[kx], im[kx]);
+#pragma unroll
+    for (int xo = 0; xo < P; ++xo) {
+      if (xo > 0 && xo < P - 1 && !face) continue;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        T acc = T(0);
+#pragma unroll
+        for (int kx = 1; kx < P; ++kx) {
+          acc = fma(re[kx][u], tw.c[(kx * (P - 1 + xo)) % N], acc);
+          acc = fma(-im[kx][u], tw.s[(kx * (P - 1 + xo)) % N], acc);
+        }
+        row[xo * 2 * SP + u] = re[0][u] + T(2) * acc;
+      }
     }
   }
   __syncthreads();
-  // kx -> xo at the check-surface points, real part; p_check += value * scale
   const double sc = tscale[tar];
-  for (int e = tid; e < sp * ns; e += nt) {
+  for (int e = tid; e < SP * ns; e += NT) {
     const int j = e / ns, i = e - j * ns;
     const int child = it[2 + j];
     if (child < 0) continue;
     const int xo = surf_ijk[3 * i], yo = surf_ijk[3 * i + 1], zo = surf_ijk[3 * i + 2];
-    const T* row = Y2 + 2 * ((size_t)j * P3 + (zo * P + yo) * P);
-    const T* wo = W + 2 * xo * N;
-    T acc = 0;
-    // Re(Y * conj(w)^m) summed over kx >= 1, doubled for the missing half
-    for (int kx = 1; kx < P; ++kx) {
-      acc = fma(row[2 * kx], wo[2 * kx], acc);
-      acc = fma(-row[2 * kx + 1], wo[2 * kx + 1], acc);
-    }
-    const T v = row[0] + T(2) * acc;
-    p_check[(size_t)child * ns + i] += (double)v * sc;
+    p_check[(size_t)child * ns + i] += (double)cell(zo, yo, xo)[(j / U) * 2 * U + j % U] * sc;
   }
 }
 
@@ -1793,12 +1815,11 @@ __global__ void k_m2l_hadamard27(const double* __restrict__ Q, const double* __r
 // (surf_conv_idx_map_down, kernel.cpp:1253-1259), and
 // p_check[child] += value * scale / N^3 (kernel.cpp:1369-1382).
 // items: 10 ints per block = tar, first slot, child cell per slot (-1 = none).
-template <typename T, int PP>
+template <typename T>
 __global__ void __launch_bounds__(256)
     k_m2l_down(const T* __restrict__ Pk, const int* __restrict__ items, const double* __restrict__ tscale,
-               const int* __restrict__ surf_ijk, const double* __restrict__ twiddle, int P_, int ns, int ntar,
+               const int* __restrict__ surf_ijk, const double* __restrict__ twiddle, int P, int ns, int ntar,
                int sp, double* __restrict__ p_check) {
-  const int P = PP > 0 ? PP : P_;
   extern __shared__ unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
   const int N = 2 * P - 1;
@@ -2133,20 +2154,32 @@ cudaError_t launch_sum_children(const int* list, int nparents, const double* Y, 
   return cudaGetLastError();
 }
 
-// orders with a compile-time instance (the register-blocked kernels)
-static bool fixed_p(int P) { return (P >= 4 && P <= 8) || P == 10; }
+// orders with a compile-time instance (the register-blocked kernels): FP32
+// runs at P <= 8 only
+template <typename T>
+static bool fixed_p(int P) {
+  return P >= 4 && P <= (sizeof(T) == 4 ? 8 : 10);
+}
 template <typename T>
 static size_t up_smem(int P, int sp) {
   const size_t N = 2 * P - 1, P3 = (size_t)P * P * P;
-  if (fixed_p(P))
-    return sizeof(T) * ((2 * N * N + 7) / 8 * 8 + 2 * (size_t)sp * P3 + std::max((size_t)sp * P3, 2 * (size_t)sp * P * N * P));
+  if (fixed_p<T>(P)) return sizeof(T) * 2 * DftSlots<T>::kBlock * P * N * P;
   return sizeof(T) * (2 * N * N + 3 * P3 + 2 * (size_t)sp * P * N * P);
 }
 template <typename T>
 static size_t down_smem(int P, int sp) {
   const size_t N = 2 * P - 1, P3 = (size_t)P * P * P;
-  if (fixed_p(P)) return sizeof(T) * (2 * (size_t)P * N + 2 * (size_t)sp * P * N * P + 2 * (size_t)sp * N * N * P);
+  if (fixed_p<T>(P)) return sizeof(T) * 2 * DftSlots<T>::kBlock * P * N * P;
   return sizeof(T) * (2 * (size_t)P * N + 2 * (size_t)P * N * P + 2 * P3 + 2 * (size_t)sp * N * N * P);
+}
+template <typename T, int N>
+static Twiddles<T, N> twiddles() {
+  Twiddles<T, N> t;
+  for (int m = 0; m < N; ++m) {
+    t.c[m] = (T)std::cos(2.0 * M_PI * m / N);
+    t.s[m] = (T)std::sin(2.0 * M_PI * m / N);
+  }
+  return t;
 }
 
 // Largest slot group (8, 4, 2, 1) whose working set fits in shared memory.
@@ -2177,28 +2210,41 @@ static cudaError_t up_p(const double* q_equiv, const int* items, int nitems, con
   if constexpr (PP > 0) {
     cudaError_t e = cudaFuncSetAttribute(k_m2l_up_rb<T, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_m2l_up_rb<T, PP><<<nitems, 256, sm, st>>>(q_equiv, items, surf_ijk, twiddle, ns, nsrc, sp, Q);
+    k_m2l_up_rb<T, PP><<<nitems, dft_threads(PP), sm, st>>>(q_equiv, items, surf_ijk, twiddles<T, 2 * PP - 1>(), nsrc,
+                                                            Q);
   } else {
-    cudaError_t e = cudaFuncSetAttribute(k_m2l_up<T, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = cudaFuncSetAttribute(k_m2l_up<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_m2l_up<T, PP><<<nitems, 256, sm, st>>>(q_equiv, items, surf_ijk, twiddle, P, ns, nsrc, sp, Q);
+    k_m2l_up<T><<<nitems, 256, sm, st>>>(q_equiv, items, surf_ijk, twiddle, P, ns, nsrc, sp, Q);
   }
   return cudaGetLastError();
+}
+
+// calls f(integral_constant<P>) for an order with a compile-time instance, else f(0)
+template <typename T, typename F>
+static cudaError_t with_order(int P, F f) {
+  switch (P) {
+    case 4: return f(std::integral_constant<int, 4>());
+    case 5: return f(std::integral_constant<int, 5>());
+    case 6: return f(std::integral_constant<int, 6>());
+    case 7: return f(std::integral_constant<int, 7>());
+    case 8: return f(std::integral_constant<int, 8>());
+    default: break;
+  }
+  if constexpr (sizeof(T) == 8) {
+    if (P == 9) return f(std::integral_constant<int, 9>());
+    if (P == 10) return f(std::integral_constant<int, 10>());
+  }
+  return f(std::integral_constant<int, 0>());
 }
 
 template <typename T>
 cudaError_t launch_m2l_up(const double* q_equiv, const int* items, int nitems, const int* surf_ijk,
                           const double* twiddle, int P, int ns, int nsrc, int sp, T* Q, cudaStream_t st) {
   if (nitems <= 0) return cudaGetLastError();
-  switch (P) {
-    case 4: return up_p<T, 4>(q_equiv, items, nitems, surf_ijk, twiddle, P, ns, nsrc, sp, Q, st);
-    case 5: return up_p<T, 5>(q_equiv, items, nitems, surf_ijk, twiddle, P, ns, nsrc, sp, Q, st);
-    case 6: return up_p<T, 6>(q_equiv, items, nitems, surf_ijk, twiddle, P, ns, nsrc, sp, Q, st);
-    case 7: return up_p<T, 7>(q_equiv, items, nitems, surf_ijk, twiddle, P, ns, nsrc, sp, Q, st);
-    case 8: return up_p<T, 8>(q_equiv, items, nitems, surf_ijk, twiddle, P, ns, nsrc, sp, Q, st);
-    case 10: return up_p<T, 10>(q_equiv, items, nitems, surf_ijk, twiddle, P, ns, nsrc, sp, Q, st);
-    default: return up_p<T, 0>(q_equiv, items, nitems, surf_ijk, twiddle, P, ns, nsrc, sp, Q, st);
-  }
+  return with_order<T>(P, [&](auto pp) {
+    return up_p<T, pp.value>(q_equiv, items, nitems, surf_ijk, twiddle, P, ns, nsrc, sp, Q, st);
+  });
 }
 
 cudaError_t launch_m2l_hadamard8(const float* Q, const float* G, const int* tsrcT, int ntar, int nsrc, int Nf,
@@ -2262,11 +2308,12 @@ static cudaError_t down_p(const T* Pk, const int* items, const double* tscale, i
     cudaError_t e =
         cudaFuncSetAttribute(k_m2l_down_rb<T, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_m2l_down_rb<T, PP><<<nitems, 256, sm, st>>>(Pk, items, tscale, surf_ijk, twiddle, ns, ntar, sp, p_check);
+    k_m2l_down_rb<T, PP><<<nitems, dft_threads(PP), sm, st>>>(Pk, items, tscale, surf_ijk,
+                                                              twiddles<T, 2 * PP - 1>(), ntar, p_check);
   } else {
-    cudaError_t e = cudaFuncSetAttribute(k_m2l_down<T, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = cudaFuncSetAttribute(k_m2l_down<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_m2l_down<T, PP><<<nitems, 256, sm, st>>>(Pk, items, tscale, surf_ijk, twiddle, P, ns, ntar, sp, p_check);
+    k_m2l_down<T><<<nitems, 256, sm, st>>>(Pk, items, tscale, surf_ijk, twiddle, P, ns, ntar, sp, p_check);
   }
   return cudaGetLastError();
 }
@@ -2276,15 +2323,9 @@ cudaError_t launch_m2l_down(const T* Pk, const int* items, const double* tscale,
                             const int* surf_ijk, const double* twiddle, int P, int ns, int ntar, int sp,
                             double* p_check, cudaStream_t st) {
   if (nitems <= 0) return cudaGetLastError();
-  switch (P) {
-    case 4: return down_p<T, 4>(Pk, items, tscale, nitems, surf_ijk, twiddle, P, ns, ntar, sp, p_check, st);
-    case 5: return down_p<T, 5>(Pk, items, tscale, nitems, surf_ijk, twiddle, P, ns, ntar, sp, p_check, st);
-    case 6: return down_p<T, 6>(Pk, items, tscale, nitems, surf_ijk, twiddle, P, ns, ntar, sp, p_check, st);
-    case 7: return down_p<T, 7>(Pk, items, tscale, nitems, surf_ijk, twiddle, P, ns, ntar, sp, p_check, st);
-    case 8: return down_p<T, 8>(Pk, items, tscale, nitems, surf_ijk, twiddle, P, ns, ntar, sp, p_check, st);
-    case 10: return down_p<T, 10>(Pk, items, tscale, nitems, surf_ijk, twiddle, P, ns, ntar, sp, p_check, st);
-    default: return down_p<T, 0>(Pk, items, tscale, nitems, surf_ijk, twiddle, P, ns, ntar, sp, p_check, st);
-  }
+  return with_order<T>(P, [&](auto pp) {
+    return down_p<T, pp.value>(Pk, items, tscale, nitems, surf_ijk, twiddle, P, ns, ntar, sp, p_check, st);
+  });
 }
 
 cudaError_t launch_dipole(const double4* body64, int n, double* partial, cudaStream_t st) {
