@@ -146,6 +146,9 @@ struct rtfmm_fmm {
   // operator tables: generation built on the host / uploaded to the device
   uint64_t ops_gen = 0, ops_dev_gen = 0;
   size_t h_xin_cap = 0;  // doubles in h_xin
+  char* h_pack = nullptr;  // pinned staging of the plan's tables (PlanPack)
+  size_t h_pack_cap = 0;
+  char d_pack = 0;  // pool key of their device buffer
   // x_in, q_in, plan.x, plan.q, plan.perm and h_xin hold the set-up bodies;
   // after a device set-up they are fetched from d_xin, d_qin and d_perm on
   // first use (ensure_host_bodies)
@@ -198,6 +201,8 @@ struct rtfmm_fmm {
   // the forward pass captured as a CUDA graph (launch_pass), dropped with
   // the device tables
   cudaGraphExec_t pass_graph = nullptr;
+  bool pass_direct = false;  // the last forward pass was issued launch by launch
+  bool pass_seen = false;    // a forward pass ran on these device tables
   bool graph_grad_q_valid = false;
   cudaEvent_t ev_g0 = nullptr, ev_g1 = nullptr;
   // the 8x8 FFT-M2L (up, Hadamard, down) runs in FP32: the mixed form at P <= 8
@@ -265,6 +270,60 @@ int dupload(rtfmm_fmm* f, T** p, const std::vector<T>& h, const void* key = null
   return RTFMM_OK;
 }
 
+// Pinned host memory of at least `bytes` (with a quarter of headroom), kept by
+// the handle: the staging of set-ups and plan uploads.  The caller waits for
+// its copies before the next use.
+char* pinned(rtfmm_fmm* f, size_t bytes) {
+  if (f->h_pack_cap < bytes) {
+    if (f->h_pack) cudaFreeHost(f->h_pack);
+    f->h_pack = nullptr;
+    f->h_pack_cap = 0;
+    if (cudaMallocHost(&f->h_pack, bytes + bytes / 4 + (1 << 16)) != cudaSuccess) {
+      cudaGetLastError();
+      f->h_pack = nullptr;
+      return nullptr;
+    }
+    f->h_pack_cap = bytes + bytes / 4 + (1 << 16);
+  }
+  return f->h_pack;
+}
+
+// The host tables of a plan on their way to the device: laid end to end in
+// one pinned buffer and moved by one copy into one pooled device buffer.  A
+// blocking copy for each of the twenty tables cost 8-10 us whatever its size,
+// most of the upload of a small plan.  Nothing may still read the buffers of
+// the plan before (upload_plan waits for the device).
+struct PlanPack {
+  struct Part {
+    void** p;
+    const void* h;
+    size_t bytes, off;
+  };
+  static constexpr size_t kMax = 4 << 20;  // a larger table is copied by itself (pinned memory is dear)
+  std::vector<Part> parts;
+  size_t total = 0;
+  template <typename T>
+  int add(rtfmm_fmm* f, T** p, const std::vector<T>& h) {
+    if (sizeof(T) * h.size() > kMax) return dupload(f, p, h);
+    parts.push_back({(void**)p, h.data(), sizeof(T) * h.size(), total});
+    total += (sizeof(T) * std::max<size_t>(1, h.size()) + 255) / 256 * 256;
+    return RTFMM_OK;
+  }
+  int upload(rtfmm_fmm* f) {
+    char* d = nullptr;
+    int rc = dalloc(f, &d, total, &f->d_pack);
+    if (rc) return rc;
+    char* h = pinned(f, total);
+    if (!h) return fail(RTFMM_ENOMEM, "pinned host allocation failed");
+    for (const Part& q : parts) {
+      if (q.bytes) std::memcpy(h + q.off, q.h, q.bytes);
+      *q.p = d + q.off;
+    }
+    CK(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, f->s0));
+    return RTFMM_OK;
+  }
+};
+
 void drop_graph(rtfmm_fmm* f) {
   if (f->pass_graph) {
     cudaGraphExecDestroy(f->pass_graph);
@@ -277,6 +336,7 @@ void drop_graph(rtfmm_fmm* f) {
 // use).  The buffers themselves stay in the pool.
 void drop_allocs(rtfmm_fmm* f) {
   drop_graph(f);
+  f->pass_seen = false;
   f->close_valid = false;
   f->n_close = 0;
   f->d_adj_q = f->d_adj_gq = f->d_adj_gw = f->d_adj_w = f->d_adj_dq = f->d_adj_dx = nullptr;
@@ -291,6 +351,9 @@ void free_device(rtfmm_fmm* f) {
     f->h_xin = nullptr;
   }
   f->h_xin_cap = 0;
+  if (f->h_pack) cudaFreeHost(f->h_pack);
+  f->h_pack = nullptr;
+  f->h_pack_cap = 0;
   drop_allocs(f);
   for (auto& kv : f->pool)
     if (kv.second.p) cudaFree(kv.second.p);
@@ -893,6 +956,22 @@ int alloc_parts(rtfmm_fmm* f) {
   return RTFMM_OK;
 }
 
+// The positions in pinned memory, where the host-buffer calls move them from;
+// a handle whose bodies came from device memory has none until such a call.
+int stage_positions(rtfmm_fmm* f) {
+  const int64_t n = f->plan.n;
+  if (f->h_xin_cap < (size_t)std::max<int64_t>(1, 3 * n)) {
+    if (f->h_xin) cudaFreeHost(f->h_xin);
+    f->h_xin = nullptr;
+    f->h_xin_cap = 0;
+    const size_t cap = (size_t)std::max<int64_t>(1, 3 * n + 3 * n / 4);
+    CK(cudaMallocHost(&f->h_xin, sizeof(double) * cap));
+    f->h_xin_cap = cap;
+  }
+  if (n > 0) std::memcpy(f->h_xin, f->x_in.data(), sizeof(double) * 3 * n);
+  return RTFMM_OK;
+}
+
 // Upload the plan (everything but the per-pass body values) to the device.
 int upload_plan(rtfmm_fmm* f) {
   const double t0 = wall_s();
@@ -915,33 +994,28 @@ int upload_plan(rtfmm_fmm* f) {
   } while (0)
   RC(dalloc(f, &f->d_body64, n));
   RC(dalloc(f, &f->d_body32, n));
-  if (f->body_leaf.empty() && n > 0) {
+  PlanPack pack;
+  const bool body_leaf_here = f->body_leaf.empty() && n > 0;
+  if (body_leaf_here)
     RC(dalloc(f, &f->d_body_leaf, n));  // filled below from the leaf table
-  } else {
-    RC(dupload(f, &f->d_body_leaf, f->body_leaf));
-  }
+  else
+    RC(pack.add(f, &f->d_body_leaf, f->body_leaf));
   if (f->host_bodies)
-    RC(dupload(f, &f->d_perm, p.perm));
+    RC(pack.add(f, &f->d_perm, p.perm));
   else
     RC(dalloc(f, &f->d_perm, n));  // written by the device tree
   RC(dalloc(f, &f->d_xin, 3 * n));
   RC(dalloc(f, &f->d_qin, n));
-  RC(dupload(f, &f->d_leaves, f->leaves));
-  if (f->body_leaf.empty() && n > 0) CK(launch_body_leaf(f->d_leaves, (int)nleaf, (int)n, f->d_body_leaf, f->s0));
-  {
-    // the exchange of a two-phase pass: every leaf's cell, and which leaves
-    // this rank computes
-    std::vector<int> lc(nleaf);
-    std::vector<char> lo(nleaf, 0);
-    for (size_t l = 0; l < nleaf; ++l) lc[l] = f->leaves[l].cell;
-    for (int l : f->own_leaves) lo[l] = 1;
-    RC(dupload(f, &f->d_leaf_cells, lc));
-    RC(dupload(f, &f->d_leaf_own, lo));
-  }
-  if (f->shard_n > 1)
-    RC(dupload(f, &f->d_leaves_own, f->leaves_own));
-  else
-    f->d_leaves_own = f->d_leaves;
+  RC(pack.add(f, &f->d_leaves, f->leaves));
+  // the exchange of a two-phase pass: every leaf's cell, and which leaves
+  // this rank computes
+  std::vector<int> leaf_cells(nleaf);
+  std::vector<char> leaf_own(nleaf, 0);
+  for (size_t l = 0; l < nleaf; ++l) leaf_cells[l] = f->leaves[l].cell;
+  for (int l : f->own_leaves) leaf_own[l] = 1;
+  RC(pack.add(f, &f->d_leaf_cells, leaf_cells));
+  RC(pack.add(f, &f->d_leaf_own, leaf_own));
+  if (f->shard_n > 1) RC(pack.add(f, &f->d_leaves_own, f->leaves_own));
   RC(dalloc(f, &f->d_qeq, ncell * ns));
   RC(dalloc(f, &f->d_pchk, ncell * ns));
   RC(dalloc(f, &f->d_leafvec, nleaf * ns));
@@ -954,20 +1028,20 @@ int upload_plan(rtfmm_fmm* f) {
   RC(dalloc(f, &f->d_out_phi, n));
   RC(dalloc(f, &f->d_out_grad, 3 * n));
   if (!f->p2p_on_device) {  // else device_p2p_tables writes them
-    RC(dupload(f, &f->d_items2, f->items2));
-    RC(dupload(f, &f->d_list_off, f->list_off));
+    RC(pack.add(f, &f->d_items2, f->items2));
+    RC(pack.add(f, &f->d_list_off, f->list_off));
     RC(alloc_parts(f));
     if (mixed)
-      RC(dupload(f, &f->d_list32, f->list32));
+      RC(pack.add(f, &f->d_list32, f->list32));
     else
-      RC(dupload(f, &f->d_list64, f->list64));
+      RC(pack.add(f, &f->d_list64, f->list64));
   }
-  RC(dupload(f, &f->d_idx_pool, f->idx_pool));
-  RC(dupload(f, &f->d_scale_pool, f->scale_pool));
+  RC(pack.add(f, &f->d_idx_pool, f->idx_pool));
+  RC(pack.add(f, &f->d_scale_pool, f->scale_pool));
   std::vector<int> tsrcT(f->tsrc8.size());
   for (int t = 0; t < f->nT8; ++t)
     for (int d = 0; d < 26; ++d) tsrcT[(size_t)d * f->nT8 + t] = f->tsrc8[(size_t)t * 26 + d];
-  RC(dupload(f, &f->d_tsrc8, tsrcT));
+  RC(pack.add(f, &f->d_tsrc8, tsrcT));
   f->m2l32 = mixed && o.P <= kM2L32MaxP;
   if (f->ops_dev_gen != f->ops_gen) {
     RC(upload_operators(f));
@@ -1006,24 +1080,19 @@ int upload_plan(rtfmm_fmm* f) {
   group(f->down8_slots, f->sp_down8, false, f->down8_items);
   group(f->up27_slots, f->sp_up27, true, f->up27_items);
   group(f->down27_slots, f->sp_down27, false, f->down27_items);
-  RC(dupload(f, &f->d_up8, f->up8_items));
-  RC(dupload(f, &f->d_down8, f->down8_items));
-  RC(dupload(f, &f->d_up27, f->up27_items));
-  RC(dupload(f, &f->d_down27, f->down27_items));
-  RC(dupload(f, &f->d_tsrc27, f->tsrc27));
-  RC(dupload(f, &f->d_tscale8, f->tscale8));
-  RC(dupload(f, &f->d_tscale27, f->tscale27));
+  RC(pack.add(f, &f->d_up8, f->up8_items));
+  RC(pack.add(f, &f->d_down8, f->down8_items));
+  RC(pack.add(f, &f->d_up27, f->up27_items));
+  RC(pack.add(f, &f->d_down27, f->down27_items));
+  RC(pack.add(f, &f->d_tsrc27, f->tsrc27));
+  RC(pack.add(f, &f->d_tscale8, f->tscale8));
+  RC(pack.add(f, &f->d_tscale27, f->tscale27));
   RC(dalloc(f, &f->d_dip, kDipoleScratch));
+  RC(pack.upload(f));
+  if (f->shard_n <= 1) f->d_leaves_own = f->d_leaves;
+  if (body_leaf_here) CK(launch_body_leaf(f->d_leaves, (int)nleaf, (int)n, f->d_body_leaf, f->s0));
+  if (f->host_bodies) RC(stage_positions(f));
 #undef RC
-  if (f->h_xin_cap < (size_t)std::max<int64_t>(1, 3 * n)) {
-    if (f->h_xin) cudaFreeHost(f->h_xin);
-    f->h_xin = nullptr;
-    f->h_xin_cap = 0;
-    const size_t cap = (size_t)std::max<int64_t>(1, 3 * n + 3 * n / 4);
-    CK(cudaMallocHost(&f->h_xin, sizeof(double) * cap));
-    f->h_xin_cap = cap;
-  }
-  if (n > 0 && f->host_bodies) std::memcpy(f->h_xin, f->x_in.data(), sizeof(double) * 3 * n);
   f->device_ready = true;
   f->setup_s[5] = wall_s() - t0;
   return RTFMM_OK;
@@ -1282,10 +1351,13 @@ int collect_times(rtfmm_fmm* f, float* total) {
   return RTFMM_OK;
 }
 
-// The forward pass as a CUDA graph: captured on first use per set of device
-// tables (the launches, their arguments and the two-stream fork/join are
-// fixed by the plan; charges, positions and outputs live in the handle's
-// buffers), then replayed with one launch.  Kernel nodes keep the priority
+// The forward pass as a CUDA graph: captured by the second pass on a set of
+// device tables (a single pass, as in a solve or a time step, is cheaper
+// issued launch by launch than captured and instantiated, 0.3 ms less for a
+// solve of 1000 bodies) and
+// replayed with one launch from then on (the launches, their arguments and the
+// two-stream fork/join are fixed by the plan; charges, positions and outputs
+// live in the handle's buffers).  Kernel nodes keep the priority
 // of the stream they were captured from, so the far-field chain still
 // preempts P2P.  Per-stage events are not recorded in a replay: the stage
 // timing and serial diagnostics (RTFMM_STAGE_TIMED, RTFMM_STAGE_SERIAL)
@@ -1298,7 +1370,9 @@ bool use_graph(const rtfmm_fmm* f) {
 int launch_pass(rtfmm_fmm* f) {
   int rc0 = ensure_close_pairs(f);
   if (rc0) return rc0;
-  if (!use_graph(f)) return enqueue_pass(f);
+  f->pass_direct = !use_graph(f) || !f->pass_seen;
+  f->pass_seen = true;
+  if (f->pass_direct) return enqueue_pass(f);
   if (!f->pass_graph) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(f->s0, cudaStreamCaptureModeThreadLocal));
@@ -1327,9 +1401,10 @@ int launch_pass(rtfmm_fmm* f) {
 // Waits for the pass launched by launch_pass; *total = its device time.
 int pass_times(rtfmm_fmm* f, float* total) {
   if (!use_graph(f)) return collect_times(f, total);
-  CK(cudaEventSynchronize(f->ev_g1));
+  cudaEvent_t e0 = f->pass_direct ? f->ev_start : f->ev_g0, e1 = f->pass_direct ? f->ev_stop : f->ev_g1;
+  CK(cudaEventSynchronize(e1));
   float ms = 0;
-  CK(cudaEventElapsedTime(&ms, f->ev_g0, f->ev_g1));
+  CK(cudaEventElapsedTime(&ms, e0, e1));
   if (total) *total = ms;
   for (int k = 0; k < ST_N; ++k) f->stage_ms[k] = 0;
   return RTFMM_OK;
@@ -1432,8 +1507,8 @@ int ensure_host_bodies(rtfmm_fmm* f, bool tree_order = true) {
     p.x[3 * i + 2] = f->x_in[3 * k + 2];
     p.q[i] = f->q_in[k];
   }
-  if (f->h_xin && f->h_xin_cap >= (size_t)(3 * n) && n > 0)
-    std::memcpy(f->h_xin, f->x_in.data(), sizeof(double) * 3 * n);
+  int rc = stage_positions(f);
+  if (rc) return rc;
   f->host_bodies = true;
   return RTFMM_OK;
 }
@@ -1469,6 +1544,7 @@ constexpr int kTableSlots = 48;
 // cached for this P, images and radius) and host tables of the plan whose
 // tree is built; st[1..3] get their wall times.
 void finish_setup(rtfmm_fmm* f, const TreeScratchFn* gpu = nullptr) {
+  const PinnedFn pin = [f](size_t bytes) { return pinned(f, bytes); };
   double* st = f->setup_s;
   double t = wall_s();
   bool device_tables = false;
@@ -1479,7 +1555,7 @@ void finish_setup(rtfmm_fmm* f, const TreeScratchFn* gpu = nullptr) {
     f->dwalk = DeviceWalk();
     // the lists stay on the device when the GPU builds the P2P tables from
     // them (the host copy is fetched only on request, rtfmm_b200_get_p2p)
-    const int rc = device_p2p_walk(f->plan, roots, f->s0, *gpu, kWalkSlots, &f->dwalk, msg, false);
+    const int rc = device_p2p_walk(f->plan, roots, f->s0, *gpu, pin, kWalkSlots, &f->dwalk, msg, false);
     if (rc == kTreeError) throw std::runtime_error(msg);
     if (rc == kTreeTooDeep) {
       f->plan.p2p.clear();
@@ -1622,7 +1698,8 @@ int rtfmm_b200_setup_device(rtfmm_fmm* f, int64_t n, const double* x_dev, const 
     f->d_qin = dq;
     f->d_perm = dp;
     std::string msg;
-    const int tr = device_build_tree(x_dev, q_dev, n, f->s0, f->plan, dp, scratch, msg);
+    const PinnedFn pin = [f](size_t bytes) { return pinned(f, bytes); };
+    const int tr = device_build_tree(x_dev, q_dev, n, f->s0, f->plan, dp, scratch, pin, msg);
     if (tr == kTreeError) {
       f->plan = Plan();
       const bool bad = msg == "non-finite body position or charge";

@@ -1115,7 +1115,7 @@ __global__ void __launch_bounds__(256)
 // [z][ky][kx][slot]; every pass works in place on it, which leaves room for
 // two to seven blocks per SM.  Up and down at N = 2^20, P = 8 (FP32): 0.20 and
 // 0.34 -> 0.12 and 0.14 ms; at P = 10 (FP64, 10^6 bodies in blobs): 1.47 and
-// 2.38 -> 0.84 and 0.78 ms, 60% of the measured HBM rate for the spectra alone.
+// 2.38 -> 0.84 and 0.78 ms, the latter 40% of the measured HBM rate for the spectra alone.
 template <typename T, int N>
 struct Twiddles {
   T c[N], s[N];  // cos, sin (2 pi m / N)

@@ -179,76 +179,81 @@ int device_walk_host_lists(const DeviceWalk& dw, Plan& plan, cudaStream_t st, st
   return kTreeOk;
 }
 
+namespace {
+// The next frames and the pairs emitted by a round.
+__global__ void k_walk_totals(const int* __restrict__ nkid, const int* __restrict__ koff, const int* __restrict__ nhit,
+                              const int* __restrict__ hoff, int nf, int* __restrict__ out) {
+  out[0] = koff[nf - 1] + nkid[nf - 1];
+  out[1] = hoff[nf - 1] + nhit[nf - 1];
+}
+}  // namespace
+
 int device_p2p_walk(Plan& plan, const std::vector<WalkRoot>& roots, cudaStream_t st, const TreeScratchFn& scratch,
-                    int slot_base, DeviceWalk* dw, std::string& msg, bool host_lists) {
+                    const PinnedFn& pinned, int slot_base, DeviceWalk* dw, std::string& msg, bool host_lists) {
   const int nc = (int)plan.cells.size();
   if (nc >= (1 << kCellBits) || roots.size() > 31) return kTreeTooDeep;
   Scratch S{scratch, slot_base};
   enum {
-    S_CX, S_CR, S_CD, S_CN, S_CO, S_OFF,
+    S_CX,
     S_FR0, S_HI0, S_LO0, S_FR1, S_HI1, S_LO1,
     S_NKID, S_NHIT, S_KOFF, S_HOFF, S_FLAG, S_TMP,
     S_HHI0, S_HLO0, S_HVAL0, S_HHI1, S_HLO1, S_HVAL1,
-    S_IDX0, S_IDX1, S_G0, S_G1, S_CB, S_CM
+    S_IDX0, S_IDX1, S_G0, S_G1
   };
-  // cells, structure of arrays
-  std::vector<double> hx(3 * (size_t)nc), hr(nc);
-  std::vector<int> hd(nc), hn(nc), ho(nc), hb(nc), hm(nc);
-  for (int c = 0; c < nc; ++c) {
-    const Cell& cl = plan.cells[c];
-    for (int k = 0; k < 3; ++k) hx[3 * (size_t)c + k] = cl.x[k];
-    hr[c] = cl.r;
-    hd[c] = cl.depth;
-    hn[c] = cl.cnum;
-    ho[c] = cl.coff;
-    hb[c] = cl.boff;
-    hm[c] = cl.bnum;
-  }
+  // one staging block for one copy: the walks' offsets, the root frames
+  // (path = walk index) and the cells as a structure of arrays; its first
+  // words come back with each round's totals
   const int nw = (int)roots.size();
-  std::vector<double> hoff(3 * nw);
-  for (int w = 0; w < nw; ++w)
-    for (int k = 0; k < 3; ++k) hoff[3 * w + k] = roots[w].off[k];
-  DevCells C;
-  double *dcx, *dcr, *doff;
-  int *dcd, *dcn, *dco;
-  LCK(S.get(S_CX, &dcx, hx.size()));
-  LCK(S.get(S_CR, &dcr, nc));
-  LCK(S.get(S_CD, &dcd, nc));
-  LCK(S.get(S_CN, &dcn, nc));
-  LCK(S.get(S_CO, &dco, nc));
-  LCK(S.get(S_OFF, &doff, hoff.size()));
-  LCK(cudaMemcpyAsync(dcx, hx.data(), sizeof(double) * hx.size(), cudaMemcpyHostToDevice, st));
-  LCK(cudaMemcpyAsync(dcr, hr.data(), sizeof(double) * nc, cudaMemcpyHostToDevice, st));
-  LCK(cudaMemcpyAsync(dcd, hd.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
-  LCK(cudaMemcpyAsync(dcn, hn.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
-  LCK(cudaMemcpyAsync(dco, ho.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
-  LCK(cudaMemcpyAsync(doff, hoff.data(), sizeof(double) * hoff.size(), cudaMemcpyHostToDevice, st));
-  int *dcb, *dcm;
-  LCK(S.get(S_CB, &dcb, nc));
-  LCK(S.get(S_CM, &dcm, nc));
-  LCK(cudaMemcpyAsync(dcb, hb.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
-  LCK(cudaMemcpyAsync(dcm, hm.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
-  C.cx = dcx;
-  C.cr = dcr;
-  C.cdepth = dcd;
-  C.ccnum = dcn;
-  C.ccoff = dco;
-
-  // the first frontier: the root frames, path = walk index
-  std::vector<int4> hfr(nw);
-  std::vector<unsigned long long> hhi(nw), hlo(nw, 0);
-  for (int w = 0; w < nw; ++w) {
-    hfr[w] = make_int4(roots[w].tc, roots[w].sc, roots[w].tcp, roots[w].scp);
-    hhi[w] = (unsigned long long)w << kWalkShift;
+  const size_t n8 = 3 * (size_t)nc + nc + 3 * (size_t)nw + 2 * (size_t)nw;  // 8-byte values after the frames
+  const size_t bytes = 64 + sizeof(int4) * nw + 8 * n8 + sizeof(int) * 5 * (size_t)nc;
+  char* hst = pinned(bytes);
+  if (!hst) {
+    msg = "pinned host allocation failed";
+    return kTreeError;
   }
-  int4* fr[2];
-  unsigned long long *khi[2], *klo[2];
-  LCK(S.get(S_FR0, &fr[0], nw));
-  LCK(S.get(S_HI0, &khi[0], nw));
-  LCK(S.get(S_LO0, &klo[0], nw));
-  LCK(cudaMemcpyAsync(fr[0], hfr.data(), sizeof(int4) * nw, cudaMemcpyHostToDevice, st));
-  LCK(cudaMemcpyAsync(khi[0], hhi.data(), sizeof(unsigned long long) * nw, cudaMemcpyHostToDevice, st));
-  LCK(cudaMemcpyAsync(klo[0], hlo.data(), sizeof(unsigned long long) * nw, cudaMemcpyHostToDevice, st));
+  char* dst = nullptr;
+  LCK(S.get(S_CX, &dst, bytes));
+  auto at = [&](char* base, size_t off) { return base + off; };
+  const size_t o_fr = 64, o_x = o_fr + sizeof(int4) * nw, o_r = o_x + 24 * (size_t)nc, o_off = o_r + 8 * (size_t)nc,
+               o_hi = o_off + 24 * (size_t)nw, o_lo = o_hi + 8 * (size_t)nw, o_i = o_lo + 8 * (size_t)nw;
+  {
+    double *hx = (double*)at(hst, o_x), *hr = (double*)at(hst, o_r), *hoff = (double*)at(hst, o_off);
+    int *hd = (int*)at(hst, o_i), *hn = hd + nc, *ho = hn + nc, *hb = ho + nc, *hm = hb + nc;
+#pragma omp parallel for schedule(static) if (nc > (1 << 15))
+    for (int c = 0; c < nc; ++c) {
+      const Cell& cl = plan.cells[c];
+      for (int k = 0; k < 3; ++k) hx[3 * (size_t)c + k] = cl.x[k];
+      hr[c] = cl.r;
+      hd[c] = cl.depth;
+      hn[c] = cl.cnum;
+      ho[c] = cl.coff;
+      hb[c] = cl.boff;
+      hm[c] = cl.bnum;
+    }
+    int4* hfr = (int4*)at(hst, o_fr);
+    unsigned long long *hhi = (unsigned long long*)at(hst, o_hi), *hlo = (unsigned long long*)at(hst, o_lo);
+    for (int w = 0; w < nw; ++w) {
+      for (int k = 0; k < 3; ++k) hoff[3 * w + k] = roots[w].off[k];
+      hfr[w] = make_int4(roots[w].tc, roots[w].sc, roots[w].tcp, roots[w].scp);
+      hhi[w] = (unsigned long long)w << kWalkShift;
+      hlo[w] = 0;
+    }
+  }
+  LCK(cudaMemcpyAsync(dst, hst, bytes, cudaMemcpyHostToDevice, st));
+  int* totals = (int*)dst;  // the block's first 64 bytes
+  double* doff = (double*)at(dst, o_off);
+  int *dci = (int*)at(dst, o_i), *dcb = dci + 3 * (size_t)nc, *dcm = dci + 4 * (size_t)nc;
+  DevCells C;
+  C.cx = (double*)at(dst, o_x);
+  C.cr = (double*)at(dst, o_r);
+  C.cdepth = dci;
+  C.ccnum = dci + nc;
+  C.ccoff = dci + 2 * (size_t)nc;
+
+  // the first frontier: the root frames
+  int4* fr[2] = {(int4*)at(dst, o_fr), nullptr};
+  unsigned long long *khi[2] = {(unsigned long long*)at(dst, o_hi), nullptr},
+                     *klo[2] = {(unsigned long long*)at(dst, o_lo), nullptr};
   int* flag;
   LCK(S.get(S_FLAG, &flag, 1));
   LCK(cudaMemsetAsync(flag, 0, sizeof(int), st));
@@ -300,13 +305,11 @@ int device_p2p_walk(Plan& plan, const std::vector<WalkRoot>& roots, cudaStream_t
     if ((rc = need_tmp(tb))) return rc;
     LCK(cub::DeviceScan::ExclusiveSum(tmp, tb, nkid, koff, nf, st));
     LCK(cub::DeviceScan::ExclusiveSum(tmp, tb, nhit, hoff_d, nf, st));
-    int last[4];
-    LCK(cudaMemcpyAsync(&last[0], koff + nf - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    LCK(cudaMemcpyAsync(&last[1], nkid + nf - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    LCK(cudaMemcpyAsync(&last[2], hoff_d + nf - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    LCK(cudaMemcpyAsync(&last[3], nhit + nf - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    k_walk_totals<<<1, 1, 0, st>>>(nkid, koff, nhit, hoff_d, nf, totals);
+    LCK(cudaGetLastError());
+    LCK(cudaMemcpyAsync(hst, totals, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     LCK(cudaStreamSynchronize(st));
-    const int64_t nkids = (int64_t)last[0] + last[1], nhits = (int64_t)last[2] + last[3];
+    const int64_t nkids = ((int*)hst)[0], nhits = ((int*)hst)[1];
     if (nkids > (1 << 30) || hcount + nhits > (1 << 30)) return kTreeTooDeep;
     if (nkids > 0 && round >= kMaxDivisions) return kTreeTooDeep;  // paths would not fit
     if ((rc = grow_hits(hcount + (int)nhits))) return rc;
@@ -324,10 +327,9 @@ int device_p2p_walk(Plan& plan, const std::vector<WalkRoot>& roots, cudaStream_t
     cur = nx;
     ++round;
   }
-  int hflag = 0;
-  LCK(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+  LCK(cudaMemcpyAsync(hst, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   LCK(cudaStreamSynchronize(st));
-  if (hflag) return kTreeTooDeep;
+  if (*(int*)hst) return kTreeTooDeep;
 
   // depth-first order, then stably by target cell
   const int H = hcount;
@@ -351,7 +353,9 @@ int device_p2p_walk(Plan& plan, const std::vector<WalkRoot>& roots, cudaStream_t
       LCK(cudaGetLastError());
       LCK(cub::DeviceRadixSort::SortPairs(tmp, tb, g1, g0, idx1, idx0, H, 0, 64, st));
     } else {
-      LCK(cub::DeviceRadixSort::SortPairs(tmp, tb, hh[hset], g0, idx0, idx1, H, 0, 64, st));
+      // the paths end at the last round's digit: zeros below
+      LCK(cub::DeviceRadixSort::SortPairs(tmp, tb, hh[hset], g0, idx0, idx1, H, 3 * std::max(0, kHiDigits - round),
+                                          kWalkShift + 5, st));
       std::swap(idx0, idx1);
     }
     // idx0: pair indices in depth-first order

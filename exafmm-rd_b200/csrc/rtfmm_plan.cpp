@@ -166,7 +166,7 @@ std::string build_tree(Plan& plan, const double* xin, const double* qin) {
   plan.ntree = (int)plan.cells.size();
   plan.x.resize(3 * n);
   plan.q.resize(n);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (n > 16384)
   for (int64_t i = 0; i < n; ++i) {
     const int64_t k = plan.perm[i];
     plan.x[3 * i + 0] = xin[3 * k + 0];
@@ -223,9 +223,9 @@ struct Walker {
 
   // The walk below one frame, its P2P pairs (target, source) appended in the
   // order the recursion emits them.
-  void walk(const Frame& f0, const V3& off, std::vector<std::pair<int, int>>& out) const {
-    std::vector<Frame> stack;
-    stack.push_back(f0);
+  template <typename Put>
+  void walk(const Frame& f0, const V3& off, std::vector<Frame>& stack, Put put) const {
+    stack.assign(1, f0);
     Frame kids[8];
     while (!stack.empty()) {
       const Frame f = stack.back();
@@ -233,7 +233,7 @@ struct Walker {
       int hit = -1;
       const int r = step(f, off, &hit, kids);
       if (r == 1) {
-        out.push_back({f.tc, hit});
+        put(f.tc, hit);
       } else if (r < 0) {
         for (int i = -r - 1; i >= 0; --i) stack.push_back(kids[i]);
       }
@@ -272,36 +272,48 @@ struct Walker {
       }
       items.swap(next);
     }
-    std::vector<std::vector<std::pair<int, int>>> outs(items.size());
+    // Chunks of items walk in parallel, each with one stack and one output (an
+    // allocation for every item was most of a small tree's walk).
+    struct Pair {
+      int tc, sc, walk;
+    };
+    const int ni = (int)items.size(), nc = std::min(ni, 256);
+    std::vector<std::vector<Pair>> outs(nc);
+    auto chunk0 = [&](int c) { return (int)((int64_t)ni * c / nc); };
 #pragma omp parallel for schedule(dynamic, 1)
-    for (int i = 0; i < (int)items.size(); ++i) {
-      const Item& it = items[(size_t)i];
-      if (it.hit >= 0)
-        outs[(size_t)i].push_back({it.f.tc, it.hit});
-      else
-        walk(it.f, offs[(size_t)it.walk], outs[(size_t)i]);
+    for (int c = 0; c < nc; ++c) {
+      std::vector<Frame> stack;
+      std::vector<Pair>& out = outs[(size_t)c];
+      for (int i = chunk0(c); i < chunk0(c + 1); ++i) {
+        const Item& it = items[(size_t)i];
+        if (it.hit >= 0)
+          out.push_back({it.f.tc, it.hit, it.walk});
+        else
+          walk(it.f, offs[(size_t)it.walk], stack, [&](int tc, int sc) { out.push_back({tc, sc, it.walk}); });
+      }
     }
-    // Merge in item order: chunks of items count their pairs per target,
-    // the counts give each chunk its place in every target's list, and the
-    // chunks fill their places in parallel -- the lists of the sequential
-    // merge, entry for entry.
-    const int ni = (int)items.size();
+    // Merge in order: runs of chunks count their pairs per target, the counts
+    // give each run its place in every target's list, and the runs fill their
+    // places in parallel -- the lists of the sequential merge, entry for entry.
+    int ncell = 0;
+    size_t npairs = 0;
+    for (const auto& o : outs) {
+      npairs += o.size();
+      for (const Pair& pr : o) ncell = std::max(ncell, pr.tc + 1);
+    }
     int T = 1;
 #ifdef _OPENMP
-    T = std::max(1, std::min(omp_get_max_threads(), ni));
+    if (npairs > 32768) T = std::max(1, std::min(omp_get_max_threads(), nc));
 #endif
-    int ncell = 0;
-    for (const auto& o : outs)
-      for (const auto& pr : o) ncell = std::max(ncell, pr.first + 1);
     std::vector<int> cnt((size_t)T * ncell, 0);
 #pragma omp parallel for num_threads(T) schedule(static, 1) if (T > 1)
     for (int t = 0; t < T; ++t) {
       int* c = &cnt[(size_t)t * ncell];
-      for (int i = ni * t / T; i < ni * (t + 1) / T; ++i)
-        for (const auto& pr : outs[(size_t)i]) c[pr.first]++;
+      for (int i = nc * t / T; i < nc * (t + 1) / T; ++i)
+        for (const Pair& pr : outs[(size_t)i]) c[pr.tc]++;
     }
     if ((int)p.p2p.v.size() < ncell) p.p2p.v.resize(ncell);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (T > 1)
     for (int c = 0; c < ncell; ++c) {
       int run = (int)p.p2p.v[(size_t)c].size();
       for (int t = 0; t < T; ++t) {
@@ -314,9 +326,9 @@ struct Walker {
 #pragma omp parallel for num_threads(T) schedule(static, 1) if (T > 1)
     for (int t = 0; t < T; ++t) {
       int* at = &cnt[(size_t)t * ncell];
-      for (int i = ni * t / T; i < ni * (t + 1) / T; ++i)
-        for (const auto& pr : outs[(size_t)i])
-          p.p2p.v[(size_t)pr.first][(size_t)at[pr.first]++] = {pr.second, offs[(size_t)items[(size_t)i].walk]};
+      for (int i = nc * t / T; i < nc * (t + 1) / T; ++i)
+        for (const Pair& pr : outs[(size_t)i])
+          p.p2p.v[(size_t)pr.tc][(size_t)at[pr.tc]++] = {pr.sc, offs[(size_t)pr.walk]};
     }
   }
 };
@@ -379,7 +391,7 @@ void traverse_finish(Plan& plan) {
   // each axis gives the octant at level l).
   const V3 lo{a.x[0] - plan.r0, a.x[1] - plan.r0, a.x[2] - plan.r0};
   std::vector<std::array<int64_t, 3>> coord(plan.ntree);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (plan.ntree > 4096)
   for (int c = 0; c < plan.ntree; ++c) {
     const Cell& cl = plan.cells[c];
     for (int k = 0; k < 3; ++k)
@@ -387,7 +399,7 @@ void traverse_finish(Plan& plan) {
   }
   // each tree cell's child by octant (-1: none)
   std::vector<std::array<int, 8>> child(plan.ntree);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (plan.ntree > 4096)
   for (int c = 0; c < plan.ntree; ++c) {
     const Cell& cl = plan.cells[c];
     child[c].fill(-1);

@@ -37,6 +37,18 @@ namespace rtfmm_b200 {
 namespace {
 
 constexpr int kKeyLevels = 21;
+// The keys are sorted by their first kSortLevels digits, half the radix passes
+// of the whole key; a tree with cells to split below that level is sorted
+// again by all of them.
+constexpr int kSortLevels = 10;
+// Largest leaf (ncrit) whose bodies are put in input order by counting, each
+// against the others of its leaf: 256 bodies take 256 shared-memory reads a
+// body, well below the six radix passes over (leaf, index) that larger ones
+// get.
+constexpr int kRankMax = 1024;
+// Child slots copied to the host along with a level's counts, before their
+// number is known: one wait per level instead of two while the level is small.
+constexpr int kSpeculate = 4096;
 
 __global__ void k_path_keys(const double* __restrict__ x, const double* __restrict__ q, int n, double cx, double cy,
                             double cz, double r0, unsigned long long* __restrict__ key, int* __restrict__ idx,
@@ -124,6 +136,26 @@ __global__ void k_leaf_keys(const int* __restrict__ lboff, const int* __restrict
   }
 }
 
+// The bodies of every leaf in input order: perm[b0 + #smaller] = index.
+__global__ void __launch_bounds__(256)
+    k_leaf_rank(const int* __restrict__ lboff, const int* __restrict__ lbnum, int nleaf, int n,
+                const int* __restrict__ idx, int64_t* __restrict__ perm) {
+  __shared__ int s[kRankMax];
+  for (int l = blockIdx.x; l < nleaf; l += gridDim.x) {
+    const int b0 = lboff[l], nb = lbnum[l];
+    if (nb > kRankMax || b0 < 0 || b0 + nb > n) continue;  // the host chose the sort for such leaves
+    __syncthreads();
+    for (int t = threadIdx.x; t < nb; t += blockDim.x) s[t] = idx[b0 + t];
+    __syncthreads();
+    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
+      const int v = s[t];
+      int r = 0;
+      for (int k = 0; k < nb; ++k) r += s[k] < v;
+      perm[b0 + r] = v;
+    }
+  }
+}
+
 __global__ void k_perm_out(const unsigned long long* __restrict__ key2, int n, int64_t* __restrict__ perm) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) perm[i] = (int64_t)(key2[i] & 0xffffffffull);
@@ -142,6 +174,18 @@ struct Scratch {
 
 int cdiv(int64_t a, int b) { return (int)((a + b - 1) / b); }
 
+// `rows` runs of `count` ints, `dpitch` / `spitch` ints apart (one 2D copy
+// while the pitches are in its range).
+cudaError_t copy_rows(int* dst, size_t dpitch, const int* src, size_t spitch, size_t count, int rows,
+                      cudaMemcpyKind kind, cudaStream_t st) {
+  if (std::max(dpitch, spitch) * sizeof(int) < (1u << 31))
+    return cudaMemcpy2DAsync(dst, dpitch * sizeof(int), src, spitch * sizeof(int), count * sizeof(int), rows, kind, st);
+  cudaError_t e = cudaSuccess;
+  for (int r = 0; r < rows && e == cudaSuccess; ++r)
+    e = cudaMemcpyAsync(dst + r * dpitch, src + r * spitch, count * sizeof(int), kind, st);
+  return e;
+}
+
 }  // namespace
 
 #define TCK(call)                                              \
@@ -154,7 +198,7 @@ int cdiv(int64_t a, int b) { return (int)((a + b - 1) / b); }
   } while (0)
 
 int device_build_tree(const double* x_dev, const double* q_dev, int64_t n64, cudaStream_t st, Plan& plan,
-                      int64_t* d_perm, const TreeScratchFn& scratch, std::string& msg) {
+                      int64_t* d_perm, const TreeScratchFn& scratch, const PinnedFn& pinned, std::string& msg) {
   const Args& a = plan.args;
   const int n = (int)n64;
   plan.n = n64;
@@ -197,67 +241,92 @@ int device_build_tree(const double* x_dev, const double* q_dev, int64_t n64, cud
   tmp_bytes = std::max(tmp_bytes, t2);
   void* tmp = nullptr;
   TCK(B.get((char**)&tmp, tmp_bytes));
-  TCK(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, key_alt, idx, idx_alt, n, 0, 3 * kKeyLevels, st));
-  // sorted keys in key_alt, indices in idx_alt
-
-  // level arrays (a level has at most n cells)
-  int *lboff[2], *lbnum[2], *noct = nullptr, *npar = nullptr, *nchild = nullptr, *coff = nullptr;
-  for (int s = 0; s < 2; ++s) {
-    TCK(B.get(&lboff[s], n));
-    TCK(B.get(&lbnum[s], n));
+  // the staging of this build and of the walk that follows it in one
+  // allocation (pinned memory takes milliseconds to get): about 4 n / ncrit
+  // cells, more only for very uneven sets
+  if (!pinned(128 * std::min<size_t>((size_t)n, 64 + 4 * (size_t)n / a.ncrit))) {
+    msg = "pinned host allocation failed";
+    return kTreeError;
   }
-  TCK(B.get(&noct, n));
-  TCK(B.get(&npar, n));
-  TCK(B.get(&nchild, n));
-  TCK(B.get(&coff, n));
-  int zero = 0;
-  TCK(cudaMemcpyAsync(lboff[0], &zero, sizeof(int), cudaMemcpyHostToDevice, st));
-  TCK(cudaMemcpyAsync(lbnum[0], &n, sizeof(int), cudaMemcpyHostToDevice, st));
+  // level arrays (a level has at most n cells): [boff | bnum | octant | parent]
+  // of the cells of two levels in turn, and [children | their offsets]
+  int *lev[2], *cnt = nullptr;
+  for (int t = 0; t < 2; ++t) TCK(B.get(&lev[t], 4 * (size_t)n));
+  TCK(B.get(&cnt, 2 * (size_t)n));
+  int *nchild = cnt, *coff = cnt + n;
+  // sorted keys in key_alt, indices in idx_alt
+  int levels = std::min(kSortLevels, kKeyLevels);
+sort_again:
+  TCK(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, key_alt, idx, idx_alt, n, 3 * (kKeyLevels - levels),
+                                      3 * kKeyLevels, st));
+  plan.cells.resize(1);
+  plan.cells[0].coff = plan.cells[0].cnum = 0;
+  {
+    int* h = (int*)pinned(2 * sizeof(int));
+    if (!h) {
+      msg = "pinned host allocation failed";
+      return kTreeError;
+    }
+    h[0] = 0;
+    h[1] = n;
+    TCK(copy_rows(lev[0], n, h, 1, 1, 2, cudaMemcpyHostToDevice, st));
+    TCK(cudaStreamSynchronize(st));  // the staging is reused below
+  }
 
   size_t lev0 = 0, lev1 = 1;
   int cur = 0, depth = 0;
-  std::vector<int> h_nchild, h_coff, h_boff, h_bnum, h_oct, h_par;
   while (true) {
     const int nl = (int)(lev1 - lev0);
-    k_split_level<<<cdiv(nl, 128), 128, 0, st>>>(key_alt, lboff[cur], lbnum[cur], nl, a.ncrit, depth, nchild,
-                                                nullptr, 0, nullptr, nullptr, nullptr, nullptr, flags + 1);
+    const int* L = lev[cur];
+    int* X = lev[cur ^ 1];
+    k_split_level<<<cdiv(nl, 128), 128, 0, st>>>(key_alt, L, L + n, nl, a.ncrit, depth, nchild, nullptr, 0, nullptr,
+                                                nullptr, nullptr, nullptr, flags + 1);
     TCK(cudaGetLastError());
     TCK(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, nchild, coff, nl, st));
-    h_nchild.resize(nl);
-    h_coff.resize(nl);
-    int h_flags[2] = {0, 0};
-    TCK(cudaMemcpyAsync(h_nchild.data(), nchild, sizeof(int) * nl, cudaMemcpyDeviceToHost, st));
-    TCK(cudaMemcpyAsync(h_coff.data(), coff, sizeof(int) * nl, cudaMemcpyDeviceToHost, st));
-    TCK(cudaMemcpyAsync(h_flags, flags, sizeof(h_flags), cudaMemcpyDeviceToHost, st));
+    if (depth < levels) {
+      k_split_level<<<cdiv(nl, 128), 128, 0, st>>>(key_alt, L, L + n, nl, a.ncrit, depth, nchild, coff, 1, X, X + n,
+                                                  X + 2 * (size_t)n, X + 3 * (size_t)n, flags + 1);
+      TCK(cudaGetLastError());
+    }
+    // staging: flags, [children | offsets], then the child arrays
+    const int room = (int)std::min<int64_t>(n, 8 * (int64_t)nl), spec = std::min(room, kSpeculate);
+    int* h = (int*)pinned(sizeof(int) * (2 + 2 * (size_t)nl + 4 * (size_t)room));
+    if (!h) {
+      msg = "pinned host allocation failed";
+      return kTreeError;
+    }
+    int *h_nchild = h + 2, *h_coff = h_nchild + nl, *h_kid = h_coff + nl;
+    TCK(cudaMemcpyAsync(h, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    TCK(copy_rows(h_nchild, nl, nchild, n, nl, 2, cudaMemcpyDeviceToHost, st));
+    if (depth < levels)
+      TCK(copy_rows(h_kid, spec, X, n, spec, 4, cudaMemcpyDeviceToHost, st));
     TCK(cudaStreamSynchronize(st));
-    if (h_flags[0]) {
+    if (h[0]) {
       msg = "non-finite body position or charge";
       return kTreeError;
     }
-    if (h_flags[1]) return kTreeTooDeep;
+    if (h[1]) return kTreeTooDeep;
     const int total = h_coff[nl - 1] + h_nchild[nl - 1];
     if (total == 0) break;
-    k_split_level<<<cdiv(nl, 128), 128, 0, st>>>(key_alt, lboff[cur], lbnum[cur], nl, a.ncrit, depth, nchild,
-                                                coff, 1, lboff[cur ^ 1], lbnum[cur ^ 1], noct, npar, flags + 1);
-    TCK(cudaGetLastError());
-    h_boff.resize(total);
-    h_bnum.resize(total);
-    h_oct.resize(total);
-    h_par.resize(total);
-    TCK(cudaMemcpyAsync(h_boff.data(), lboff[cur ^ 1], sizeof(int) * total, cudaMemcpyDeviceToHost, st));
-    TCK(cudaMemcpyAsync(h_bnum.data(), lbnum[cur ^ 1], sizeof(int) * total, cudaMemcpyDeviceToHost, st));
-    TCK(cudaMemcpyAsync(h_oct.data(), noct, sizeof(int) * total, cudaMemcpyDeviceToHost, st));
-    TCK(cudaMemcpyAsync(h_par.data(), npar, sizeof(int) * total, cudaMemcpyDeviceToHost, st));
-    TCK(cudaStreamSynchronize(st));
+    if (depth >= levels) {  // deeper than the sorted digits
+      levels = kKeyLevels;
+      goto sort_again;
+    }
+    int ld = spec;
+    if (total > spec) {
+      ld = total;
+      TCK(copy_rows(h_kid, ld, X, n, ld, 4, cudaMemcpyDeviceToHost, st));
+      TCK(cudaStreamSynchronize(st));
+    }
     for (int k = 0; k < nl; ++k) {
       if (h_nchild[k] == 0) continue;
       plan.cells[lev0 + k].coff = (int)lev1 + h_coff[k];
       plan.cells[lev0 + k].cnum = h_nchild[k];
     }
     for (int j = 0; j < total; ++j) {
-      const Cell P = plan.cells[lev0 + h_par[j]];  // a copy: the push below may reallocate
+      const Cell P = plan.cells[lev0 + h_kid[3 * (size_t)ld + j]];  // a copy: the push below may reallocate
       Cell ch;
-      ch.octant = h_oct[j];
+      ch.octant = h_kid[2 * (size_t)ld + j];
       ch.depth = P.depth + 1;
       ch.r = P.r / 2;
       // Tree::get_child_cell_x, as the host build computes it
@@ -266,8 +335,8 @@ int device_build_tree(const double* x_dev, const double* q_dev, int64_t n64, cud
       ch.x[2] = P.x[2] + ((ch.octant & 1) ? P.r / 2 : -P.r / 2);
       ch.coff = 0;
       ch.cnum = 0;
-      ch.boff = h_boff[j];
-      ch.bnum = h_bnum[j];
+      ch.boff = h_kid[j];
+      ch.bnum = h_kid[(size_t)ld + j];
       plan.cells.push_back(ch);
     }
     lev0 = lev1;
@@ -278,25 +347,39 @@ int device_build_tree(const double* x_dev, const double* q_dev, int64_t n64, cud
   plan.ntree = (int)plan.cells.size();
 
   // input order inside each leaf
-  std::vector<int> lb, ln;
+  int nleaf = 0, largest = 0;
   for (const Cell& c : plan.cells)
     if (c.cnum == 0) {
-      lb.push_back(c.boff);
-      ln.push_back(c.bnum);
+      ++nleaf;
+      largest = std::max(largest, c.bnum);
     }
-  const int nleaf = (int)lb.size();
-  int *d_lb = nullptr, *d_ln = nullptr;
-  TCK(B.get(&d_lb, nleaf));
-  TCK(B.get(&d_ln, nleaf));
-  TCK(cudaMemcpyAsync(d_lb, lb.data(), sizeof(int) * nleaf, cudaMemcpyHostToDevice, st));
-  TCK(cudaMemcpyAsync(d_ln, ln.data(), sizeof(int) * nleaf, cudaMemcpyHostToDevice, st));
-  k_leaf_keys<<<std::min(nleaf, 4096), 128, 0, st>>>(d_lb, d_ln, nleaf, idx_alt, key);
-  TCK(cudaGetLastError());
-  int bits = 1;
-  while ((1ll << bits) < n64) ++bits;
-  TCK(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, key, key_alt, n, 0, 32 + bits, st));
-  k_perm_out<<<cdiv(n, 256), 256, 0, st>>>(key_alt, n, d_perm);
-  TCK(cudaGetLastError());
+  int* h = (int*)pinned(2 * sizeof(int) * (size_t)nleaf);
+  if (!h) {
+    msg = "pinned host allocation failed";
+    return kTreeError;
+  }
+  int l = 0;
+  for (const Cell& c : plan.cells)
+    if (c.cnum == 0) {
+      h[l] = c.boff;
+      h[nleaf + l++] = c.bnum;
+    }
+  int* d_lb = nullptr;
+  TCK(B.get(&d_lb, 2 * (size_t)nleaf));
+  TCK(cudaMemcpyAsync(d_lb, h, 2 * sizeof(int) * (size_t)nleaf, cudaMemcpyHostToDevice, st));
+  if (largest <= kRankMax) {
+    k_leaf_rank<<<std::min(nleaf, 148 * 64), 256, 0, st>>>(d_lb, d_lb + nleaf, nleaf, n, idx_alt, d_perm);
+    TCK(cudaGetLastError());
+  } else {
+    k_leaf_keys<<<std::min(nleaf, 4096), 128, 0, st>>>(d_lb, d_lb + nleaf, nleaf, idx_alt, key);
+    TCK(cudaGetLastError());
+    int bits = 1;
+    while ((1ll << bits) < n64) ++bits;
+    TCK(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, key, key_alt, n, 0, 32 + bits, st));
+    k_perm_out<<<cdiv(n, 256), 256, 0, st>>>(key_alt, n, d_perm);
+    TCK(cudaGetLastError());
+  }
+  TCK(cudaStreamSynchronize(st));  // the staging is reused by the caller
   return kTreeOk;
 }
 

@@ -19,6 +19,10 @@ constexpr int kTreeError = -1;   // CUDA error or non-finite position (msg says 
 // Device scratch by slot (0, 1, 2, ...): a buffer of at least `bytes`,
 // nullptr when none can be had.  The caller keeps the buffers between calls.
 using TreeScratchFn = std::function<void*(int slot, size_t bytes)>;
+// Pinned host staging of at least `bytes`, nullptr when none can be had; one
+// buffer, kept by the caller, whose contents do not outlive the next call
+// that asks for it.
+using PinnedFn = std::function<char*(size_t bytes)>;
 
 // Fills plan.cells (tree cells, breadth-first), plan.ntree, plan.n and
 // plan.r0 from n bodies in device memory (x_dev n x 3, q_dev n), with
@@ -27,7 +31,7 @@ using TreeScratchFn = std::function<void*(int slot, size_t bytes)>;
 // positions.  Work runs on `st`; the permutation may still be in flight on
 // return.  Non-finite positions or charges give kTreeError.
 int device_build_tree(const double* x_dev, const double* q_dev, int64_t n, cudaStream_t st, Plan& plan,
-                      int64_t* d_perm, const TreeScratchFn& scratch, std::string& msg);
+                      int64_t* d_perm, const TreeScratchFn& scratch, const PinnedFn& pinned, std::string& msg);
 
 // The P2P lists of the dual-tree walk from `roots` (traverse_begin) on the
 // GPU: the same entries in the same order as traverse_p2p, into plan.p2p
@@ -49,7 +53,7 @@ struct DeviceWalk {
   std::vector<V3> host_offs;  // the walks' offsets (roots' order)
 };
 int device_p2p_walk(Plan& plan, const std::vector<WalkRoot>& roots, cudaStream_t st, const TreeScratchFn& scratch,
-                    int slot_base, DeviceWalk* dw, std::string& msg, bool host_lists = true);
+                    const PinnedFn& pinned, int slot_base, DeviceWalk* dw, std::string& msg, bool host_lists = true);
 // plan.p2p from a walk left on the device (its pairs copied back).
 int device_walk_host_lists(const DeviceWalk& dw, Plan& plan, cudaStream_t st, std::string& msg);
 

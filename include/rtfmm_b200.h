@@ -56,9 +56,9 @@ typedef enum rtfmm_precision {
  * that per-stage times are those of each stage alone. */
 #define RTFMM_STAGE_SERIAL 4u
 /* Diagnostic bit: record per-stage events (rtfmm_b200_stage_times).  Without
- * it, and without RTFMM_STAGE_SERIAL, a forward pass is captured as a CUDA
- * graph on first use and replayed by every later call on the same device
- * tables; rtfmm_b200_stage_times then reports zeros. */
+ * it, and without RTFMM_STAGE_SERIAL, the second forward pass on the same
+ * device tables is captured as a CUDA graph, which every later call replays;
+ * rtfmm_b200_stage_times then reports zeros. */
 #define RTFMM_STAGE_TIMED 8u
 
 /*

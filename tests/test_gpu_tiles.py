@@ -78,3 +78,43 @@ def test_near_field_with_long_lists(pkg, oracle, images, precision):
                              divide_4pi=1).solve(stages="near")
     tol = 1e-5 if precision else 1e-12  # FP64: a sum of 2000 terms, ~1e-15 each
     assert l2(grad, rgrad) < tol and l2(phi, rphi) < tol
+
+
+# octrees below the first sorted digits (12 levels), and leaves above the size
+# ordered by counting (1500 bodies)
+@pytest.mark.parametrize("ncrit,scale", [(4, 2e-4), (1500, 1.0)])
+def test_device_tree_beyond_its_fast_paths(pkg, ncrit, scale):
+    x, q = uniform01(6000, 8)
+    x = 0.3 + scale * (x - 0.3)
+    a = args(pkg, 4, ncrit, 1, 1)
+    h = pkg.LaplaceFMM(x, q, a)
+    h.setup()
+    d = pkg.LaplaceFMM(x, q, a)
+    xd, qd = torch.from_numpy(x).cuda(), torch.from_numpy(q).cuda()
+    torch.cuda.synchronize()
+    for _ in range(2):  # a second set-up reuses every buffer
+        d.setup_device(xd.data_ptr(), qd.data_ptr(), len(q))
+    if ncrit == 4:
+        assert h.info()["depth_max"] > 10
+    assert all(np.array_equal(u, v) for u, v in zip(h.cells(), d.cells()))
+    assert np.array_equal(h.perm(), d.perm())
+    assert all(np.array_equal(u, v) for u, v in zip(h.leaf_lists(), d.leaf_lists()))
+    ph, gh = h.evaluate()
+    d.evaluate_device()
+    pd, gd = d.download()
+    assert np.array_equal(ph, pd) and np.array_equal(gh, gd)
+    h.close()
+    d.close()
+
+
+# the first pass of a plan is issued launch by launch, the second captured,
+# the third replayed: the same outputs
+@pytest.mark.parametrize("precision", [0, 1])
+def test_first_pass_equals_replayed_ones(pkg, precision):
+    x, q = uniform01(5000, 9)
+    f = pkg.LaplaceFMM(x, q, args(pkg, 5, 40, 2, precision))
+    first = f.solve()
+    for _ in range(3):
+        again = f.evaluate()
+        assert all(np.array_equal(u, v) for u, v in zip(first, again))
+    f.close()
