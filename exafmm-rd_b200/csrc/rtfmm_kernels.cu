@@ -834,29 +834,43 @@ __global__ void __launch_bounds__(kGThreads) k_apply_f64_tc(ApplyBatch b) {
   for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
+  // the warp's column tiles are every other 8 of the block's 64, so that a
+  // block at the end of ns (24 of 64 columns at ns = 152, 40 at 296) splits
+  // its tiles over both column warps; the ones past ns are not multiplied
+  const int nv = min(4, max(0, (ns - c0 - 8 * wn + 15) / 16));
 #pragma unroll
   for (int st = 0; st < kGStages - 1; ++st) {
     if (st < total) issue(st);
     cp_async_commit();
   }
+  auto step = [&](int kt, auto nvc) {
+    constexpr int NV = decltype(nvc)::value;
+    const double* as = As + (kt % kGStages) * kAStage + (wm * 32 + (lane >> 2)) * kAPitch + (lane & 3);
+    const double* bs = Bs + (kt % kGStages) * kBStage + (lane & 3) * kBPitch + wn * 8 + (lane >> 2);
+#pragma unroll
+    for (int k4 = 0; k4 < kGK; k4 += 4) {
+      double fa[4], fb[NV];
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) fa[mt] = as[mt * 8 * kAPitch + k4];
+#pragma unroll
+      for (int nt = 0; nt < NV; ++nt) fb[nt] = bs[k4 * kBPitch + nt * 16];
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NV; ++nt) dmma8x8x4(acc[mt][nt], fa[mt], fb[nt]);
+    }
+  };
   for (int kt = 0; kt < total; ++kt) {
     cp_async_wait<kGStages - 2>();
     __syncthreads();  // step kt is in shared memory; step kt-1's buffer is free
     if (kt + kGStages - 1 < total) issue(kt + kGStages - 1);
     cp_async_commit();
-    const double* as = As + (kt % kGStages) * kAStage + (wm * 32 + (lane >> 2)) * kAPitch + (lane & 3);
-    const double* bs = Bs + (kt % kGStages) * kBStage + (lane & 3) * kBPitch + wn * 32 + (lane >> 2);
-#pragma unroll
-    for (int k4 = 0; k4 < kGK; k4 += 4) {
-      double fa[4], fb[4];
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt) fa[mt] = as[mt * 8 * kAPitch + k4];
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) fb[nt] = bs[k4 * kBPitch + nt * 8];
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) dmma8x8x4(acc[mt][nt], fa[mt], fb[nt]);
+    switch (nv) {  // warp-uniform
+      case 4: step(kt, std::integral_constant<int, 4>()); break;
+      case 3: step(kt, std::integral_constant<int, 3>()); break;
+      case 2: step(kt, std::integral_constant<int, 2>()); break;
+      case 1: step(kt, std::integral_constant<int, 1>()); break;
+      default: break;
     }
   }
   cp_async_wait<0>();
@@ -869,7 +883,7 @@ __global__ void __launch_bounds__(kGThreads) k_apply_f64_tc(ApplyBatch b) {
     const double sc = b.scale ? b.scale[row] : 1.0;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      const int n = c0 + wn * 32 + nt * 8 + 2 * (lane & 3);
+      const int n = c0 + (2 * nt + wn) * 8 + 2 * (lane & 3);
       if (n >= ns) continue;  // n even, ns even: n + 1 < ns as well
       double2* cp = reinterpret_cast<double2*>(b.C + (size_t)o * ns + n);
       double2 v = make_double2(sc * acc[mt][nt][0], sc * acc[mt][nt][1]);

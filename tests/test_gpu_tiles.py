@@ -118,3 +118,35 @@ def test_first_pass_equals_replayed_ones(pkg, precision):
         again = f.evaluate()
         assert all(np.array_equal(u, v) for u, v in zip(first, again))
     f.close()
+
+
+# 15000 leaves run their operators in 64 x 64 tiles, a sixteenth of them in
+# 16 x 32 ones: every body's outputs are the same bit for bit
+def test_small_and_large_operator_tiles_agree(pkg):
+    x, q = uniform01(30000, 10)
+    a, n, R = args(pkg, 6, 4, 0, 0), 30000, 16
+    f = pkg.LaplaceFMM(x, q, a)
+    f.setup()
+    phi, grad = f.evaluate()
+    f.close()
+    hs = []
+    for r in range(R):
+        f = pkg.LaplaceFMM(x, q, a)
+        f.shard(r, R)
+        f.setup()
+        f.upload()
+        hs.append(f)
+    total = torch.zeros(hs[0].shard_sizes()[1], dtype=torch.float64, device="cuda")
+    for f in hs:
+        buf = torch.zeros_like(total)
+        torch.cuda.synchronize()
+        f.shard_upward(buf.data_ptr())  # returns when buf is complete
+        total += buf
+    p = torch.zeros(n, dtype=torch.float64, device="cuda")
+    g = torch.zeros((n, 3), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    for f in hs:
+        f.shard_downward(total.data_ptr(), p.data_ptr(), g.data_ptr())
+        idx = f.shard_bodies()
+        assert np.array_equal(p.cpu().numpy()[idx], phi[idx]) and np.array_equal(g.cpu().numpy()[idx], grad[idx])
+        f.close()
