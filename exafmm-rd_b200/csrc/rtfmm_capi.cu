@@ -512,7 +512,8 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
     return k;
   };
   f->list_off.assign(nlf + 1, 0);
-  std::vector<int> item_off(nlf + 1, 0), bodies(nlf, 0);
+  std::vector<int> item_off(nlf + 1, 0);
+  std::vector<int64_t> bodies(nlf, 0);
   unsigned long long work = 0;
 #pragma omp parallel for schedule(dynamic, 64) reduction(+ : work)
   for (int l = 0; l < nlf; ++l) {
@@ -533,7 +534,7 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
   const int part = p2p_part_bodies(work);
   std::vector<int> slot_off(nlf + 1, 0);
   for (int l = 0; l < nlf; ++l) {
-    const int groups = (f->leaves[l].bnum + 31) / 32, nparts = std::max(1, (bodies[l] + part - 1) / part);
+    const int groups = (f->leaves[l].bnum + 31) / 32, nparts = (int)std::max<int64_t>(1, (bodies[l] + part - 1) / part);
     f->list_off[l + 1] += f->list_off[l];
     item_off[l + 1] = item_off[l] + groups * nparts;
     slot_off[l + 1] = slot_off[l] + (nparts > 1 ? groups * nparts : 0);
@@ -558,9 +559,10 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
     // times the parts of the list: part p starts at the first entry with
     // p/nparts of the bodies before it
     const int groups = (T.bnum + 31) / 32, nparts = groups ? (item_off[l + 1] - item_off[l]) / groups : 0;
-    int before = 0, next = 0;  // bodies of the entries so far, parts begun
+    int64_t before = 0;  // bodies of the entries so far
+    int next = 0;        // parts begun
     auto begin_parts = [&](int entry, bool end) {
-      for (; next < nparts && (end || before >= (int64_t)next * bodies[l] / nparts); ++next)
+      for (; next < nparts && (end || before >= next * bodies[l] / nparts); ++next)
         for (int g = 0; g < groups; ++g) {
           const int rem = std::min(32, T.bnum - 32 * g);
           int lw = 5;

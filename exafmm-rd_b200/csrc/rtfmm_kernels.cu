@@ -39,8 +39,15 @@
 #ifndef P2P_WARPS
 #define P2P_WARPS 1
 #endif
+// FP64 P2P: the same
+#ifndef P2P64_UNROLL
+#define P2P64_UNROLL 4
+#endif
+#ifndef P2P64_MINB
+#define P2P64_MINB 28
+#endif
 #ifndef P2P_FLUSH
-#define P2P_FLUSH 4
+#define P2P_FLUSH 1
 #endif
 // FP32 Hadamard: targets per thread, directions per FP32 partial sum,
 // resident blocks per SM
@@ -193,11 +200,15 @@ __global__ void k_body_leaf(const LeafInfo* __restrict__ leaves, int nleaf, int 
 // depend on which one that is.  Measured: 150001 bodies in blobs (longest list
 // 60593 bodies, mean 1435), FP64, 3.98 -> 0.50 ms; 30011 in blobs, FP32,
 // 0.36 -> 0.052; 2^22 in blobs, FP32, 13.0 -> 8.2; uniform 2^20, ncrit = 256:
-// FP32 3.13 -> 3.07, FP64 9.28 -> 8.14 (24 -> 18 FP64 operations a pair).
-// FP32: bound by the FMA pipe (65% busy, 13 operations and one rsqrt a pair).
+// FP32 3.13 -> 3.12, FP64 9.28 -> 7.68 (24 -> 18 FP64 operations a pair).
+// FP32: bound by the register reads of the packed FMAs (3 cycles each measured,
+// 31 a pair of sources with the 2-cycle additions and products); each tile's 32
+// sources go into FP64 (every four tiles: 3.07 ms, but the gradient's error
+// against FP64 2.8 times as large).  FP64: bound by dependent operations (pipe
+// 66% busy); 28 resident warps 7.68 ms, 20 7.94, 24 8.04, 32 7.76.
 // ---------------------------------------------------------------------------
 constexpr int kP2PWarps = P2P_WARPS;
-constexpr int kP2PUnroll = P2P_UNROLL;
+constexpr int kP2PUnroll = P2P_UNROLL, kP2PUnroll64 = P2P64_UNROLL;
 constexpr int kP2PFlush = P2P_FLUSH;  // tiles summed in FP32 before they go into FP64
 
 // A chunk of up to 32 list entries, one per lane: `start` is the lane's
@@ -379,10 +390,10 @@ __device__ __forceinline__ void p2p32_item(const float4* __restrict__ body32, co
       p2p32_tile<G, false, false>(sw, grp, (cnt + 1) >> 1, px, py, pz, p, fx, fy, fz);
     if (++tiles == kP2PFlush || !more) {
       tiles = 0;
-      P += (double)p.x + (double)p.y;
-      Gx += (double)fx.x + (double)fx.y;
-      Gy += (double)fy.x + (double)fy.y;
-      Gz += (double)fz.x + (double)fz.y;
+      P += (double)(p.x + p.y);
+      Gx += (double)(fx.x + fx.y);
+      Gy += (double)(fy.x + fy.y);
+      Gz += (double)(fz.x + fz.y);
       p = fx = fy = fz = make_float2(0.f, 0.f);
     }
   }
@@ -465,7 +476,7 @@ __device__ __forceinline__ void p2p64_item(const double4* __restrict__ body64, c
       }
     }
     if (more) stage(base);
-#pragma unroll 4
+#pragma unroll kP2PUnroll64
     for (int k = grp; k < cnt; k += G) {
       const double4 s = sw[k];
       const double dx = xt.x - s.x, dy = xt.y - s.y, dz = xt.z - s.z;
@@ -488,7 +499,7 @@ __device__ __forceinline__ void p2p64_item(const double4* __restrict__ body64, c
   p2p_store(it, active && grp == 0, ti, P, Gx, Gy, Gz, part, done, phi, grad);
 }
 
-__global__ void __launch_bounds__(32 * kP2PWarps)
+__global__ void __launch_bounds__(32 * kP2PWarps, P2P64_MINB)
     k_p2p64(const double4* __restrict__ body64, const P2PItem* __restrict__ items, int nitems,
             const P2PSrc64* __restrict__ list, double4* __restrict__ part, int* __restrict__ done,
             double* __restrict__ phi, double* __restrict__ grad) {

@@ -440,13 +440,14 @@ __device__ __forceinline__ void leaf_run(const LeafTables& T, int c, int* lo, in
 
 // cnt: list entries of leaf l; bodies: bodies of those entries; work: their
 // sum over the leaves, times the leaf's target groups.
-__global__ void k_leaf_list_count(LeafTables T, int* __restrict__ cnt, int* __restrict__ bodies,
+__global__ void k_leaf_list_count(LeafTables T, int* __restrict__ cnt, long long* __restrict__ bodies,
                                   unsigned long long* __restrict__ work) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= T.nlf) return;
   int path[kMaxPathLen];
   const int np = leaf_path(T, T.leaves[l].cell, path);
-  int c = 0, nb = 0;
+  int c = 0;
+  long long nb = 0;
   for (int i = 0; i < np; ++i)
     for (int e = T.cstart[path[i]]; e < T.cend[path[i]]; ++e) {
       const int sc = (int)((T.pairs[e] >> 5) & ((1ull << kCellBits) - 1));
@@ -461,16 +462,16 @@ __global__ void k_leaf_list_count(LeafTables T, int* __restrict__ cnt, int* __re
 }
 
 // Work items of leaf l: its target groups of 32 times the parts of its list.
-__global__ void k_leaf_item_count(LeafTables T, const int* __restrict__ bodies,
+__global__ void k_leaf_item_count(LeafTables T, const long long* __restrict__ bodies,
                                   const unsigned long long* __restrict__ work, int* __restrict__ icnt) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= T.nlf) return;
   const int S = p2p_part_bodies(*work);
-  icnt[l] = (T.leaves[l].bnum + 31) / 32 * max(1, (bodies[l] + S - 1) / S);
+  icnt[l] = (T.leaves[l].bnum + 31) / 32 * (int)max(1ll, (bodies[l] + S - 1) / S);
 }
 
 __global__ void k_leaf_list_fill(LeafTables T, const int* __restrict__ off, const int* __restrict__ ioff,
-                                 const int* __restrict__ bodies, int mixed, P2PSrc32* __restrict__ l32,
+                                 const long long* __restrict__ bodies, int mixed, P2PSrc32* __restrict__ l32,
                                  P2PSrc64* __restrict__ l64, P2PItem* __restrict__ items,
                                  unsigned long long* __restrict__ pair_total, int* __restrict__ nslots) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
@@ -485,9 +486,10 @@ __global__ void k_leaf_list_fill(LeafTables T, const int* __restrict__ off, cons
   // p starts at the first entry with p/nparts of the bodies before it
   const int groups = (Tl.bnum + 31) / 32, nparts = groups ? (ioff[l + 1] - ioff[l]) / groups : 0;
   const int slot0 = nparts > 1 ? atomicAdd(nslots, groups * nparts) : 0;
-  int before = 0, next = 0;  // bodies of the entries so far, parts begun
+  long long before = 0;  // bodies of the entries so far
+  int next = 0;          // parts begun
   auto begin_parts = [&](int entry, bool end) {
-    for (; next < nparts && (end || before >= (long long)next * bodies[l] / nparts); ++next)
+    for (; next < nparts && (end || before >= next * bodies[l] / nparts); ++next)
       for (int g = 0; g < groups; ++g) {
         const int rem = min(32, Tl.bnum - 32 * g);
         int lw = 5;
@@ -549,7 +551,8 @@ int device_p2p_tables(const DeviceWalk& w, const DeviceLeafInput& in, bool mixed
                       std::string& msg) {
   Scratch S{scratch, slot_base};
   const int nlf = in.nlf;
-  int *cstart, *cend, *cnt, *icnt, *off, *ioff, *bodies;
+  int *cstart, *cend, *cnt, *icnt, *off, *ioff;
+  long long* bodies;
   unsigned long long* total;  // body pairs, work, slots
   LCK(S.get(0, &cstart, w.ncell));
   LCK(S.get(1, &cend, w.ncell));
