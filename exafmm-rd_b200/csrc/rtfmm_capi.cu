@@ -198,12 +198,16 @@ struct rtfmm_fmm {
   // tables, the setup call, and the upload of the device tables (in the call
   // that did it)
   double setup_s[12] = {};
-  // the forward pass captured as a CUDA graph (launch_pass), dropped with
-  // the device tables
-  cudaGraphExec_t pass_graph = nullptr;
+  // the forward pass and the adjoint's transposed pass captured as CUDA
+  // graphs (issue_pass), dropped with the device tables
+  struct PassGraph {
+    cudaGraphExec_t exec = nullptr;
+    bool seen = false;  // the pass has run on these device tables
+    bool grad_q_valid = false;
+    int64_t launches = 0;
+  };
+  PassGraph g_forward, g_adjoint;
   bool pass_direct = false;  // the last forward pass was issued launch by launch
-  bool pass_seen = false;    // a forward pass ran on these device tables
-  bool graph_grad_q_valid = false;
   cudaEvent_t ev_g0 = nullptr, ev_g1 = nullptr;
   // the 8x8 FFT-M2L (up, Hadamard, down) runs in FP32: the mixed form at P <= 8
   bool m2l32 = false;
@@ -325,9 +329,9 @@ struct PlanPack {
 };
 
 void drop_graph(rtfmm_fmm* f) {
-  if (f->pass_graph) {
-    cudaGraphExecDestroy(f->pass_graph);
-    f->pass_graph = nullptr;
+  for (rtfmm_fmm::PassGraph* g : {&f->g_forward, &f->g_adjoint}) {
+    if (g->exec) cudaGraphExecDestroy(g->exec);
+    *g = rtfmm_fmm::PassGraph();
   }
 }
 
@@ -336,7 +340,6 @@ void drop_graph(rtfmm_fmm* f) {
 // use).  The buffers themselves stay in the pool.
 void drop_allocs(rtfmm_fmm* f) {
   drop_graph(f);
-  f->pass_seen = false;
   f->close_valid = false;
   f->n_close = 0;
   f->d_adj_q = f->d_adj_gq = f->d_adj_gw = f->d_adj_w = f->d_adj_dq = f->d_adj_dx = nullptr;
@@ -1126,6 +1129,12 @@ int run_apply(rtfmm_fmm* f, const ApplyCall& c, bool adjoint = false) {
   return RTFMM_OK;
 }
 
+// Passes are captured and replayed (issue_pass) unless the stage timing or
+// serial diagnostics ask for direct launches.
+bool use_graph(const rtfmm_fmm* f) {
+  return USE_PASS_GRAPH && !(f->args.stages & (RTFMM_STAGE_SERIAL | RTFMM_STAGE_TIMED));
+}
+
 // One evaluation pass on the device-resident bodies (d_body64).  With
 // `adjoint` the pass applies the transposed operator chain to the body
 // charges (which then hold the weights w): P2P, M2L and the tree-level
@@ -1150,6 +1159,8 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
   const bool serial = stages & RTFMM_STAGE_SERIAL;
   cudaStream_t s0 = f->s0, s1 = serial ? f->s0 : f->s1;
   const bool up = phase != 2, down = phase != 1;
+  const bool timed = !use_graph(f);  // the stages' events, where they are read
+  auto stage_end = [&](Stage k) { return timed ? cudaEventRecord(f->ev_st[k], s0) : cudaSuccess; };
   f->launches = 0;
   if (phase == 1) {
     // the bodies of other ranks' leaves get no P2P or L2P here: zero outputs
@@ -1188,7 +1199,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
     int rc = near_field();
     if (rc) return rc;
   }
-  if (up) CK(cudaEventRecord(f->ev_st[ST_PREP], s0));
+  if (up) CK(stage_end(ST_PREP));
   if (far && phase == 0) CK(cudaMemsetAsync(f->d_pchk, 0, sizeof(double) * p.cells.size() * ns, s0));
   if (far && up) {
     CK(launch_p2m_check(f->d_body64, f->d_leaves_own, nleaf, f->d_surf_unit, ns, f->d_leafvec, s0,
@@ -1198,7 +1209,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
       int rc = run_apply(f, c);
       if (rc) return rc;
     }
-    CK(cudaEventRecord(f->ev_st[ST_P2M], s0));
+    CK(stage_end(ST_P2M));
   }
   if (phase == 1) {
     // every leaf's q_equiv row into the exchange buffer (others' rows zero)
@@ -1220,7 +1231,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
       int rc = run_apply(f, c, adjoint);
       if (rc) return rc;
     }
-    CK(cudaEventRecord(f->ev_st[ST_M2M], s0));
+    CK(stage_end(ST_M2M));
     const int nup8 = (int)f->up8_items.size() / 10, nup27 = (int)f->up27_items.size() / 10;
     const int ndn8 = (int)f->down8_items.size() / 10, ndn27 = (int)f->down27_items.size() / 10;
     if (f->m2l32) {
@@ -1233,7 +1244,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
     CK(launch_m2l_up<double>(f->d_qeq, f->d_up27, nup27, f->d_surf_ijk, f->d_twiddle, P, ns, f->nS27,
                              f->sp_up27, f->d_Q27, s0));
     f->launches += (nup8 > 0) + (nup27 > 0);
-    CK(cudaEventRecord(f->ev_st[ST_UP], s0));
+    CK(stage_end(ST_UP));
     if (f->m2l32) {
       CK(launch_m2l_hadamard8((const float*)f->d_Q8, (const float*)f->d_G8, f->d_tsrc8, f->nT8, f->nS8,
                                      Nf, (float*)f->d_Pk8, s0));
@@ -1243,7 +1254,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
     }
     CK(launch_m2l_hadamard27(f->d_Q27, f->d_G27, f->d_tsrc27, f->nT27, f->nS27, Nf, f->d_Pk27, s0));
     f->launches += (f->nT8 > 0) + (f->nT27 > 0);
-    CK(cudaEventRecord(f->ev_st[ST_HAD], s0));
+    CK(stage_end(ST_HAD));
     if (f->m2l32) {
       CK(launch_m2l_down<float>((const float*)f->d_Pk8, f->d_down8, f->d_tscale8, ndn8, f->d_surf_ijk,
                                 f->d_twiddle, P, ns, f->nT8, f->sp_down8, f->d_pchk, s0));
@@ -1254,12 +1265,12 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
     CK(launch_m2l_down<double>(f->d_Pk27, f->d_down27, f->d_tscale27, ndn27, f->d_surf_ijk, f->d_twiddle, P, ns,
                                f->nT27, f->sp_down27, f->d_pchk, s0));
     f->launches += (ndn8 > 0) + (ndn27 > 0);
-    CK(cudaEventRecord(f->ev_st[ST_DOWN], s0));
+    CK(stage_end(ST_DOWN));
     for (auto& c : f->l2l_calls) {
       int rc = run_apply(f, c, adjoint);
       if (rc) return rc;
     }
-    CK(cudaEventRecord(f->ev_st[ST_L2L], s0));
+    CK(stage_end(ST_L2L));
     for (auto& c : f->l2p_call) {
       int rc = run_apply(f, c);
       if (rc) return rc;
@@ -1267,16 +1278,16 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
     CK(launch_l2p_eval(f->d_body64, f->d_leaves_own, nleaf, f->d_surf_unit, ns, f->d_leafvec2, f->d_far_phi,
                        f->d_far_grad, s0, !mixed));
     f->launches++;
-    CK(cudaEventRecord(f->ev_st[ST_L2P], s0));
+    CK(stage_end(ST_L2P));
   } else {
-    for (int k = ST_P2M; k <= ST_L2P; ++k) CK(cudaEventRecord(f->ev_st[k], s0));
+    for (int k = ST_P2M; k <= ST_L2P; ++k) CK(stage_end((Stage)k));
   }
   if (near && serial) {
     int rc = near_field();
     if (rc) return rc;
   }
   if (near && !serial) CK(cudaStreamWaitEvent(s0, f->ev_near, 0));
-  CK(cudaEventRecord(f->ev_st[ST_P2P], s0));
+  CK(stage_end(ST_P2P));
   const Args& a = f->args;
   const int dipole = (adjoint || no_dipole) ? 0 : a.dipole_correction;
   if (dipole) {
@@ -1288,7 +1299,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
                  f->d_body64, f->d_perm, n, f->d_dip, coef, dipole, a.x.data(),
                  a.divide_4pi ? 1.0 / (4 * M_PI) : 1.0, f->d_out_phi, f->d_out_grad, s0));
   f->launches++;
-  CK(cudaEventRecord(f->ev_st[ST_POST], s0));
+  CK(stage_end(ST_POST));
   CK(cudaEventRecord(f->ev_stop, s0));
   f->grad_q_valid = !adjoint && dipole == 0 && near && far;
   return RTFMM_OK;
@@ -1353,50 +1364,57 @@ int collect_times(rtfmm_fmm* f, float* total) {
   return RTFMM_OK;
 }
 
-// The forward pass as a CUDA graph: captured by the second pass on a set of
-// device tables (a single pass, as in a solve or a time step, is cheaper
-// issued launch by launch than captured and instantiated, 0.3 ms less for a
-// solve of 1000 bodies) and
-// replayed with one launch from then on (the launches, their arguments and the
-// two-stream fork/join are fixed by the plan; charges, positions and outputs
-// live in the handle's buffers).  Kernel nodes keep the priority
-// of the stream they were captured from, so the far-field chain still
+// A pass as a CUDA graph (the forward pass, and the adjoint's transposed pass
+// the same way): captured by the second pass on a set of device tables (a
+// single pass, as in a solve or a time step, is cheaper issued launch by
+// launch than captured and instantiated, by 0.3 ms for a solve of 1000
+// bodies) and replayed with one launch from then on (the launches, their
+// arguments and the two-stream fork/join are fixed by the plan; charges,
+// positions and outputs live in the handle's buffers).  Kernel nodes keep the
+// priority of the stream they were captured from, so the far-field chain still
 // preempts P2P.  Per-stage events are not recorded in a replay: the stage
-// timing and serial diagnostics (RTFMM_STAGE_TIMED, RTFMM_STAGE_SERIAL)
-// issue the launches directly.
-bool use_graph(const rtfmm_fmm* f) {
-  return USE_PASS_GRAPH && !(f->args.stages & (RTFMM_STAGE_SERIAL | RTFMM_STAGE_TIMED));
+// timing and serial diagnostics (RTFMM_STAGE_TIMED, RTFMM_STAGE_SERIAL) issue
+// the launches directly.
+
+// Enqueues a pass on s0: its launches directly the first time, else its graph.
+int issue_pass(rtfmm_fmm* f, bool adjoint, bool direct) {
+  rtfmm_fmm::PassGraph& g = adjoint ? f->g_adjoint : f->g_forward;
+  g.seen = true;
+  if (direct) return enqueue_pass(f, adjoint);
+  if (!g.exec) {
+    cudaGraph_t graph = nullptr;
+    CK(cudaStreamBeginCapture(f->s0, cudaStreamCaptureModeThreadLocal));
+    int rc = enqueue_pass(f, adjoint);
+    cudaError_t e = cudaStreamEndCapture(f->s0, &graph);
+    if (rc) {
+      if (graph) cudaGraphDestroy(graph);
+      return rc;
+    }
+    if (e != cudaSuccess) return fail(RTFMM_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    e = cudaGraphInstantiateWithFlags(&g.exec, graph, cudaGraphInstantiateFlagUseNodePriority);
+    cudaGraphDestroy(graph);
+    if (e != cudaSuccess) {
+      g.exec = nullptr;
+      return fail(RTFMM_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+    }
+    g.grad_q_valid = f->grad_q_valid;
+    g.launches = f->launches;
+  }
+  CK(cudaGraphLaunch(g.exec, f->s0));
+  f->grad_q_valid = g.grad_q_valid;
+  f->launches = g.launches;
+  return RTFMM_OK;
 }
 
 // Enqueues one forward pass on s0 (graph replay or direct launches).
 int launch_pass(rtfmm_fmm* f) {
-  int rc0 = ensure_close_pairs(f);
-  if (rc0) return rc0;
-  f->pass_direct = !use_graph(f) || !f->pass_seen;
-  f->pass_seen = true;
-  if (f->pass_direct) return enqueue_pass(f);
-  if (!f->pass_graph) {
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(f->s0, cudaStreamCaptureModeThreadLocal));
-    int rc = enqueue_pass(f);
-    cudaError_t e = cudaStreamEndCapture(f->s0, &g);
-    if (rc) {
-      if (g) cudaGraphDestroy(g);
-      return rc;
-    }
-    if (e != cudaSuccess) return fail(RTFMM_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiateWithFlags(&f->pass_graph, g, cudaGraphInstantiateFlagUseNodePriority);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) {
-      f->pass_graph = nullptr;
-      return fail(RTFMM_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    }
-    f->graph_grad_q_valid = f->grad_q_valid;
-  }
+  int rc = ensure_close_pairs(f);
+  if (rc) return rc;
+  f->pass_direct = !use_graph(f) || !f->g_forward.seen;
+  if (f->pass_direct) return issue_pass(f, false, true);
   CK(cudaEventRecord(f->ev_g0, f->s0));
-  CK(cudaGraphLaunch(f->pass_graph, f->s0));
+  if ((rc = issue_pass(f, false, false))) return rc;
   CK(cudaEventRecord(f->ev_g1, f->s0));
-  f->grad_q_valid = f->graph_grad_q_valid;
   return RTFMM_OK;
 }
 
@@ -1933,7 +1951,7 @@ int adjoint_core(rtfmm_fmm* f, const double* w, double* dq, double* dx) {
   const bool have_gq = f->grad_q_valid;
   if (have_gq) CK(cudaMemcpyAsync(f->d_adj_gq, f->d_out_grad, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s0));
   CK(launch_swap_charges(f->d_body64, w, f->d_perm, n, f->d_adj_q, s0));
-  rc = enqueue_pass(f, true);
+  rc = issue_pass(f, true, !use_graph(f) || !f->g_adjoint.seen);
   if (rc) return rc;
   if (dq) CK(cudaMemcpyAsync(dq, f->d_out_phi, sizeof(double) * n, cudaMemcpyDeviceToDevice, s0));
   CK(launch_restore_charges(f->d_body64, f->d_adj_q, n, s0));

@@ -150,3 +150,20 @@ def test_small_and_large_operator_tiles_agree(pkg):
         idx = f.shard_bodies()
         assert np.array_equal(p.cpu().numpy()[idx], phi[idx]) and np.array_equal(g.cpu().numpy()[idx], grad[idx])
         f.close()
+
+
+# a forward and backward step repeated on one set-up: the adjoint's transposed
+# pass is issued launch by launch, then captured, then replayed, with other
+# weights each time
+@pytest.mark.parametrize("precision", [0, 1])
+def test_repeated_adjoints_agree(pkg, precision):
+    x, q = uniform01(6000, 11)
+    f = pkg.LaplaceFMM(x, q, args(pkg, 5, 40, 1, precision))
+    f.setup()
+    w = [np.random.default_rng(k).standard_normal(len(q)) for k in (1, 2)]
+    first = [f.adjoint(v) for v in w]
+    for _ in range(2):
+        f.evaluate(q)
+        for v, ref in zip(w, first):
+            assert all(np.array_equal(a, b) for a, b in zip(f.adjoint(v), ref))
+    f.close()
