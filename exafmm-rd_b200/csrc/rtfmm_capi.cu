@@ -4,6 +4,8 @@
 //   stream s0 (far field):  P2M -> M2M levels -> FFT-M2L (up, Hadamard, down)
 //                           -> L2L levels -> L2P            ... then post
 //   stream s1 (near field): P2P, concurrently with the far field
+//   stream s2 (image levels): their M2M, 1x27 FFT-M2L and L2L, concurrently
+//                           with the 8x8 FFT-M2L
 //
 // This is LaplaceFMM::solve (3dpp/src/fmm.cpp:13-81) split at its hot block.
 #include <chrono>
@@ -132,7 +134,8 @@ struct rtfmm_fmm {
 
   // device
   int dev = -1;
-  cudaStream_t s0 = nullptr, s1 = nullptr;
+  cudaStream_t s0 = nullptr, s1 = nullptr, s2 = nullptr;
+  cudaEvent_t ev_img0 = nullptr, ev_img1 = nullptr;  // the image levels' fork and join
   cudaEvent_t ev_start = nullptr, ev_near0 = nullptr, ev_near = nullptr, ev_stop = nullptr;
   cudaEvent_t ev_st[ST_N] = {};
   // device buffers by the handle field that holds them, kept across set-ups
@@ -366,9 +369,10 @@ void free_device(rtfmm_fmm* f) {
   f->flush_bytes = 0;
   if (f->s0) cudaStreamDestroy(f->s0);
   if (f->s1) cudaStreamDestroy(f->s1);
-  f->s0 = f->s1 = nullptr;
+  if (f->s2) cudaStreamDestroy(f->s2);
+  f->s0 = f->s1 = f->s2 = nullptr;
   cudaEvent_t* evs[] = {&f->ev_start, &f->ev_near0, &f->ev_near, &f->ev_stop, &f->ev_adj0, &f->ev_adj1,
-                        &f->ev_g0, &f->ev_g1};
+                        &f->ev_g0, &f->ev_g1, &f->ev_img0, &f->ev_img1};
   for (auto e : evs)
     if (*e) {
       cudaEventDestroy(*e);
@@ -845,9 +849,11 @@ int ensure_device(rtfmm_fmm* f) {
 #if STREAM_PRIO
     CK(cudaStreamCreateWithPriority(&f->s0, cudaStreamNonBlocking, prio_hi));
     CK(cudaStreamCreateWithPriority(&f->s1, cudaStreamNonBlocking, prio_lo));
+    CK(cudaStreamCreateWithPriority(&f->s2, cudaStreamNonBlocking, prio_hi));
 #else
     CK(cudaStreamCreateWithFlags(&f->s0, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&f->s1, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&f->s2, cudaStreamNonBlocking));
 #endif
     CK(cudaEventCreate(&f->ev_start));
     CK(cudaEventCreate(&f->ev_near0));
@@ -857,6 +863,8 @@ int ensure_device(rtfmm_fmm* f) {
     CK(cudaEventCreate(&f->ev_adj1));
     CK(cudaEventCreate(&f->ev_g0));
     CK(cudaEventCreate(&f->ev_g1));
+    CK(cudaEventCreateWithFlags(&f->ev_img0, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&f->ev_img1, cudaEventDisableTiming));
     for (int k = 0; k < ST_N; ++k) CK(cudaEventCreate(&f->ev_st[k]));
   } else {
     CK(cudaSetDevice(f->dev));
@@ -1103,7 +1111,7 @@ int upload_plan(rtfmm_fmm* f) {
   return RTFMM_OK;
 }
 
-int run_apply(rtfmm_fmm* f, const ApplyCall& c, bool adjoint = false) {
+int run_apply(rtfmm_fmm* f, const ApplyCall& c, cudaStream_t st, bool adjoint = false) {
   ApplyBatch b;
   double* bufs[BUF_NUM] = {f->d_qeq, f->d_pchk, f->d_leafvec, f->d_leafvec2, f->d_y};
   b.A = bufs[c.abuf];
@@ -1120,10 +1128,10 @@ int run_apply(rtfmm_fmm* f, const ApplyCall& c, bool adjoint = false) {
   b.ns = f->ops.ns;
   b.beta = c.beta;
   b.max_rows = c.rows_max;
-  CK(launch_apply(b, f->s0));
+  CK(launch_apply(b, st));
   f->launches++;
   if (c.nsum > 0) {
-    CK(launch_sum_children(f->d_idx_pool + c.sum_off, c.nsum, f->d_y, f->ops.ns, f->d_qeq, f->s0));
+    CK(launch_sum_children(f->d_idx_pool + c.sum_off, c.nsum, f->d_y, f->ops.ns, f->d_qeq, st));
     f->launches++;
   }
   return RTFMM_OK;
@@ -1206,7 +1214,7 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
                         !mixed));
     f->launches++;
     for (auto& c : f->p2m_call) {
-      int rc = run_apply(f, c);
+      int rc = run_apply(f, c, s0);
       if (rc) return rc;
     }
     CK(stage_end(ST_P2M));
@@ -1227,52 +1235,103 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
   }
   if (far && down) {
     if (phase == 2) CK(cudaMemsetAsync(f->d_pchk, 0, sizeof(double) * p.cells.size() * ns, s0));
-    for (auto& c : f->m2m_calls) {
-      int rc = run_apply(f, c, adjoint);
-      if (rc) return rc;
-    }
-    CK(stage_end(ST_M2M));
     const int nup8 = (int)f->up8_items.size() / 10, nup27 = (int)f->up27_items.size() / 10;
     const int ndn8 = (int)f->down8_items.size() / 10, ndn27 = (int)f->down27_items.size() / 10;
-    if (f->m2l32) {
-      CK(launch_m2l_up<float>(f->d_qeq, f->d_up8, nup8, f->d_surf_ijk, f->d_twiddle, P, ns, f->nS8, f->sp_up8,
-                              (float*)f->d_Q8, s0));
+    // applications of the tree levels (img = false) or of the image levels
+    auto applies = [&](const std::vector<ApplyCall>& calls, bool img, cudaStream_t st) -> int {
+      for (const ApplyCall& c : calls) {
+        if ((c.bsel == B_IMGSUMT || c.bsel == B_IMG13) != img) continue;
+        int rc = run_apply(f, c, st, adjoint);
+        if (rc) return rc;
+      }
+      return RTFMM_OK;
+    };
+    auto up8 = [&]() -> int {
+      if (f->m2l32)
+        CK(launch_m2l_up<float>(f->d_qeq, f->d_up8, nup8, f->d_surf_ijk, f->d_twiddle, P, ns, f->nS8, f->sp_up8,
+                                (float*)f->d_Q8, s0));
+      else
+        CK(launch_m2l_up<double>(f->d_qeq, f->d_up8, nup8, f->d_surf_ijk, f->d_twiddle, P, ns, f->nS8, f->sp_up8,
+                                 (double*)f->d_Q8, s0));
+      f->launches += nup8 > 0;
+      return RTFMM_OK;
+    };
+    auto had8 = [&]() -> int {
+      if (f->m2l32)
+        CK(launch_m2l_hadamard8((const float*)f->d_Q8, (const float*)f->d_G8, f->d_tsrc8, f->nT8, f->nS8, Nf,
+                                (float*)f->d_Pk8, s0));
+      else
+        CK(launch_m2l_hadamard8((const double*)f->d_Q8, (const double*)f->d_G8, f->d_tsrc8, f->nT8, f->nS8, Nf,
+                                (double*)f->d_Pk8, s0));
+      f->launches += f->nT8 > 0;
+      return RTFMM_OK;
+    };
+    auto down8 = [&]() -> int {
+      if (f->m2l32)
+        CK(launch_m2l_down<float>((const float*)f->d_Pk8, f->d_down8, f->d_tscale8, ndn8, f->d_surf_ijk, f->d_twiddle,
+                                  P, ns, f->nT8, f->sp_down8, f->d_pchk, s0));
+      else
+        CK(launch_m2l_down<double>((const double*)f->d_Pk8, f->d_down8, f->d_tscale8, ndn8, f->d_surf_ijk,
+                                   f->d_twiddle, P, ns, f->nT8, f->sp_down8, f->d_pchk, s0));
+      f->launches += ndn8 > 0;
+      return RTFMM_OK;
+    };
+    auto up27 = [&](cudaStream_t st) -> int {
+      CK(launch_m2l_up<double>(f->d_qeq, f->d_up27, nup27, f->d_surf_ijk, f->d_twiddle, P, ns, f->nS27, f->sp_up27,
+                               f->d_Q27, st));
+      f->launches += nup27 > 0;
+      return RTFMM_OK;
+    };
+    auto had27 = [&](cudaStream_t st) -> int {
+      CK(launch_m2l_hadamard27(f->d_Q27, f->d_G27, f->d_tsrc27, f->nT27, f->nS27, Nf, f->d_Pk27, st));
+      f->launches += f->nT27 > 0;
+      return RTFMM_OK;
+    };
+    auto down27 = [&](cudaStream_t st) -> int {
+      CK(launch_m2l_down<double>(f->d_Pk27, f->d_down27, f->d_tscale27, ndn27, f->d_surf_ijk, f->d_twiddle, P, ns,
+                                 f->nT27, f->sp_down27, f->d_pchk, st));
+      f->launches += ndn27 > 0;
+      return RTFMM_OK;
+    };
+    int rc = 0;
+    if ((rc = applies(f->m2m_calls, false, s0))) return rc;
+    if (timed) {
+      if ((rc = applies(f->m2m_calls, true, s0))) return rc;
+      CK(stage_end(ST_M2M));
+      if ((rc = up8()) || (rc = up27(s0))) return rc;
+      CK(stage_end(ST_UP));
+      if ((rc = had8()) || (rc = had27(s0))) return rc;
+      CK(stage_end(ST_HAD));
+      if ((rc = down8()) || (rc = down27(s0))) return rc;
+      CK(stage_end(ST_DOWN));
+      if ((rc = applies(f->l2l_calls, true, s0))) return rc;
     } else {
-      CK(launch_m2l_up<double>(f->d_qeq, f->d_up8, nup8, f->d_surf_ijk, f->d_twiddle, P, ns, f->nS8, f->sp_up8,
-                               (double*)f->d_Q8, s0));
+      // The image levels read the root's multipole and write image cells and
+      // the root only, the 8x8 M2L reads cells below the root and writes
+      // those: two branches between the tree's M2M and L2L.  The image branch
+      // is a chain of ten kernels of one or two rows each, worth hiding where
+      // the pass is short: 8192 bodies at P = 6 (FP64) 192 -> 174 us, 2^20 at
+      // P = 6, ncrit = 64 (3.4e6 target spectra) 2.67 -> 2.63 ms; 2^20 at
+      // P = 8, ncrit = 256 (4.6e6) 6.16 -> 6.21 ms, where P2P fills the chip
+      // while the image kernels run by themselves.
+      const bool fork = f->args.images > 0 && (int64_t)f->nT8 * Nf <= 4000000;
+      cudaStream_t si = fork ? f->s2 : s0;
+      if (fork) {
+        CK(cudaEventRecord(f->ev_img0, s0));
+        CK(cudaStreamWaitEvent(si, f->ev_img0, 0));
+      }
+      if ((rc = up8())) return rc;
+      if ((rc = applies(f->m2m_calls, true, si)) || (rc = up27(si)) || (rc = had27(si)) || (rc = down27(si)) ||
+          (rc = applies(f->l2l_calls, true, si)))
+        return rc;
+      if (fork) CK(cudaEventRecord(f->ev_img1, si));
+      if ((rc = had8()) || (rc = down8())) return rc;
+      if (fork) CK(cudaStreamWaitEvent(s0, f->ev_img1, 0));
     }
-    CK(launch_m2l_up<double>(f->d_qeq, f->d_up27, nup27, f->d_surf_ijk, f->d_twiddle, P, ns, f->nS27,
-                             f->sp_up27, f->d_Q27, s0));
-    f->launches += (nup8 > 0) + (nup27 > 0);
-    CK(stage_end(ST_UP));
-    if (f->m2l32) {
-      CK(launch_m2l_hadamard8((const float*)f->d_Q8, (const float*)f->d_G8, f->d_tsrc8, f->nT8, f->nS8,
-                                     Nf, (float*)f->d_Pk8, s0));
-    } else {
-      CK(launch_m2l_hadamard8((const double*)f->d_Q8, (const double*)f->d_G8, f->d_tsrc8, f->nT8,
-                                      f->nS8, Nf, (double*)f->d_Pk8, s0));
-    }
-    CK(launch_m2l_hadamard27(f->d_Q27, f->d_G27, f->d_tsrc27, f->nT27, f->nS27, Nf, f->d_Pk27, s0));
-    f->launches += (f->nT8 > 0) + (f->nT27 > 0);
-    CK(stage_end(ST_HAD));
-    if (f->m2l32) {
-      CK(launch_m2l_down<float>((const float*)f->d_Pk8, f->d_down8, f->d_tscale8, ndn8, f->d_surf_ijk,
-                                f->d_twiddle, P, ns, f->nT8, f->sp_down8, f->d_pchk, s0));
-    } else {
-      CK(launch_m2l_down<double>((const double*)f->d_Pk8, f->d_down8, f->d_tscale8, ndn8, f->d_surf_ijk,
-                                 f->d_twiddle, P, ns, f->nT8, f->sp_down8, f->d_pchk, s0));
-    }
-    CK(launch_m2l_down<double>(f->d_Pk27, f->d_down27, f->d_tscale27, ndn27, f->d_surf_ijk, f->d_twiddle, P, ns,
-                               f->nT27, f->sp_down27, f->d_pchk, s0));
-    f->launches += (ndn8 > 0) + (ndn27 > 0);
-    CK(stage_end(ST_DOWN));
-    for (auto& c : f->l2l_calls) {
-      int rc = run_apply(f, c, adjoint);
-      if (rc) return rc;
-    }
+    if ((rc = applies(f->l2l_calls, false, s0))) return rc;
     CK(stage_end(ST_L2L));
     for (auto& c : f->l2p_call) {
-      int rc = run_apply(f, c);
+      int rc = run_apply(f, c, s0);
       if (rc) return rc;
     }
     CK(launch_l2p_eval(f->d_body64, f->d_leaves_own, nleaf, f->d_surf_unit, ns, f->d_leafvec2, f->d_far_phi,
