@@ -84,7 +84,6 @@ namespace rtfmm_b200 {
 // ---------------------------------------------------------------------------
 template <typename T> struct Cplx;
 template <> struct Cplx<float> { using type = float2; };
-template <> struct Cplx<double> { using type = double2; };
 // two complex values in one vector load
 template <typename T> struct Cplx2;
 template <> struct Cplx2<float> { using type = float4; };
@@ -109,9 +108,6 @@ __device__ __forceinline__ void ld_sector(const float* p, float (&v)[8]) {
   asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
                : "l"(p));
-}
-__device__ __forceinline__ void ld_sector(const double* p, double (&v)[4]) {
-  asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
 }
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
@@ -1130,21 +1126,27 @@ __global__ void __launch_bounds__(256)
 // The up and down kernels above with register blocking, for the orders P
 // fixed at compile time.  A thread takes one line of a pass (the values along
 // the transformed axis) for 16 bytes of child slots (two in FP32, one in
-// FP64) and forms every output of the line in registers.  Frequencies k and
-// N - k share their cosines and sines,
-//   X_k e^(it) + X_(N-k) e^(-it) = (X_k + X_(N-k)) cos t + i (X_k - X_(N-k)) sin t,
-// which halves the multiply-adds of a complex transform, and the twiddles,
+// FP64) and forms every output of the line in registers.  The twiddles,
 // indexed by constants after unrolling, are operands in the kernel's
 // parameter bank (the form before read each as a shared-memory broadcast, one
 // for two multiply-adds, which bounded it).  Shared memory holds one array
 // [z][ky][kx][slot]; every pass works in place on it, which leaves room for
-// two to seven blocks per SM.  Up and down at N = 2^20, P = 8 (FP32): 0.20 and
-// 0.34 -> 0.12 and 0.14 ms; at P = 10 (FP64, 10^6 bodies in blobs): 1.47 and
-// 2.38 -> 0.84 and 0.78 ms, the latter 40% of the measured HBM rate for the spectra alone.
+// two to seven blocks per SM.  In FP64 frequencies k and N - k share their
+// cosines and sines,
+//   X_k e^(it) + X_(N-k) e^(-it) = (X_k + X_(N-k)) cos t + i (X_k - X_(N-k)) sin t,
+// which halves the multiply-adds; in FP32 each output sums its terms in the
+// order of k_m2l_up / k_m2l_down, bit for bit: the mixed form's error is the
+// rounding of these spectra, and another order would move results by as much.
+// Up and down at N = 2^20, P = 8 (FP32): 0.20 and 0.34 -> 0.14 and 0.14 ms (paired
+// 0.12 and 0.14);
+// at P = 10 (FP64, 10^6 bodies in blobs): 1.47 and 2.38 -> 0.84 and 0.78 ms, the
+// latter 40% of the measured HBM rate for the spectra alone.
 template <typename T, int N>
 struct Twiddles {
   T c[N], s[N];  // cos, sin (2 pi m / N)
 };
+template <typename T>
+constexpr bool kPairFrequencies = sizeof(T) == 8;
 template <typename T>
 struct DftSlots {
   static constexpr int kPer = 16 / (2 * sizeof(T));  // child slots of a thread
@@ -1183,42 +1185,63 @@ __device__ __forceinline__ void dft_forward(const T* in, int si, const Twiddles<
   T xr[P][U], xi[P][U];
 #pragma unroll
   for (int y = 0; y < P; ++y) ld_slots(in + y * si, xr[y], xi[y]);
+  if constexpr (!kPairFrequencies<T>) {
 #pragma unroll
-  for (int k = 0; k < P; ++k) {
-    T ar[U], ai[U], br[U], bi[U];  // sums of x cos and x sin
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      ar[u] = xr[0][u];
-      ai[u] = xi[0][u];
-      br[u] = bi[u] = T(0);
-    }
-#pragma unroll
-    for (int y = 1; y < P; ++y) {
-      const T c = tw.c[(k * y) % N], s = tw.s[(k * y) % N];
+    for (int k = 0; k < N; ++k) {
+      T re[U], im[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        ar[u] = fma(xr[y][u], c, ar[u]);
-        ai[u] = fma(xi[y][u], c, ai[u]);
-        if (k > 0) {
-          br[u] = fma(xr[y][u], s, br[u]);
-          bi[u] = fma(xi[y][u], s, bi[u]);
+        re[u] = xr[0][u];
+        im[u] = xi[0][u];
+#pragma unroll
+        for (int y = 1; y < P; ++y) {
+          const T c = tw.c[(k * y) % N], s = tw.s[(k * y) % N];
+          re[u] = fma(xr[y][u], c, re[u]);
+          re[u] = fma(xi[y][u], s, re[u]);
+          im[u] = fma(-xr[y][u], s, im[u]);
+          im[u] = fma(xi[y][u], c, im[u]);
         }
       }
+      put(k, re, im);
     }
-    T re[U], im[U];
+  } else {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      re[u] = ar[u] + bi[u];
-      im[u] = ai[u] - br[u];
-    }
-    put(k, re, im);
-    if (k > 0) {
+    for (int k = 0; k < P; ++k) {
+      T ar[U], ai[U], br[U], bi[U];  // sums of x cos and x sin
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        re[u] = ar[u] - bi[u];
-        im[u] = ai[u] + br[u];
+        ar[u] = xr[0][u];
+        ai[u] = xi[0][u];
+        br[u] = bi[u] = T(0);
       }
-      put(N - k, re, im);
+#pragma unroll
+      for (int y = 1; y < P; ++y) {
+        const T c = tw.c[(k * y) % N], s = tw.s[(k * y) % N];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          ar[u] = fma(xr[y][u], c, ar[u]);
+          ai[u] = fma(xi[y][u], c, ai[u]);
+          if (k > 0) {
+            br[u] = fma(xr[y][u], s, br[u]);
+            bi[u] = fma(xi[y][u], s, bi[u]);
+          }
+        }
+      }
+      T re[U], im[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        re[u] = ar[u] + bi[u];
+        im[u] = ai[u] - br[u];
+      }
+      put(k, re, im);
+      if (k > 0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          re[u] = ar[u] - bi[u];
+          im[u] = ai[u] + br[u];
+        }
+        put(N - k, re, im);
+      }
     }
   }
 }
@@ -1240,21 +1263,40 @@ __device__ __forceinline__ void dft_inverse(const T* in, size_t si, const Twiddl
         im[o][u] = xi[u];
       }
   }
+  if constexpr (!kPairFrequencies<T>) {
 #pragma unroll
-  for (int k = 1; k < P; ++k) {
-    T xr[U], xi[U], yr[U], yi[U];
-    ld_slots(in + k * si, xr, xi);
-    ld_slots(in + (N - k) * si, yr, yi);
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const T sr = xr[u] + yr[u], sim = xi[u] + yi[u], dr = xr[u] - yr[u], di = xi[u] - yi[u];
+    for (int k = 1; k < N; ++k) {
+      T xr[U], xi[U];
+      ld_slots(in + k * si, xr, xi);
 #pragma unroll
       for (int o = 0; o < P; ++o) {
         const T c = tw.c[(k * (P - 1 + o)) % N], s = tw.s[(k * (P - 1 + o)) % N];
-        re[o][u] = fma(sr, c, re[o][u]);
-        re[o][u] = fma(-di, s, re[o][u]);
-        im[o][u] = fma(sim, c, im[o][u]);
-        im[o][u] = fma(dr, s, im[o][u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          re[o][u] = fma(xr[u], c, re[o][u]);
+          re[o][u] = fma(-xi[u], s, re[o][u]);
+          im[o][u] = fma(xr[u], s, im[o][u]);
+          im[o][u] = fma(xi[u], c, im[o][u]);
+        }
+      }
+    }
+  } else {
+#pragma unroll
+    for (int k = 1; k < P; ++k) {
+      T xr[U], xi[U], yr[U], yi[U];
+      ld_slots(in + k * si, xr, xi);
+      ld_slots(in + (N - k) * si, yr, yi);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const T sr = xr[u] + yr[u], sim = xi[u] + yi[u], dr = xr[u] - yr[u], di = xi[u] - yi[u];
+#pragma unroll
+        for (int o = 0; o < P; ++o) {
+          const T c = tw.c[(k * (P - 1 + o)) % N], s = tw.s[(k * (P - 1 + o)) % N];
+          re[o][u] = fma(sr, c, re[o][u]);
+          re[o][u] = fma(-di, s, re[o][u]);
+          im[o][u] = fma(sim, c, im[o][u]);
+          im[o][u] = fma(dr, s, im[o][u]);
+        }
       }
     }
   }
