@@ -352,18 +352,16 @@ void drop_allocs(rtfmm_fmm* f) {
 
 void free_device(rtfmm_fmm* f) {
   if (f->dev >= 0) cudaSetDevice(f->dev);
-  if (f->h_xin) {
-    cudaFreeHost(f->h_xin);
-    f->h_xin = nullptr;
-  }
-  f->h_xin_cap = 0;
-  if (f->h_pack) cudaFreeHost(f->h_pack);
-  f->h_pack = nullptr;
-  f->h_pack_cap = 0;
   drop_allocs(f);
   for (auto& kv : f->pool)
     if (kv.second.p) cudaFree(kv.second.p);
   f->pool.clear();
+  // after the cudaFree above, which waits for copies from these
+  if (f->h_xin) cudaFreeHost(f->h_xin);
+  if (f->h_pack) cudaFreeHost(f->h_pack);
+  f->h_xin = nullptr;
+  f->h_pack = nullptr;
+  f->h_xin_cap = f->h_pack_cap = 0;
   f->ops_dev_gen = 0;
   f->d_flush = nullptr;
   f->flush_bytes = 0;
