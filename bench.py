@@ -167,6 +167,9 @@ def measured_peaks():
 # reference arm / CPU baseline
 # ----------------------------------------------------------------------------
 REF_BIN = os.path.join(ROOT, "oracle", "_ref", "rtfmm_ref_pass")
+# The oracle's single process takes 5.6 s a pass at this size and does not end
+# within ten minutes at the workload's 2^20 bodies.
+ORACLE_BODIES = 16384
 
 
 def cpu_model():
@@ -183,12 +186,15 @@ def reference_passes(n, threads, passes, seed=2):
     """The reference's own CPU FMM on n bodies of the workload: its tree,
     lists and operator tables built once, then `passes` runs of its hot block
     (LaplaceFMM's P2M ... P2P, 3dpp/src/fmm.cpp:51-60; oracle/_ref
-    rtfmm_ref_pass --repeat).  Returns (pass seconds list, set-up seconds,
-    kind, note); without the compiled reference, the numpy oracle's whole
-    pass (single process) instead."""
+    rtfmm_ref_pass --repeat).  Returns (bodies, pass seconds list, set-up
+    seconds, kind, note); without the compiled reference, the numpy oracle's
+    pass (single process) on a sample of ORACLE_BODIES instead."""
     W = WORKLOAD
+    have_ref = os.path.exists(REF_BIN)
+    if not have_ref:
+        n = min(n, ORACLE_BODIES)
     x, q = make_bodies(n, seed)
-    if os.path.exists(REF_BIN):
+    if have_ref:
         with tempfile.TemporaryDirectory() as td:
             fin = os.path.join(td, "in.bin")
             np.concatenate([x - 0.5, q[:, None]], axis=1).astype(np.float64).tofile(fin)
@@ -205,7 +211,7 @@ def reference_passes(n, threads, passes, seed=2):
                 setup = float(line.split()[1])
         if len(ts) != passes:
             raise RuntimeError("reference run printed %d of %d pass timers" % (len(ts), passes))
-        return ts, setup, "reference", "the reference's LaplaceFMM hot block (P2M..P2P) repeated after one set-up"
+        return n, ts, setup, "reference", "the reference's LaplaceFMM hot block (P2M..P2P) repeated after one set-up"
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import rtfmm_oracle as orc
     ts = []
@@ -214,23 +220,27 @@ def reference_passes(n, threads, passes, seed=2):
         t0 = time.perf_counter()
         F.solve()
         ts.append(time.perf_counter() - t0)
-    return ts, None, "port", "numpy oracle pass (single process)"
+    return n, ts, None, "port", "numpy oracle pass (single process), N=%d bodies" % n
 
 
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    if not os.path.exists(REF_BIN):
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "oracle/_ref is not built: the reference's sources were not present "
+                                         "(oracle/build_ref.sh)"}), flush=True)
+        return
     threads = os.cpu_count() or 1
-    n = args.ref_n
-    ts, setup, kind, note = reference_passes(n, threads, args.warmup + args.steps)
+    n, ts, setup, kind, note = reference_passes(args.ref_n, threads, args.warmup + args.steps)
     timed = ts[args.warmup:]
     value = n / float(np.mean(timed))
     # the published runs used 8 threads (3dpp/exp/test_i.sh:17): two passes
     # at that setting beside the all-core figure
     th8 = None
     if threads != 8 and kind == "reference":
-        t8, _, _, _ = reference_passes(n, 8, 2)
+        _, t8, _, _, _ = reference_passes(n, 8, 2)
         th8 = {"value": n / t8[-1], "unit": "particles/s", "threads": 8}
     W = WORKLOAD
     line = {"impl": "reference", "metric": METRIC, "value": value, "unit": "particles/s", "n_gpus": args.gpus,
@@ -560,10 +570,10 @@ def run_ours(args):
     if world == 1 and not args.no_cpu_baseline:
         try:
             ncores = os.cpu_count() or 1
-            ts, setup, kind, note = reference_passes(args.ref_n, ncores, 2)
-            cpu = {"value": args.ref_n / ts[-1], "unit": "particles/s", "cores": ncores, "kind": kind,
+            ref_n, ts, setup, kind, note = reference_passes(args.ref_n, ncores, 2)
+            cpu = {"value": ref_n / ts[-1], "unit": "particles/s", "cores": ncores, "kind": kind,
                    "sample": "N=%d bodies of the workload (P=8 ncrit=256 images=3), the second of two passes "
-                             "after one set-up (%.1f s); %s" % (args.ref_n, setup or 0.0, note),
+                             "after one set-up (%.1f s); %s" % (ref_n, setup or 0.0, note),
                    "cpu_model": cpu_model()}
         except Exception as e:  # the baseline is reported, never required
             cpu = {"value": None, "unit": "particles/s", "cores": 0, "kind": "none", "sample": "failed: %s" % e}
