@@ -16,9 +16,9 @@ ours:       value = N / pass time, FP32-mixed form, bodies resident in HBM,
             e2e   = the same metric through the C ABI with pinned host
             buffers (charges in, potential and gradient out) per step.
 reference:  the reference's own CPU FMM (compiled from its sources into
-            oracle/_ref, else the numpy oracle) on the same workload, all
-            host threads: its tree, lists and tables built once, then one
-            run of its hot block per step.
+            oracle/_ref; without it the line says "unavailable") on the same
+            workload, all host threads: its tree, lists and tables built
+            once, then one run of its hot block per step.
 
 Multi-GPU (torchrun): by default each rank runs an independent replica on
 its own GPU; value = all ranks' bodies / max-over-ranks time.  With --shard
