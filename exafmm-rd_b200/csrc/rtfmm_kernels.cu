@@ -1712,10 +1712,11 @@ __global__ void __launch_bounds__(HadCfg<T>::THREADS, HadCfg<T>::MINB)
 // A block takes one frequency and 96 targets, a warp 24 of them as three
 // tiles of 8; lane 4 r + q holds source slot q (and q + 4) of target row r.
 // A tile none of whose targets has a source in a direction skips it.
-// Three tiles a warp leave room for four blocks an SM (128 registers): 1.79 ms
-// at N = 2^20, P = 8, ncrit = 256 against 1.87 with four tiles and three
-// blocks and 1.97 with two and five; 3.58 ms for the product in full on the
-// FMA pipe.  The FP64 tensor pipe is 70% busy (27 of DGEMM's 35 TFLOP/s,
+// Three tiles a warp leave room for four blocks an SM (128 registers): 1.91 ms
+// at N = 2^20, P = 8, ncrit = 256 and 1.82 ms at N = 2^18, ncrit = 64, against
+// 2.04 and 1.95 ms with four tiles and three blocks; two tiles and five blocks
+// took 1.10 times as long as three and four.  3.58 ms for the product in full
+// on the FMA pipe (N = 2^20).  The FP64 tensor pipe is 70% busy (27 of DGEMM's 35 TFLOP/s,
 // counting the 40% of the (target, direction) slots that are empty there).
 // ---------------------------------------------------------------------------
 constexpr int kHad64Tiles = 3, kHad64Threads = 128, kHad64Blocks = 4;
