@@ -111,6 +111,7 @@ struct rtfmm_fmm {
   std::vector<P2PItem> items2;    // P2P work items (target groups x list parts), both precisions
   std::vector<int> list_off;
   int n_items2 = 0;               // work items (host or device built)
+  bool p2p_long = false;          // FP32 P2P entry by entry (p2p_long_entries)
   int n_slots = 0;                // slots of the items whose list is cut into parts
   int64_t p2p_pairs = 0;          // body pairs of the P2P lists
   // the P2P lists, offsets and items were built on the GPU (device set-up):
@@ -519,8 +520,8 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
   f->list_off.assign(nlf + 1, 0);
   std::vector<int> item_off(nlf + 1, 0);
   std::vector<int64_t> bodies(nlf, 0);
-  unsigned long long work = 0;
-#pragma omp parallel for schedule(dynamic, 64) reduction(+ : work)
+  unsigned long long work = 0, entries = 0;
+#pragma omp parallel for schedule(dynamic, 64) reduction(+ : work, entries)
   for (int l = 0; l < nlf; ++l) {
     int path[kMaxPath];
     const int np = path_lists(f->leaves[l].cell, path);
@@ -534,9 +535,11 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
       }
     f->list_off[l + 1] = (int)cnt;
     work += (unsigned long long)bodies[l] * ((f->leaves[l].bnum + 31) / 32);
+    entries += (unsigned long long)cnt * ((f->leaves[l].bnum + 31) / 32);
   }
   // long lists are cut into parts of about `part` bodies
   const int part = p2p_part_bodies(work);
+  f->p2p_long = p2p_long_entries(work, entries);
   std::vector<int> slot_off(nlf + 1, 0);
   for (int l = 0; l < nlf; ++l) {
     const int groups = (f->leaves[l].bnum + 31) / 32, nparts = (int)std::max<int64_t>(1, (bodies[l] + part - 1) / part);
@@ -1185,8 +1188,8 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
     }
     CK(cudaEventRecord(f->ev_near0, s1));
     if (mixed) {
-      CK(launch_p2p32(f->d_body32, f->d_items2, f->n_items2, f->d_list32, f->d_part, f->d_part_done,
-                      f->d_near_phi, f->d_near_grad, s1));
+      CK(launch_p2p32(f->d_body32, f->d_items2, f->n_items2, f->p2p_long, f->n_slots > 0, f->d_list32,
+                      f->d_part, f->d_part_done, f->d_near_phi, f->d_near_grad, s1));
       f->launches += 1;
       if (f->n_close > 0) {
         CK(launch_close_fix(f->d_body64, f->d_body32, f->d_list32, f->d_close_off, f->d_close_pairs, n,
@@ -1696,6 +1699,7 @@ int device_tables(rtfmm_fmm* f, const TreeScratchFn& scratch) {
     return fail(RTFMM_ECUDA, msg);
   f->n_items2 = out.nitems;
   f->n_slots = out.nslots;
+  f->p2p_long = out.long_entries;
   f->p2p_pairs = out.pairs;
   return alloc_parts(f);
 }

@@ -26,29 +26,6 @@
 
 #include <cub/cub.cuh>
 
-// FP32 P2P: inner unroll and resident blocks per SM.  A block is one warp
-// (P2P_WARPS): work items differ in cost several-fold, and a block of four
-// held the slots of its finished warps until its slowest one was done
-// (3.33 against 3.12 ms at N = 2^20, P = 8).
-#ifndef P2P_UNROLL
-#define P2P_UNROLL 4
-#endif
-#ifndef P2P_MINB
-#define P2P_MINB 20
-#endif
-#ifndef P2P_WARPS
-#define P2P_WARPS 1
-#endif
-// FP64 P2P: the same
-#ifndef P2P64_UNROLL
-#define P2P64_UNROLL 4
-#endif
-#ifndef P2P64_MINB
-#define P2P64_MINB 28
-#endif
-#ifndef P2P_FLUSH
-#define P2P_FLUSH 1
-#endif
 // FP32 Hadamard: targets per thread, directions per FP32 partial sum,
 // resident blocks per SM
 #ifndef HAD_TT
@@ -183,29 +160,52 @@ __global__ void k_body_leaf(const LeafInfo* __restrict__ leaves, int nleaf, int 
 
 // ---------------------------------------------------------------------------
 // P2P: one warp per work item, up to 32 targets of one leaf against a part of
-// the leaf's source list (entries e0..e1).  The bodies of the list's entries
-// are taken as one sequence and staged 32 at a time in a per-warp
-// shared-memory slot, so a tile is full whatever the sizes of the source
-// leaves; the next tile's bodies and the next 32 entries load while the
-// current tile is computed.
+// the leaf's source list (entries e0..e1), staged 32 bodies at a time in a
+// per-warp shared-memory slot; the next tile's bodies load while the current
+// tile is computed.
+//
+// Long entries (p2p_long_entries, FP32): a tile is up to 32 bodies of one
+// entry.  Short entries and FP64: the bodies of the entries are taken as one
+// sequence, so that a tile is full whatever the sizes of the source leaves,
+// and 32 entries load at once.
+//
+// Error of the FP32 form.  Each source leaf has its own frame: the target is
+// moved into it (x_t - offset, one rounding that all sources of the leaf
+// share, so that it cancels where their charges do; the offset added to each
+// source instead gave the potential of a lattice up to 1.4 times the error).
+// FP32 sums run over one long entry, or over 8 pairs of short ones (the
+// potential over 4) divided by the number of lane groups, and their two
+// halves go into FP64 each by itself.  Over 27 sets (uniform, blobs, lattices;
+// mean entries of 4-256 bodies) the error against FP64 is at most 1.01 times
+// that of sums over one entry each, 0.8-1.0 times for short ones; sums over 16
+// pairs across entries gave 1.0-1.9 times for the potential and up to 1.2
+// times for the gradient.
 //
 // A clustered tree has leaves whose lists hold forty times the mean number of
 // bodies (a large leaf beside many small ones): such a list is cut into parts
 // (p2p_part_bodies), each part leaves its sums in a slot of its own, and the
 // last part to finish adds the slots up in order, so that the result does not
-// depend on which one that is.  Measured: 150001 bodies in blobs (longest list
-// 60593 bodies, mean 1435), FP64, 3.98 -> 0.50 ms; 30011 in blobs, FP32,
-// 0.36 -> 0.052; 2^22 in blobs, FP32, 13.0 -> 8.2; uniform 2^20, ncrit = 256:
-// FP32 3.13 -> 3.12, FP64 9.28 -> 7.68 (24 -> 18 FP64 operations a pair).
+// depend on which one that is.  A plan without cut lists runs an instance
+// without that code, whose two registers fewer are 0.9% (3.57 against 3.60 ms,
+// 2^20 bodies in leaves of 256).
+//
+// Measured, with one entry a tile and uncut lists -> here: 150001 bodies in
+// blobs (longest list 60593 bodies, mean 1435), FP64, 3.98 -> 0.47 ms; 30011 in
+// blobs, FP32, 0.36 -> 0.052; 10^6 in blobs, FP32, 12.8 -> 2.47; uniform 2^20,
+// FP32, ncrit = 32 1.36 -> 0.87, 64 0.68 and 0.68, 256 3.13 and 3.13, 512 3.58
+// and 3.58; FP64, ncrit = 256, 9.28 -> 7.68 (24 -> 18 FP64 operations a pair).
 // FP32: bound by the register reads of the packed FMAs (3 cycles each measured,
-// 31 a pair of sources with the 2-cycle additions and products); each tile's 32
-// sources go into FP64 (every four tiles: 3.07 ms, but the gradient's error
-// against FP64 2.8 times as large).  FP64: bound by dependent operations (pipe
-// 66% busy); 28 resident warps 7.68 ms, 20 7.94, 24 8.04, 32 7.76.
+// 31 a pair of sources with the 2-cycle additions and products).  FP64: bound
+// by dependent operations (pipe 66% busy); 28 resident warps 7.68 ms, 20 7.94,
+// 24 8.04, 32 7.76.
 // ---------------------------------------------------------------------------
-constexpr int kP2PWarps = P2P_WARPS;
-constexpr int kP2PUnroll = P2P_UNROLL, kP2PUnroll64 = P2P64_UNROLL;
-constexpr int kP2PFlush = P2P_FLUSH;  // tiles summed in FP32 before they go into FP64
+// A block is one warp: work items differ in cost several-fold, and a block of
+// four held the slots of its finished warps until its slowest one was done
+// (FP32 3.33 against 3.12 ms at N = 2^20, P = 8).
+constexpr int kP2PWarps = 1;
+constexpr int kP2PUnroll = 4, kP2PUnroll64 = 4;  // pairs (FP32), sources (FP64)
+constexpr int kP2PRun = 8, kP2PRunPhi = 4;       // pairs of short entries summed in FP32
+constexpr int kP2PMinBlocks = 20, kP2PMinBlocksShort = 24, kP2PMinBlocks64 = 28;  // resident blocks per SM
 
 // A chunk of up to 32 list entries, one per lane: `start` is the lane's
 // entry's first body in the chunk's sequence, `src` + position the body in
@@ -240,11 +240,12 @@ __device__ __forceinline__ int p2p_entry(const P2PChunk& c, int base, int lane) 
 }
 
 // The sums of a work item: written, or left in the item's slot when its list
-// is cut into parts.
+// is cut into parts (only where CUT).
+template <bool CUT>
 __device__ __forceinline__ void p2p_store(const P2PItem& it, bool writer, int ti, double P, double Gx, double Gy,
                                           double Gz, double4* __restrict__ part, int* __restrict__ done,
                                           double* __restrict__ phi, double* __restrict__ grad) {
-  if (it.nparts > 1) {
+  if (CUT && it.nparts > 1) {
     if (writer) part[(size_t)(it.slot + it.part) * 32 + ti] = make_double4(P, Gx, Gy, Gz);
     __threadfence();
     __syncwarp();
@@ -302,18 +303,46 @@ __device__ __forceinline__ void p2p32_pair2(const float4* __restrict__ s, int k,
   fz = __ffma2_rn(q3, dz, fz);
 }
 
-// Lanes of group k0 (of G groups) take the tile's source pairs k0, k0+G, ...;
-// a full tile has a constant bound.
-template <int G, bool MASK, bool FULL>
-__device__ __forceinline__ void p2p32_tile(const float4* __restrict__ s, int k0, int npair, float2 px, float2 py,
-                                           float2 pz, float2& p, float2& fx, float2& fy, float2& fz) {
-  const int n = FULL ? 16 : npair;
+// The two interleaved halves of an FP32 sum into FP64, each by itself.
+__device__ __forceinline__ void widen(double& d, float2 v) { d += (double)v.x + (double)v.y; }
+
+// Lanes of group k0 (of G groups) take the tile's source pairs k0, k0+G, ...,
+// all of one entry.
+template <int G, bool MASK>
+__device__ __forceinline__ void p2p32_run(const float4* __restrict__ s, int k0, int npair, float2 px, float2 py,
+                                          float2 pz, float2& p, float2& fx, float2& fy, float2& fz) {
 #pragma unroll kP2PUnroll
-  for (int k = k0; k < n; k += G) p2p32_pair2<MASK>(s, k, px, py, pz, p, fx, fy, fz);
+  for (int k = k0; k < npair; k += G) p2p32_pair2<MASK>(s, k, px, py, pz, p, fx, fy, fz);
+}
+// The same for a whole tile across entries, pair k of the entry with the
+// offset so[k]; FP32 sums over R pairs (the potential over RP), a lane group
+// over as many fewer as there are groups.
+template <int G, bool MASK>
+__device__ __forceinline__ void p2p32_pairs(const float4* __restrict__ s, const float4* __restrict__ so, int k0,
+                                            float4 xt, double& P, double& Gx, double& Gy, double& Gz) {
+  constexpr int N = 16 / G, R = kP2PRun >= G ? kP2PRun / G : 1, RP = kP2PRunPhi >= G ? kP2PRunPhi / G : 1;
+#pragma unroll 1
+  for (int u = 0; u < N; u += R) {
+    float2 p = make_float2(0.f, 0.f), fx = p, fy = p, fz = p;
+#pragma unroll
+    for (int v = 0; v < R; ++v) {
+      const int k = k0 + (u + v) * G;
+      const float4 o = so[k];
+      const float px = xt.x - o.x, py = xt.y - o.y, pz = xt.z - o.z;
+      p2p32_pair2<MASK>(s, k, make_float2(px, px), make_float2(py, py), make_float2(pz, pz), p, fx, fy, fz);
+      if (v % RP == RP - 1) {
+        widen(P, p);
+        p = make_float2(0.f, 0.f);
+      }
+    }
+    widen(Gx, fx);
+    widen(Gy, fy);
+    widen(Gz, fz);
+  }
 }
 
 // One work item: W = 32/G lanes per target group, G groups per warp.
-template <int G>
+template <bool LONG, bool CUT, int G>
 __device__ __forceinline__ void p2p32_item(const float4* __restrict__ body32, const P2PItem& it,
                                            const P2PSrc32* __restrict__ list, float4* __restrict__ sw, int lane,
                                            double4* __restrict__ part, int* __restrict__ done,
@@ -324,73 +353,115 @@ __device__ __forceinline__ void p2p32_item(const float4* __restrict__ body32, co
   // tile padding: no charge, far from every target (finite 1/r)
   const float4 pad = make_float4(1e18f, 1e18f, 1e18f, 0.f);
   const float4 xt = active ? body32[it.boff + ti] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float2 px = make_float2(xt.x, xt.x), py = make_float2(xt.y, xt.y), pz = make_float2(xt.z, xt.z);
   double P = 0.0, Gx = 0.0, Gy = 0.0, Gz = 0.0;
-  float2 p = make_float2(0.f, 0.f), fx = p, fy = p, fz = p;
-  auto entry = [&](int e) { return e < it.e1 ? list[e] : P2PSrc32{}; };
-  P2PSrc32 cur{}, nxt{};  // this lane's entry of the chunk and of the next one
-  P2PChunk c{};
-  int self0 = 0, self1 = 0;  // the target leaf's own bodies in the chunk's sequence
-  auto chunk = [&](int e0) {
-    c = p2p_chunk(cur.boff, cur.bnum, min(32, it.e1 - e0), lane);
-    const unsigned own = __ballot_sync(0xffffffffu, cur.self);
-    const int o = own ? __ffs(own) - 1 : 0;
-    self0 = own ? __shfl_sync(0xffffffffu, c.start, o) : 0;
-    self1 = own ? self0 + __shfl_sync(0xffffffffu, cur.bnum, o) : 0;
-  };
-  float4 b = pad;  // the next tile's body of this lane and its leaf's offset
-  float ox = 0.f, oy = 0.f, oz = 0.f;
-  auto stage = [&](int base) {
-    const int s = p2p_entry(c, base, lane), pos = base + lane;
-    const int i = __shfl_sync(0xffffffffu, c.src, s) + pos;
-    ox = __shfl_sync(0xffffffffu, cur.dx, s);
-    oy = __shfl_sync(0xffffffffu, cur.dy, s);
-    oz = __shfl_sync(0xffffffffu, cur.dz, s);
-    b = pos < c.total ? body32[i] : pad;
-  };
-  int e = it.e0, base = 0, tiles = 0;
-  bool more = e < it.e1;
-  if (more) {
-    cur = entry(e + lane);
-    nxt = entry(e + 32 + lane);
-    chunk(e);
-    stage(0);
-  }
   float* sf = reinterpret_cast<float*>(sw) + 8 * (lane >> 1) + (lane & 1);
-  while (more) {
-    const int cnt = min(32, c.total - base);
-    const bool mask = self0 < base + 32 && self1 > base;
-    __syncwarp();
-    sf[0] = -(b.x + ox);
-    sf[2] = -(b.y + oy);
-    sf[4] = -(b.z + oz);
-    sf[6] = b.w;
-    __syncwarp();
-    base += 32;
-    if (base >= c.total) {
-      e += 32;
-      base = 0;
-      more = e < it.e1;
-      if (more) {
+  if constexpr (LONG) {
+    int e = it.e0;
+    const int e1 = it.e1;
+    P2PSrc32 cur{}, nxt{};
+    float4 b = pad;
+    if (e < e1) {
+      cur = list[e];
+      if (lane < cur.bnum) b = body32[cur.boff + lane];
+    }
+    if (e + 1 < e1) nxt = list[e + 1];
+    int c0 = 0;
+    float2 p = make_float2(0.f, 0.f), fx = p, fy = p, fz = p;
+    while (e < e1) {
+      const int cnt = min(32, cur.bnum - c0);
+      __syncwarp();
+      sf[0] = -b.x;
+      sf[2] = -b.y;
+      sf[4] = -b.z;
+      sf[6] = b.w;
+      __syncwarp();
+      // next tile: the rest of this entry, else the first of the next one
+      const bool last = c0 + 32 >= cur.bnum;
+      b = pad;
+      if (!last) {
+        if (lane < cur.bnum - c0 - 32) b = body32[cur.boff + c0 + 32 + lane];
+      } else if (e + 1 < e1) {
+        if (lane < nxt.bnum) b = body32[nxt.boff + lane];
+      }
+      const float px = xt.x - cur.dx, py = xt.y - cur.dy, pz = xt.z - cur.dz;
+      const int npair = (cnt + 1) >> 1;
+      if (cur.self)
+        p2p32_run<G, true>(sw, grp, npair, make_float2(px, px), make_float2(py, py), make_float2(pz, pz), p, fx, fy,
+                           fz);
+      else
+        p2p32_run<G, false>(sw, grp, npair, make_float2(px, px), make_float2(py, py), make_float2(pz, pz), p, fx, fy,
+                            fz);
+      if (last) {
+        P += (double)p.x + (double)p.y;
+        Gx += (double)fx.x + (double)fx.y;
+        Gy += (double)fy.x + (double)fy.y;
+        Gz += (double)fz.x + (double)fz.y;
+        p = fx = fy = fz = make_float2(0.f, 0.f);
+        ++e;
+        c0 = 0;
         cur = nxt;
-        nxt = entry(e + 32 + lane);
-        chunk(e);
+        if (e + 1 < e1) nxt = list[e + 1];
+      } else {
+        c0 += 32;
       }
     }
-    if (more) stage(base);
-    if (mask)
-      p2p32_tile<G, true, false>(sw, grp, (cnt + 1) >> 1, px, py, pz, p, fx, fy, fz);
-    else if (cnt == 32)
-      p2p32_tile<G, false, true>(sw, grp, 16, px, py, pz, p, fx, fy, fz);
-    else
-      p2p32_tile<G, false, false>(sw, grp, (cnt + 1) >> 1, px, py, pz, p, fx, fy, fz);
-    if (++tiles == kP2PFlush || !more) {
-      tiles = 0;
-      P += (double)(p.x + p.y);
-      Gx += (double)(fx.x + fx.y);
-      Gy += (double)(fy.x + fy.y);
-      Gz += (double)(fz.x + fz.y);
-      p = fx = fy = fz = make_float2(0.f, 0.f);
+  } else {
+    float4* so = sw + 32;  // offsets of the tile's pairs
+    auto entry = [&](int e) { return e < it.e1 ? list[e] : P2PSrc32{}; };
+    P2PSrc32 cur{}, nxt{};  // this lane's entry of the chunk and of the next one
+    P2PChunk c{};
+    int self0 = 0, self1 = 0;  // the target leaf's own bodies in the chunk's sequence
+    auto chunk = [&](int e0) {
+      // entries of an odd number of bodies take a padding slot: no pair of two
+      c = p2p_chunk(cur.boff, (cur.bnum + 1) & ~1, min(32, it.e1 - e0), lane);
+      const unsigned own = __ballot_sync(0xffffffffu, cur.self);
+      const int o = own ? __ffs(own) - 1 : 0;
+      self0 = own ? __shfl_sync(0xffffffffu, c.start, o) : 0;
+      self1 = own ? self0 + __shfl_sync(0xffffffffu, cur.bnum, o) : 0;
+    };
+    float4 b = pad, o = pad;  // the next tile's body of this lane and its entry's offset
+    auto stage = [&](int base) {
+      const int s = p2p_entry(c, base, lane), pos = base + lane;
+      const int i = __shfl_sync(0xffffffffu, c.src, s) + pos;
+      const int end = __shfl_sync(0xffffffffu, c.start + cur.bnum, s);
+      o.x = __shfl_sync(0xffffffffu, cur.dx, s);
+      o.y = __shfl_sync(0xffffffffu, cur.dy, s);
+      o.z = __shfl_sync(0xffffffffu, cur.dz, s);
+      b = pos < end ? body32[i] : pad;
+    };
+    int e = it.e0, base = 0;
+    bool more = e < it.e1;
+    if (more) {
+      cur = entry(e + lane);
+      nxt = entry(e + 32 + lane);
+      chunk(e);
+      stage(0);
+    }
+    while (more) {
+      const bool mask = self0 < base + 32 && self1 > base;
+      __syncwarp();
+      sf[0] = -b.x;
+      sf[2] = -b.y;
+      sf[4] = -b.z;
+      sf[6] = b.w;
+      if (!(lane & 1)) so[lane >> 1] = o;
+      __syncwarp();
+      base += 32;
+      if (base >= c.total) {
+        e += 32;
+        base = 0;
+        more = e < it.e1;
+        if (more) {
+          cur = nxt;
+          nxt = entry(e + 32 + lane);
+          chunk(e);
+        }
+      }
+      if (more) stage(base);
+      if (mask)
+        p2p32_pairs<G, true>(sw, so, grp, xt, P, Gx, Gy, Gz);
+      else
+        p2p32_pairs<G, false>(sw, so, grp, xt, P, Gx, Gy, Gz);
     }
   }
   // sum the source groups (lanes ti, ti + W, ...)
@@ -401,23 +472,24 @@ __device__ __forceinline__ void p2p32_item(const float4* __restrict__ body32, co
     Gy += __shfl_xor_sync(0xffffffffu, Gy, o);
     Gz += __shfl_xor_sync(0xffffffffu, Gz, o);
   }
-  p2p_store(it, active && grp == 0, ti, P, Gx, Gy, Gz, part, done, phi, grad);
+  p2p_store<CUT>(it, active && grp == 0, ti, P, Gx, Gy, Gz, part, done, phi, grad);
 }
 
-__global__ void __launch_bounds__(32 * kP2PWarps, P2P_MINB)
+template <bool LONG, bool CUT>
+__global__ void __launch_bounds__(32 * kP2PWarps, LONG ? kP2PMinBlocks : kP2PMinBlocksShort)
     k_p2p32(const float4* __restrict__ body32, const P2PItem* __restrict__ items, int nitems,
             const P2PSrc32* __restrict__ list, double4* __restrict__ part, int* __restrict__ done,
             double* __restrict__ phi, double* __restrict__ grad) {
-  __shared__ float4 sbuf[kP2PWarps][32];
+  __shared__ float4 sbuf[kP2PWarps][LONG ? 32 : 48];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = blockIdx.x * kP2PWarps + warp;
   if (item >= nitems) return;  // warp-uniform
   const P2PItem it = items[item];
   switch (it.lw) {
-    case 5: p2p32_item<1>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
-    case 4: p2p32_item<2>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
-    case 3: p2p32_item<4>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
-    default: p2p32_item<8>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    case 5: p2p32_item<LONG, CUT, 1>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    case 4: p2p32_item<LONG, CUT, 2>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    case 3: p2p32_item<LONG, CUT, 4>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
+    default: p2p32_item<LONG, CUT, 8>(body32, it, list, sbuf[warp], lane, part, done, phi, grad); break;
   }
 }
 
@@ -492,10 +564,10 @@ __device__ __forceinline__ void p2p64_item(const double4* __restrict__ body64, c
     Gy += __shfl_xor_sync(0xffffffffu, Gy, o);
     Gz += __shfl_xor_sync(0xffffffffu, Gz, o);
   }
-  p2p_store(it, active && grp == 0, ti, P, Gx, Gy, Gz, part, done, phi, grad);
+  p2p_store<true>(it, active && grp == 0, ti, P, Gx, Gy, Gz, part, done, phi, grad);
 }
 
-__global__ void __launch_bounds__(32 * kP2PWarps, P2P64_MINB)
+__global__ void __launch_bounds__(32 * kP2PWarps, kP2PMinBlocks64)
     k_p2p64(const double4* __restrict__ body64, const P2PItem* __restrict__ items, int nitems,
             const P2PSrc64* __restrict__ list, double4* __restrict__ part, int* __restrict__ done,
             double* __restrict__ phi, double* __restrict__ grad) {
@@ -571,7 +643,7 @@ __global__ void __launch_bounds__(256)
     if (!__any_sync(mask, bx * bx + by * by + bz * bz < rc2)) continue;
     for (int k = 0; k < s.bnum; ++k) {
       const float4 b = body32[s.boff + k];
-      const float dx = xt.x - (b.x + s.dx), dy = xt.y - (b.y + s.dy), dz = xt.z - (b.z + s.dz);
+      const float dx = px - b.x, dy = py - b.y, dz = pz - b.z;
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
       if (r2 < rc2 && !(s.self && s.boff + k == t)) {
         if (EMIT) {
@@ -603,8 +675,8 @@ __global__ void k_close_fix(const double4* __restrict__ body64, const float4* __
     const P2PSrc32 s = list[pr.y];
     // the FP32 terms exactly as k_p2p32 formed them
     const float4 b = body32[pr.x];
-    const float dx = __fadd_rn(xt.x, -__fadd_rn(b.x, s.dx)), dy = __fadd_rn(xt.y, -__fadd_rn(b.y, s.dy)),
-                dz = __fadd_rn(xt.z, -__fadd_rn(b.z, s.dz));
+    const float px = xt.x - s.dx, py = xt.y - s.dy, pz = xt.z - s.dz;
+    const float dx = __fadd_rn(px, -b.x), dy = __fadd_rn(py, -b.y), dz = __fadd_rn(pz, -b.z);
     float r2 = __fmul_rn(dz, dz);
     r2 = __fmaf_rn(dy, dy, r2);
     r2 = __fmaf_rn(dx, dx, r2);
@@ -2109,10 +2181,13 @@ cudaError_t launch_prep32(const double4* body64, const int* body_leaf, const Lea
   return cudaGetLastError();
 }
 
-cudaError_t launch_p2p32(const float4* body32, const P2PItem* items, int nitems, const P2PSrc32* list, double4* part,
-                         int* done, double* phi, double* grad, cudaStream_t st) {
-  if (nitems > 0)
-    k_p2p32<<<cdiv(nitems, kP2PWarps), 32 * kP2PWarps, 0, st>>>(body32, items, nitems, list, part, done, phi, grad);
+cudaError_t launch_p2p32(const float4* body32, const P2PItem* items, int nitems, bool long_entries, bool cut,
+                         const P2PSrc32* list, double4* part, int* done, double* phi, double* grad, cudaStream_t st) {
+  if (nitems > 0) {
+    auto kernel = long_entries ? cut ? k_p2p32<true, true> : k_p2p32<true, false>
+                               : cut ? k_p2p32<false, true> : k_p2p32<false, false>;
+    kernel<<<cdiv(nitems, kP2PWarps), 32 * kP2PWarps, 0, st>>>(body32, items, nitems, list, part, done, phi, grad);
+  }
   return cudaGetLastError();
 }
 

@@ -47,6 +47,19 @@ inline int p2p_part_bodies(unsigned long long work) {
   return s < 256 ? 256 : s > (1 << 20) ? 1 << 20 : (int)s;
 }
 
+// Whether a plan's FP32 P2P takes its sources entry by entry or fills its tiles
+// across entries, by the mean bodies of an entry: `work` as above, `entries` =
+// sum over leaves of list entries x target groups of 32.  Entry by entry leaves
+// tiles part empty, across entries costs a frame offset a pair and more sums
+// into FP64.  Stage times, entry by entry and across: mean 12.8 bodies (2^20
+// uniform) 1.48 and 0.87 ms, 15.6 (64,000 on a lattice) 0.049 and 0.046, 17.9
+// (100,003 uniform) 0.093 and 0.085, 24.4 0.073 and 0.081, 27.6 (150,001 in
+// blobs) 0.245 and 0.251, 32 (2^20) 0.70 and 0.76, 256 3.7 and 4.6.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool p2p_long_entries(unsigned long long work, unsigned long long entries) { return work >= 20 * entries; }
+
 // One P2P list entry (source leaf) of a target leaf, FP32 form.  Both forms
 // carry the source's body range so that the kernels read bodies with one
 // dependent load.
@@ -84,7 +97,7 @@ cudaError_t launch_prep32(const double4* body64, const int* body_leaf, const Lea
                           float4* body32, int n, cudaStream_t st);
 // part: 32 double4 per slot of the items, done: one counter per slot, zero
 // before the first pass (every pass leaves them zero)
-cudaError_t launch_p2p32(const float4* body32, const P2PItem* items, int nitems,
+cudaError_t launch_p2p32(const float4* body32, const P2PItem* items, int nitems, bool long_entries, bool cut,
                          const P2PSrc32* list, double4* part, int* done, double* phi, double* grad,
                          cudaStream_t st);
 cudaError_t launch_p2p64(const double4* body64, const P2PItem* items, int nitems,

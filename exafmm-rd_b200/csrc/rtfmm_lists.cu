@@ -438,8 +438,8 @@ __device__ __forceinline__ void leaf_run(const LeafTables& T, int c, int* lo, in
   *hi = T.dfs_pos[T.body_leaf[b0 + nb - 1]] + 1;
 }
 
-// cnt: list entries of leaf l; bodies: bodies of those entries; work: their
-// sum over the leaves, times the leaf's target groups.
+// cnt: list entries of leaf l; bodies: bodies of those entries; work[0], [1]:
+// the sums of bodies and entries over the leaves, times the leaf's target groups.
 __global__ void k_leaf_list_count(LeafTables T, int* __restrict__ cnt, long long* __restrict__ bodies,
                                   unsigned long long* __restrict__ work) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
@@ -458,7 +458,9 @@ __global__ void k_leaf_list_count(LeafTables T, int* __restrict__ cnt, long long
     }
   cnt[l] = c;
   bodies[l] = nb;
-  atomicAdd(work, (unsigned long long)nb * ((T.leaves[l].bnum + 31) / 32));
+  const unsigned long long groups = (T.leaves[l].bnum + 31) / 32;
+  atomicAdd(work, (unsigned long long)nb * groups);
+  atomicAdd(work + 1, (unsigned long long)c * groups);
 }
 
 // Work items of leaf l: its target groups of 32 times the parts of its list.
@@ -553,19 +555,19 @@ int device_p2p_tables(const DeviceWalk& w, const DeviceLeafInput& in, bool mixed
   const int nlf = in.nlf;
   int *cstart, *cend, *cnt, *icnt, *off, *ioff;
   long long* bodies;
-  unsigned long long* total;  // body pairs, work, slots
+  unsigned long long* total;  // body pairs, work, entries, slots
   LCK(S.get(0, &cstart, w.ncell));
   LCK(S.get(1, &cend, w.ncell));
   LCK(S.get(2, &cnt, nlf + 1));
   LCK(S.get(3, &icnt, nlf + 1));
   LCK(S.get(4, &ioff, nlf + 1));
-  LCK(S.get(5, &total, 3));
+  LCK(S.get(5, &total, 4));
   LCK(S.get(7, &bodies, nlf));
   LCK(cudaMemsetAsync(cstart, 0, sizeof(int) * w.ncell, st));
   LCK(cudaMemsetAsync(cend, 0, sizeof(int) * w.ncell, st));
   LCK(cudaMemsetAsync(cnt + nlf, 0, sizeof(int), st));
   LCK(cudaMemsetAsync(icnt + nlf, 0, sizeof(int), st));
-  LCK(cudaMemsetAsync(total, 0, 3 * sizeof(unsigned long long), st));
+  LCK(cudaMemsetAsync(total, 0, 4 * sizeof(unsigned long long), st));
   if (w.npairs > 0) {
     k_pair_bounds<<<cdiv(w.npairs, 256), 256, 0, st>>>(w.pairs, w.npairs, cstart, cend);
     LCK(cudaGetLastError());
@@ -602,14 +604,15 @@ int device_p2p_tables(const DeviceWalk& w, const DeviceLeafInput& in, bool mixed
     return kTreeError;
   }
   k_leaf_list_fill<<<cdiv(nlf, 128), 128, 0, st>>>(T, off, ioff, bodies, mixed ? 1 : 0, l32, l64, items, total,
-                                                   reinterpret_cast<int*>(total + 2));
+                                                   reinterpret_cast<int*>(total + 3));
   LCK(cudaGetLastError());
-  unsigned long long sums[3];
+  unsigned long long sums[4];
   LCK(cudaMemcpyAsync(sums, total, sizeof(sums), cudaMemcpyDeviceToHost, st));
   LCK(cudaStreamSynchronize(st));
   out->nlist = tot[0];
   out->nitems = tot[1];
-  out->nslots = (int)(unsigned)sums[2];
+  out->nslots = (int)(unsigned)sums[3];
+  out->long_entries = p2p_long_entries(sums[1], sums[2]);
   out->pairs = (int64_t)sums[0];
   return kTreeOk;
 }

@@ -79,6 +79,7 @@ struct P2PTableAlloc {
 };
 struct P2PTablesOut {
   int nlist = 0, nitems = 0, nslots = 0;
+  bool long_entries = false;  // p2p_long_entries
   int64_t pairs = 0;  // body pairs: sum over entries of n_target * n_source
 };
 int device_p2p_tables(const DeviceWalk& w, const DeviceLeafInput& in, bool mixed, cudaStream_t st,

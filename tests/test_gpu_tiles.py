@@ -80,6 +80,54 @@ def test_near_field_with_long_lists(pkg, oracle, images, precision):
     assert l2(grad, rgrad) < tol and l2(phi, rphi) < tol
 
 
+# a part of a list may hold no entry at all: leaves of 625 bodies beside parts
+# of 256
+@pytest.mark.parametrize("precision", [0, 1])
+def test_near_field_with_entries_above_a_part(pkg, precision):
+    x, q = uniform01(5000, 12)
+    f = pkg.LaplaceFMM(x, q, args(pkg, 4, 900, 0, precision, pkg.STAGE_NEAR))
+    phi, grad = f.solve()
+    assert f.info()["nleaf"] == 8  # each beside all others: the near field is the direct sum
+    f.close()
+    d = x[:, None] - x[None]
+    r2 = (d * d).sum(2)
+    np.fill_diagonal(r2, np.inf)
+    t = q / np.sqrt(r2) / (4 * np.pi)
+    tol = 1e-5 if precision else 1e-12
+    assert l2(phi, t.sum(1)) < tol
+    assert l2(grad, -np.einsum("ij,ijk->ik", t / r2, d)) < tol
+
+
+# FP32 terms meet in FP64: neither the two halves of a packed sum nor the terms
+# of two small leaves are added in FP32, where a term of 2^-30 beside one of 1
+# is lost.  One leaf of 3 bodies, one of 40 (the form for long entries), and
+# 26 leaves of one body around a target
+@pytest.mark.parametrize("case", ["leaf of 3", "leaf of 40", "leaves of 1"])
+def test_fp32_terms_meet_in_fp64(pkg, case):
+    if case == "leaves of 1":
+        x = (np.stack(np.meshgrid(*[np.arange(3)] * 3, indexing="ij"), -1).reshape(-1, 3) + 0.5) / 4
+        target, strong, weak, ncrit = 13, 4, [k for k in range(27) if k not in (4, 13)], 1
+    else:
+        n = 3 if case == "leaf of 3" else 40
+        x = np.random.default_rng(3).random((n, 3)) * 0.2
+        x[:3] = [[0.25, 0.5, 0.5], [0.5, 0.75, 0.5], [0.5, 0.5, 0.5]]  # sources 0 and 1 of a pair
+        target, strong, weak, ncrit = 2, 0, [1], 64
+    q = np.zeros(len(x))
+    f = pkg.LaplaceFMM(x, q, args(pkg, 4, ncrit, 0, 1, pkg.STAGE_NEAR))
+    f.setup()
+    q[strong] = 1.0
+    phi0, grad0 = f.evaluate(q)
+    q[weak] = 2.0 ** -30
+    phi, grad = f.evaluate(q)
+    f.close()
+    d = x[target] - x[weak]
+    t = 2.0 ** -30 / np.linalg.norm(d, axis=1) / (4 * np.pi)
+    g = t[:, None] * d / (d * d).sum(1)[:, None]
+    # the weak terms' own FP32 rounding (reciprocal square root: 2^-22)
+    assert abs(phi[target] - phi0[target] - t.sum()) < 1e-5 * t.sum()
+    assert np.abs(grad[target] - grad0[target] + g.sum(0)).max() < 1e-5 * np.abs(g).sum()
+
+
 # octrees below the first sorted digits (12 levels), and leaves above the size
 # ordered by counting (1500 bodies)
 @pytest.mark.parametrize("ncrit,scale", [(4, 2e-4), (1500, 1.0)])
