@@ -17,6 +17,7 @@
 // Every index a kernel forms is checked against the extent of the buffer it
 // addresses; no kernel waits on another block.
 #include "rtfmm_kernels.cuh"
+#include "rtfmm_rsqrt.cuh"
 
 #include <cuda_runtime.h>
 
@@ -91,40 +92,6 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-
-// 1/sqrt(x) in FP64 from the hardware seed (one special-function op, 9.1e-7
-// relative), and zero for x = 0; other x must be normal (pairs closer than
-// 1e-154 are not supported).  The zero is made by the seed's words on the
-// integer pipe: a comparison would take the FP64 pipe, which bounds every
-// kernel that calls this.
-__device__ __forceinline__ double rsqrt_seed(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const int hi = __double2hiint(x);
-  return __hiloint2double(hi ? __double2hiint(y) : 0, hi ? __double2loint(y) : 0);
-}
-// To full precision: with e = 1 - x y^2 the Taylor series of (1 - e)^(-1/2) to
-// second order, y (1 + e/2 + 3 e^2/8) (Householder's method of third order;
-// the remainder 5/16 e^3 is 2e-18): five operations, where two Newton steps
-// take seven.
-__device__ __forceinline__ double rsqrt_or_zero(double x) {
-  const double y = rsqrt_seed(x);
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-// Twice 1/sqrt(x) to 1.3e-12 (maximum against CUDA's rsqrt over 1e-30..1e30):
-// one Newton step y (3 - x y^2), whose factor 1/2 the callers put into the
-// charges, three operations instead of four.
-__device__ __forceinline__ double rsqrt_twice(double x) {
-  const double y = rsqrt_seed(x);
-  return y * fma(-(x * y), y, 3.0);
-}
-// What the surface kernels use: FULL 1/sqrt(x), else 2/sqrt(x) with charges
-// halved (kHalf, exact).
-template <bool FULL>
-__device__ __forceinline__ double rsqrt_surf(double x) {
-  return FULL ? rsqrt_or_zero(x) : rsqrt_twice(x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1767,33 +1734,31 @@ __global__ void __launch_bounds__(HadCfg<T>::THREADS, HadCfg<T>::MINB)
 // Hadamard 8x8 in FP64, on the FP64 tensor path.
 //
 // The 8x8 block of a direction depends on a child pair only through its
-// offset, so along x it is a 2x2 Toeplitz matrix of 4x4 blocks (a on the
-// diagonal, b for source x = 1 and target x = 0, c for the converse), and
-//   y0 = a (x0 + x1) + (b - a) x1,   y1 = a (x0 + x1) + (c - a) x0
-// takes three 4x4 products instead of four.  The sum over the directions is
-// linear, so the three products are accumulated on their own and combined
-// once at the end.  Each is a real 8x8 matrix (4 complex slots) applied to 8
-// targets: two mma.sync.m8n8k4 (real parts, then imaginary parts of the four
-// source slots).  Against the product in full this does 192 instead of 256
-// multiply-adds per (target, direction, frequency), and a coefficient read
-// feeds 32 targets instead of one, which is what bounded the FP64 form on the
-// FMA pipe (every multiply-add waited for its share of a shared-memory
-// broadcast).  The rounding error of the spectra against 80-bit sums is
-// 0.6-1.1 times that of the full product (P = 4-10).
+// offset, so along x it is a 2x2 Toeplitz matrix of three 4x4 blocks (a on the
+// diagonal, b for source x = 1 and target x = 0, c for the converse):
+//   y0 = a x0 + b x1,   y1 = c x0 + a x1.
+// Each product is a real 8x8 matrix (4 complex slots) applied to 8 targets by
+// two mma.sync.m8n8k4 (real parts, then imaginary parts of the four source
+// slots), and a coefficient read feeds 24 targets, which on the FMA pipe
+// bounded this product (every multiply-add waited for its share of a
+// shared-memory broadcast).  A direction's products are summed by themselves
+// and then added to the sum over the directions: 0.99-1.0 times the error of
+// the same order of sums in plain FP64 (tests/kernel_errors.cu).  Three
+// products instead of four, a (x0 + x1), (b - a) x1 and (c - a) x0, accumulated
+// over all directions take 1.92 ms instead of 2.51 (below) but have 1.4 to 4.7
+// times that error.
 //
 // A block takes one frequency and 96 targets, a warp 24 of them as three
 // tiles of 8; lane 4 r + q holds source slot q (and q + 4) of target row r.
 // A tile none of whose targets has a source in a direction skips it.
-// Three tiles a warp leave room for four blocks an SM (128 registers): 1.91 ms
-// at N = 2^20, P = 8, ncrit = 256 and 1.82 ms at N = 2^18, ncrit = 64, against
-// 2.04 and 1.95 ms with four tiles and three blocks; two tiles and five blocks
-// took 1.10 times as long as three and four.  3.58 ms for the product in full
-// on the FMA pipe (N = 2^20).  The FP64 tensor pipe is 70% busy (27 of DGEMM's 35 TFLOP/s,
-// counting the 40% of the (target, direction) slots that are empty there).
+// Three tiles a warp and four blocks an SM (122 registers): 2.51 ms at
+// N = 2^20, P = 8, ncrit = 256 and 2.43 ms at N = 2^18, ncrit = 64, against
+// 2.68 and 2.61 with four tiles and three blocks, 2.80 and 2.68 with two and
+// five; 3.60 and 3.34 ms for the product on the FMA pipe.
 // ---------------------------------------------------------------------------
 constexpr int kHad64Tiles = 3, kHad64Threads = 128, kHad64Blocks = 4;
 
-// Coefficients of a frequency: [direction][product][source slot][target slot]
+// Coefficients of a frequency: [direction][block][source slot][target slot]
 constexpr int kG64PerDir = 3 * 16;
 
 __device__ __forceinline__ double2 ld_nc_f64x2(const double* p) {
@@ -1806,7 +1771,7 @@ __global__ void __launch_bounds__(kHad64Threads, kHad64Blocks)
     k_m2l_hadamard8_f64(const double* __restrict__ Q, const double2* __restrict__ G, const int* __restrict__ tsrcT,
                         int ntar, int nsrc, double* __restrict__ Pk) {
   constexpr int MT = kHad64Tiles;
-  // B fragments of both mma of a product, per lane
+  // B fragments of both mma of a block, per lane
   __shared__ __align__(16) double2 Bs[26 * 3 * 32];
   const int f = blockIdx.y;
   const double2* Gf = G + (size_t)f * 26 * kG64PerDir;
@@ -1837,23 +1802,30 @@ __global__ void __launch_bounds__(kHad64Threads, kHad64Blocks)
       }
     }
   };
-  double acc[3][MT][2];
+  double acc[2][MT][2];
 #pragma unroll
-  for (int k = 0; k < 3; ++k)
+  for (int k = 0; k < 2; ++k)
 #pragma unroll
     for (int m = 0; m < MT; ++m) acc[k][m][0] = acc[k][m][1] = 0.0;
   auto mac = [&](int d, const int (&sd)[MT], const double2 (&x0)[MT], const double2 (&x1)[MT]) {
-    const double2 b0 = Bs[(3 * d + 0) * 32 + lane], b1 = Bs[(3 * d + 1) * 32 + lane], b2 = Bs[(3 * d + 2) * 32 + lane];
+    const double2 a = Bs[(3 * d + 0) * 32 + lane], b = Bs[(3 * d + 1) * 32 + lane], c = Bs[(3 * d + 2) * 32 + lane];
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
       if (!__any_sync(0xffffffffu, sd[m] >= 0)) continue;
-      const double sr = x0[m].x + x1[m].x, si = x0[m].y + x1[m].y;
-      dmma8x8x4(acc[0][m], x1[m].x, b0.x);
-      dmma8x8x4(acc[1][m], sr, b1.x);
-      dmma8x8x4(acc[2][m], x0[m].x, b2.x);
-      dmma8x8x4(acc[0][m], x1[m].y, b0.y);
-      dmma8x8x4(acc[1][m], si, b1.y);
-      dmma8x8x4(acc[2][m], x0[m].y, b2.y);
+      double y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0};
+      dmma8x8x4(y0, x0[m].x, a.x);
+      dmma8x8x4(y1, x0[m].x, c.x);
+      dmma8x8x4(y0, x0[m].y, a.y);
+      dmma8x8x4(y1, x0[m].y, c.y);
+      dmma8x8x4(y0, x1[m].x, b.x);
+      dmma8x8x4(y1, x1[m].x, a.x);
+      dmma8x8x4(y0, x1[m].y, b.y);
+      dmma8x8x4(y1, x1[m].y, a.y);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        acc[0][m][e] += y0[e];
+        acc[1][m][e] += y1[e];
+      }
     }
   };
   // two-stage pipeline over the directions: the source rows of direction d+1
@@ -1891,8 +1863,8 @@ __global__ void __launch_bounds__(kHad64Threads, kHad64Blocks)
     const int t = t0 + 8 * m;
     if (t >= ntar) break;
     double2* out = reinterpret_cast<double2*>(Pk) + ((size_t)f * ntar + t) * 8 + q;
-    out[0] = make_double2(acc[1][m][0] + acc[0][m][0], acc[1][m][1] + acc[0][m][1]);
-    out[4] = make_double2(acc[1][m][0] + acc[2][m][0], acc[1][m][1] + acc[2][m][1]);
+    out[0] = make_double2(acc[0][m][0], acc[0][m][1]);
+    out[4] = make_double2(acc[1][m][0], acc[1][m][1]);
   }
 }
 
@@ -1909,21 +1881,16 @@ __global__ void k_g8_layout(const double2* __restrict__ cc8, int Nf, float2* __r
   }
 }
 
-// The same for the FP64 form: the coefficients of its three products,
-// G[((f * 26 + d) * 3 + k) * 16 + 4 s + t] = b - a, a, c - a (k = 0, 1, 2) of
-// source slot s and target slot t (y and z octant bits).
+// The same for the FP64 form: the coefficients of its three blocks,
+// G[((f * 26 + d) * 3 + k) * 16 + 4 s + t] = a, b, c (k = 0, 1, 2) of source
+// slot s and target slot t (y and z octant bits).
 __global__ void k_g8_layout64(const double2* __restrict__ cc8, int Nf, double2* __restrict__ G) {
   const size_t total = (size_t)26 * kG64PerDir * Nf;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
     const int t = (int)(e % 4), s = (int)(e / 4 % 4), k = (int)(e / 16 % 3), d = (int)(e / 48 % 26);
     const size_t f = e / (48 * 26);
     auto at = [&](int isrc, int itar) { return cc8[((size_t)d * 64 + isrc * 8 + itar) * Nf + f]; };
-    double2 v = at(s, t);
-    if (k != 1) {
-      const double2 o = k == 0 ? at(s + 4, t) : at(s, t + 4);
-      v = make_double2(o.x - v.x, o.y - v.y);
-    }
-    G[e] = v;
+    G[e] = k == 0 ? at(s, t) : k == 1 ? at(s + 4, t) : at(s, t + 4);
   }
 }
 
