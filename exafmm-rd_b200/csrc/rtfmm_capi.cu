@@ -150,10 +150,11 @@ struct rtfmm_fmm {
   // operator tables: generation built on the host / uploaded to the device
   uint64_t ops_gen = 0, ops_dev_gen = 0;
   size_t h_xin_cap = 0;  // doubles in h_xin
+  bool xin_staged = false;  // h_xin holds the positions of the set-up
   char* h_pack = nullptr;  // pinned staging of the plan's tables (PlanPack)
   size_t h_pack_cap = 0;
   char d_pack = 0;  // pool key of their device buffer
-  // x_in, q_in, plan.x, plan.q, plan.perm and h_xin hold the set-up bodies;
+  // x_in, q_in, plan.x, plan.q and plan.perm hold the set-up bodies;
   // after a device set-up they are fetched from d_xin, d_qin and d_perm on
   // first use (ensure_host_bodies)
   bool host_bodies = true;
@@ -970,9 +971,11 @@ int alloc_parts(rtfmm_fmm* f) {
   return RTFMM_OK;
 }
 
-// The positions in pinned memory, where the host-buffer calls move them from;
-// a handle whose bodies came from device memory has none until such a call.
+// The host bodies' positions in pinned memory, where the host-buffer calls move
+// them from: made by the first call of a set-up that does (queries and
+// device-buffer calls never need it).
 int stage_positions(rtfmm_fmm* f) {
+  if (f->xin_staged) return RTFMM_OK;
   const int64_t n = f->plan.n;
   if (f->h_xin_cap < (size_t)std::max<int64_t>(1, 3 * n)) {
     if (f->h_xin) cudaFreeHost(f->h_xin);
@@ -983,6 +986,7 @@ int stage_positions(rtfmm_fmm* f) {
     f->h_xin_cap = cap;
   }
   if (n > 0) std::memcpy(f->h_xin, f->x_in.data(), sizeof(double) * 3 * n);
+  f->xin_staged = true;
   return RTFMM_OK;
 }
 
@@ -1105,7 +1109,6 @@ int upload_plan(rtfmm_fmm* f) {
   RC(pack.upload(f));
   if (f->shard_n <= 1) f->d_leaves_own = f->d_leaves;
   if (body_leaf_here) CK(launch_body_leaf(f->d_leaves, (int)nleaf, (int)n, f->d_body_leaf, f->s0));
-  if (f->host_bodies) RC(stage_positions(f));
 #undef RC
   f->device_ready = true;
   f->setup_s[5] = wall_s() - t0;
@@ -1558,7 +1561,7 @@ namespace {
 
 // After a device set-up: the input-order bodies and the permutation from
 // the device into x_in, q_in, plan.perm, plus (with tree_order) plan.x,
-// plan.q and the pinned staging copy.  Called before anything overwrites
+// plan.q.  Called before anything overwrites
 // d_xin or d_qin.
 int ensure_host_bodies(rtfmm_fmm* f, bool tree_order = true) {
   if (f->host_bodies) return RTFMM_OK;
@@ -1587,8 +1590,6 @@ int ensure_host_bodies(rtfmm_fmm* f, bool tree_order = true) {
     p.x[3 * i + 2] = f->x_in[3 * k + 2];
     p.q[i] = f->q_in[k];
   }
-  int rc = stage_positions(f);
-  if (rc) return rc;
   f->host_bodies = true;
   return RTFMM_OK;
 }
@@ -1707,6 +1708,7 @@ int device_tables(rtfmm_fmm* f, const TreeScratchFn& scratch) {
 void begin_setup(rtfmm_fmm* f, int64_t n) {
   f->setup_done = false;
   f->pass_done = false;
+  f->xin_staged = false;
   f->plan = Plan();
   f->plan.args = f->args;
   f->plan.n = n;
@@ -1834,7 +1836,7 @@ int rtfmm_b200_upload(rtfmm_fmm* f) {
   }
   CK(cudaSetDevice(f->dev));
   int rc = ensure_host_bodies(f);
-  if (rc) return rc;
+  if (rc || (rc = stage_positions(f))) return rc;
   const int64_t n = f->plan.n;
   if (n > 0) {
     // input order up (positions from the pinned copy), tree order on the device
@@ -1923,7 +1925,7 @@ int rtfmm_b200_evaluate(rtfmm_fmm* f, const double* q, double* phi, double* grad
   const bool staged = q && f->pos_on_device;
   if (!staged) {
     int rc0 = ensure_host_bodies(f);
-    if (rc0) return rc0;
+    if (rc0 || (!f->pos_on_device && (rc0 = stage_positions(f)))) return rc0;
   } else {
     int rc0 = dalloc(f, &f->d_stage_q, (size_t)n);
     if (rc0) return rc0;
@@ -2047,7 +2049,7 @@ int rtfmm_b200_adjoint(rtfmm_fmm* f, const double* w, double* dLdq, double* dLdx
   int rc = ensure_adj_scratch(f);
   if (rc) return rc;
   rc = ensure_host_bodies(f);
-  if (rc) return rc;
+  if (rc || (rc = stage_positions(f))) return rc;
   // the bodies with the set-up charges, as the forward solve had them
   CK(cudaMemcpyAsync(f->d_xin, f->h_xin, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, f->s0));
   CK(cudaMemcpyAsync(f->d_qin, f->q_in.data(), sizeof(double) * n, cudaMemcpyHostToDevice, f->s0));

@@ -239,3 +239,28 @@ def test_solve_sets_up_on_the_gpu(pkg, precision):
     assert np.array_equal(phi2, rphi2) and np.array_equal(grad2, rgrad2)
     f.close()
     g.close()
+
+
+# a query after a device set-up fetches the bodies, but makes no pinned copy of
+# the positions: that is for the calls which move them
+def test_queries_pin_no_positions(pkg):
+    x, q = uniform01(20000, 21)
+    a = pkg.Argument(P=4, ncrit=64, images=0, cycle=1.0, x=(0.5, 0.5, 0.5), dipole_correction=0, divide_4pi=1)
+    d = pkg.LaplaceFMM(np.empty((0, 3)), np.empty(0), a)
+    xd, qd = torch.from_numpy(x).cuda(), torch.from_numpy(q).cuda()
+    torch.cuda.synchronize()
+    d.setup_device(xd.data_ptr(), qd.data_ptr(), len(q))
+
+    def calls(f):
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU,
+                                                torch.profiler.ProfilerActivity.CUDA]) as prof:
+            f()
+            torch.cuda.synchronize()
+        return {e.name for e in prof.events()}
+
+    seen = calls(lambda: d.perm())
+    assert "cudaMemcpyAsync" in seen  # the library's calls are recorded
+    assert not {"cudaMallocHost", "cudaHostAlloc"} & seen
+    seen = calls(lambda: d.adjoint(q))
+    assert {"cudaMallocHost", "cudaHostAlloc"} & seen
+    d.close()
