@@ -102,7 +102,6 @@ struct rtfmm_fmm {
   bool device_ready = false;
   bool pass_done = false;
   std::vector<double> x_in;  // input-order positions of the set-up bodies
-  double* h_xin = nullptr;   // pinned copy of x_in (host -> device source)
   std::vector<double> q_in;
 
   // host plan tables
@@ -149,8 +148,6 @@ struct rtfmm_fmm {
   std::unordered_map<const void*, DevSlot> pool;
   // operator tables: generation built on the host / uploaded to the device
   uint64_t ops_gen = 0, ops_dev_gen = 0;
-  size_t h_xin_cap = 0;  // doubles in h_xin
-  bool xin_staged = false;  // h_xin holds the positions of the set-up
   char* h_pack = nullptr;  // pinned staging of the plan's tables (PlanPack)
   size_t h_pack_cap = 0;
   char d_pack = 0;  // pool key of their device buffer
@@ -308,7 +305,11 @@ struct PlanPack {
     const void* h;
     size_t bytes, off;
   };
-  static constexpr size_t kMax = 4 << 20;  // a larger table is copied by itself (pinned memory is dear)
+  // A larger table is copied by itself: pinned memory takes the first upload of
+  // a handle about a millisecond a megabyte (30011 bodies: 17 ms with tables up
+  // to 4 MB in it, 13 with this), and a blocking copy costs little beside the
+  // move of 512 KB (a time step of 100003 bodies 2.60 ms, 2.65-2.75 with 4 MB).
+  static constexpr size_t kMax = 512 << 10;
   std::vector<Part> parts;
   size_t total = 0;
   template <typename T>
@@ -358,12 +359,10 @@ void free_device(rtfmm_fmm* f) {
   for (auto& kv : f->pool)
     if (kv.second.p) cudaFree(kv.second.p);
   f->pool.clear();
-  // after the cudaFree above, which waits for copies from these
-  if (f->h_xin) cudaFreeHost(f->h_xin);
+  // after the cudaFree above, which waits for copies from it
   if (f->h_pack) cudaFreeHost(f->h_pack);
-  f->h_xin = nullptr;
   f->h_pack = nullptr;
-  f->h_xin_cap = f->h_pack_cap = 0;
+  f->h_pack_cap = 0;
   f->ops_dev_gen = 0;
   f->d_flush = nullptr;
   f->flush_bytes = 0;
@@ -968,25 +967,6 @@ int alloc_parts(rtfmm_fmm* f) {
   if ((rc = dalloc(f, &f->d_part, 32 * (size_t)f->n_slots)) || (rc = dalloc(f, &f->d_part_done, (size_t)f->n_slots)))
     return rc;
   CK(cudaMemsetAsync(f->d_part_done, 0, sizeof(int) * std::max(1, f->n_slots), f->s0));
-  return RTFMM_OK;
-}
-
-// The host bodies' positions in pinned memory, where the host-buffer calls move
-// them from: made by the first call of a set-up that does (queries and
-// device-buffer calls never need it).
-int stage_positions(rtfmm_fmm* f) {
-  if (f->xin_staged) return RTFMM_OK;
-  const int64_t n = f->plan.n;
-  if (f->h_xin_cap < (size_t)std::max<int64_t>(1, 3 * n)) {
-    if (f->h_xin) cudaFreeHost(f->h_xin);
-    f->h_xin = nullptr;
-    f->h_xin_cap = 0;
-    const size_t cap = (size_t)std::max<int64_t>(1, 3 * n + 3 * n / 4);
-    CK(cudaMallocHost(&f->h_xin, sizeof(double) * cap));
-    f->h_xin_cap = cap;
-  }
-  if (n > 0) std::memcpy(f->h_xin, f->x_in.data(), sizeof(double) * 3 * n);
-  f->xin_staged = true;
   return RTFMM_OK;
 }
 
@@ -1708,7 +1688,6 @@ int device_tables(rtfmm_fmm* f, const TreeScratchFn& scratch) {
 void begin_setup(rtfmm_fmm* f, int64_t n) {
   f->setup_done = false;
   f->pass_done = false;
-  f->xin_staged = false;
   f->plan = Plan();
   f->plan.args = f->args;
   f->plan.n = n;
@@ -1836,11 +1815,11 @@ int rtfmm_b200_upload(rtfmm_fmm* f) {
   }
   CK(cudaSetDevice(f->dev));
   int rc = ensure_host_bodies(f);
-  if (rc || (rc = stage_positions(f))) return rc;
+  if (rc) return rc;
   const int64_t n = f->plan.n;
   if (n > 0) {
-    // input order up (positions from the pinned copy), tree order on the device
-    CK(cudaMemcpyAsync(f->d_xin, f->h_xin, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, f->s0));
+    // input order up, tree order on the device
+    CK(cudaMemcpyAsync(f->d_xin, f->x_in.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice, f->s0));
     CK(cudaMemcpyAsync(f->d_qin, f->q_in.data(), sizeof(double) * n, cudaMemcpyHostToDevice, f->s0));
     CK(launch_gather_bodies(f->d_xin, f->d_qin, f->d_perm, (int)n, f->d_body64, f->s0));
     CK(cudaStreamSynchronize(f->s0));
@@ -1925,7 +1904,7 @@ int rtfmm_b200_evaluate(rtfmm_fmm* f, const double* q, double* phi, double* grad
   const bool staged = q && f->pos_on_device;
   if (!staged) {
     int rc0 = ensure_host_bodies(f);
-    if (rc0 || (!f->pos_on_device && (rc0 = stage_positions(f)))) return rc0;
+    if (rc0) return rc0;
   } else {
     int rc0 = dalloc(f, &f->d_stage_q, (size_t)n);
     if (rc0) return rc0;
@@ -1943,7 +1922,7 @@ int rtfmm_b200_evaluate(rtfmm_fmm* f, const double* q, double* phi, double* grad
   if (f->pos_on_device) {
     CK(launch_set_charges(f->d_body64, qdst, f->d_perm, (int)n, f->s0));
   } else {
-    CK(cudaMemcpyAsync(f->d_xin, f->h_xin, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, f->s0));
+    CK(cudaMemcpyAsync(f->d_xin, f->x_in.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice, f->s0));
     CK(launch_gather_bodies(f->d_xin, f->d_qin, f->d_perm, (int)n, f->d_body64, f->s0));
     f->pos_on_device = true;
   }
@@ -2049,9 +2028,10 @@ int rtfmm_b200_adjoint(rtfmm_fmm* f, const double* w, double* dLdq, double* dLdx
   int rc = ensure_adj_scratch(f);
   if (rc) return rc;
   rc = ensure_host_bodies(f);
-  if (rc || (rc = stage_positions(f))) return rc;
+  if (rc) return rc;
   // the bodies with the set-up charges, as the forward solve had them
-  CK(cudaMemcpyAsync(f->d_xin, f->h_xin, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, f->s0));
+  if (!f->pos_on_device)
+    CK(cudaMemcpyAsync(f->d_xin, f->x_in.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice, f->s0));
   CK(cudaMemcpyAsync(f->d_qin, f->q_in.data(), sizeof(double) * n, cudaMemcpyHostToDevice, f->s0));
   CK(launch_gather_bodies(f->d_xin, f->d_qin, f->d_perm, (int)n, f->d_body64, f->s0));
   f->grad_q_valid = false;

@@ -241,9 +241,9 @@ def test_solve_sets_up_on_the_gpu(pkg, precision):
     g.close()
 
 
-# a query after a device set-up fetches the bodies, but makes no pinned copy of
-# the positions: that is for the calls which move them
-def test_queries_pin_no_positions(pkg):
+# a query after a device set-up fetches the bodies and the host-buffer adjoint
+# finds the positions on the device: neither makes a pinned copy of them
+def test_queries_and_adjoint_pin_no_positions(pkg):
     x, q = uniform01(20000, 21)
     a = pkg.Argument(P=4, ncrit=64, images=0, cycle=1.0, x=(0.5, 0.5, 0.5), dipole_correction=0, divide_4pi=1)
     d = pkg.LaplaceFMM(np.empty((0, 3)), np.empty(0), a)
@@ -258,9 +258,8 @@ def test_queries_pin_no_positions(pkg):
             torch.cuda.synchronize()
         return {e.name for e in prof.events()}
 
-    seen = calls(lambda: d.perm())
-    assert "cudaMemcpyAsync" in seen  # the library's calls are recorded
-    assert not {"cudaMallocHost", "cudaHostAlloc"} & seen
-    seen = calls(lambda: d.adjoint(q))
-    assert {"cudaMallocHost", "cudaHostAlloc"} & seen
+    for f in (d.perm, lambda: d.adjoint(q)):
+        seen = calls(f)
+        assert "cudaMemcpyAsync" in seen  # the library's calls are recorded
+        assert not {"cudaMallocHost", "cudaHostAlloc"} & seen
     d.close()
