@@ -1,5 +1,5 @@
 // C ABI of the B200 FMM evaluation pass: handle, device buffers and the
-// orchestration of one pass across two CUDA streams.
+// orchestration of one pass across three CUDA streams.
 //
 //   stream s0 (far field):  P2M -> M2M levels -> FFT-M2L (up, Hadamard, down)
 //                           -> L2L levels -> L2P            ... then post
@@ -430,7 +430,7 @@ void build_tables(rtfmm_fmm* f, bool host_p2p = true) {
     f->body_leaf.clear();
   }
 
-  // P2P lists in CSR by target leaf; work items of 32 / 64 targets.  The
+  // P2P lists in CSR by target leaf; work items of up to 32 targets.  The
   // reference's M2P/P2L-to-P2P conversions (traverser.cpp:75-86) can pair a
   // non-leaf cell with a leaf, evaluated over the cell's whole body range
   // (p2p_1toN_256, kernel.cpp:276-301).  Such a pair is expanded here into
@@ -1293,12 +1293,14 @@ int enqueue_pass(rtfmm_fmm* f, bool adjoint = false, bool no_dipole = false, int
       // The image levels read the root's multipole and write image cells and
       // the root only, the 8x8 M2L reads cells below the root and writes
       // those: two branches between the tree's M2M and L2L.  The image branch
-      // is a chain of ten kernels of one or two rows each, worth hiding where
-      // the pass is short: 8192 bodies at P = 6 (FP64) 192 -> 174 us, 2^20 at
-      // P = 6, ncrit = 64 (3.4e6 target spectra) 2.67 -> 2.63 ms; 2^20 at
-      // P = 8, ncrit = 256 (4.6e6) 6.16 -> 6.21 ms, where P2P fills the chip
-      // while the image kernels run by themselves.
-      const bool fork = f->args.images > 0 && (int64_t)f->nT8 * Nf <= 4000000;
+      // is a chain of ten kernels of one or two rows each.  Beside the 8x8 M2L
+      // against after it, 126 plans (1000 to 2^21 bodies, P = 4 to 10, ncrit 32
+      // to 256, 1, 3 and 4 images): FP64 form 0.15 to 23% faster, all 63; mixed
+      // form below 2.6e6 target spectra up to 25% faster and at most 0.4%
+      // slower (52 plans), from 3.4e6 on between 1.5% faster and 4.2% slower
+      // (9.2e6 and 16.9e6 at P = 10, where P2P is short), which the number of
+      // spectra does not order: so there one after the other.
+      const bool fork = f->args.images > 0 && (!mixed || (int64_t)f->nT8 * Nf <= 3000000);
       cudaStream_t si = fork ? f->s2 : s0;
       if (fork) {
         CK(cudaEventRecord(f->ev_img0, s0));
@@ -1412,7 +1414,7 @@ int collect_times(rtfmm_fmm* f, float* total) {
 // single pass, as in a solve or a time step, is cheaper issued launch by
 // launch than captured and instantiated, by 0.3 ms for a solve of 1000
 // bodies) and replayed with one launch from then on (the launches, their
-// arguments and the two-stream fork/join are fixed by the plan; charges,
+// arguments and the fork and join of the streams are fixed by the plan; charges,
 // positions and outputs live in the handle's buffers).  Kernel nodes keep the
 // priority of the stream they were captured from, so the far-field chain still
 // preempts P2P.  Per-stage events are not recorded in a replay: the stage
