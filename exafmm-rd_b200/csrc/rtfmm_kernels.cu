@@ -14,8 +14,10 @@
 //   dipole_correction, scale_bodies, sort_bodies_by_idx
 //                         (kernel.cpp:1580-1596, body.cpp:88-96,177-190)  k_dipole_*, k_post
 //
-// Every index a kernel forms is checked against the extent of the buffer it
-// addresses; no kernel waits on another block.
+// Row, cell, body and slot indices come from the plan's tables, which the
+// set-up fills with values below the extents of the buffers it sizes by them;
+// thread indices are checked against the counts.  No kernel waits on another
+// block.
 #include "rtfmm_kernels.cuh"
 #include "rtfmm_rsqrt.cuh"
 
@@ -27,41 +29,11 @@
 
 #include <cub/cub.cuh>
 
-// FP32 Hadamard: targets per thread, directions per FP32 partial sum,
-// resident blocks per SM
-#ifndef HAD_TT
-#define HAD_TT 2
-#endif
-#ifndef HAD_DF
-#define HAD_DF 8
-#endif
-#ifndef HAD_MINB
-#define HAD_MINB 4
-#endif
-// FP32 Hadamard: FP64 accumulators in shared memory (1) or registers (0)
-#ifndef HAD_ACC_SMEM
-#define HAD_ACC_SMEM 1
-#endif
-// 8x8 source spectra in 32-byte chunks (1) or whole rows (0), q8_index; the
-// FP64 spectra too (Q8_CHUNKED64)
-#ifndef Q8_CHUNKED
-#define Q8_CHUNKED 1
-#endif
-#ifndef Q8_CHUNKED64
-#define Q8_CHUNKED64 1
-#endif
-// FP32 Hadamard: packed FP32x2 FMAs (1) or scalar FMAs (0)
-#ifndef HAD_F2
-#define HAD_F2 1
-#endif
-
 namespace rtfmm_b200 {
 
 // ---------------------------------------------------------------------------
 // small helpers
 // ---------------------------------------------------------------------------
-template <typename T> struct Cplx;
-template <> struct Cplx<float> { using type = float2; };
 // two complex values in one vector load
 template <typename T> struct Cplx2;
 template <> struct Cplx2<float> { using type = float4; };
@@ -76,9 +48,7 @@ template <> struct Cplx2<double> { using type = double4; };
 template <typename T>
 __host__ __device__ __forceinline__ size_t q8_index(size_t f, int src, int slot, int nsrc) {
   constexpr int per = 32 / (2 * sizeof(T)), nch = 8 / per;  // slots per chunk, chunks per row
-  if (Q8_CHUNKED && (sizeof(T) == 4 || Q8_CHUNKED64))
-    return ((f * nch + slot / per) * nsrc + src) * per + slot % per;
-  return (f * nsrc + src) * 8 + slot;
+  return ((f * nch + slot / per) * nsrc + src) * per + slot % per;
 }
 
 // 32-byte (one sector) vector loads, sm_100: one lane reads a whole sector.
@@ -568,10 +538,7 @@ __global__ void __launch_bounds__(32 * kP2PWarps, kP2PMinBlocks64)
 // minus it.  What remains of the FP32 term is its rounding inside the FP32
 // partial sum, ~2^-24 of the term.
 // ---------------------------------------------------------------------------
-#ifndef CLOSE_FRAC
-#define CLOSE_FRAC 0.125f
-#endif
-constexpr float kCloseFrac = CLOSE_FRAC;
+constexpr float kCloseFrac = 0.125f;
 
 // One warp per P2P work item, one lane per target (lanes >= nt idle); the
 // lanes of an item share its list, so source loads are warp broadcasts.
@@ -947,16 +914,13 @@ __global__ void __launch_bounds__(kGThreads) k_apply_f64_tc(ApplyBatch b) {
 // on a few SMs (the upper tree levels, the image levels with one row, small
 // body sets): a 64 x 64 tile alone takes ns/16 steps of 1024 tensor cycles on
 // one SM whatever its rows hold (5 us at ns = 152, 17 us at ns = 488), a
-// 16 x 32 tile a sixteenth of the cycles and a chain of ns/4 dependent mma.
+// 16 x 32 tile an eighth of the cycles and a chain of ns/4 dependent mma.
 // Each output sums its products in the same order as above, so the choice of
 // the tile does not change a result.
 constexpr int kSM = 16, kSN = 32, kSK = 32, kSStages = 4;
 constexpr int kSAPitch = kSK + 4, kSBPitch = kSN + 4;
 constexpr int kSAStage = kSM * kSAPitch, kSBStage = kSK * kSBPitch;
-#ifndef APPLY_SMALL
-#define APPLY_SMALL 296
-#endif
-constexpr int kApplySmallBelow = APPLY_SMALL;
+constexpr int kApplySmallBelow = 296;
 constexpr size_t kSSmem = sizeof(double) * kSStages * (kSAStage + kSBStage);
 
 __global__ void __launch_bounds__(128) k_apply_f64_small(ApplyBatch b) {
@@ -1490,102 +1454,52 @@ __global__ void __launch_bounds__(dft_threads(P), dft_blocks(P, sizeof(T)))
 // direction) reads one 64-byte source row with sector loads.  L1 wavefronts
 // per FMA fall as 1/(4 TT) + 1/16, which is what bounds this kernel.
 // FP32 partial sums over DF directions are accumulated into FP64.
-template <typename T> struct HadCfg;
-template <> struct HadCfg<float> {
-  static constexpr int TT = HAD_TT, DF = HAD_DF, THREADS = 256 / HAD_TT, MINB = HAD_MINB;
-  static constexpr bool ACC_SMEM = HAD_ACC_SMEM;
-};
+constexpr int kHadTT = 2, kHadDF = 8;
+constexpr int kHadThreads = 128, kHadBlocks = 4;  // resident blocks per SM
 
-template <typename T>
-__device__ __forceinline__ void load_row8(const T* qrow, typename Cplx<T>::type (&q)[8]) {
-  constexpr int kPer = 32 / sizeof(T);  // values per 32-byte sector
+// The source rows of this thread's targets, zero where there is none: chunk c
+// holds slots 4c .. 4c+3, one sector.
+__device__ __forceinline__ void had_rows(const float2* __restrict__ Qf, int nsrc, const int (&sd)[kHadTT],
+                                         float2 (&q)[kHadTT][8]) {
 #pragma unroll
-  for (int c = 0; c < 16 / kPer; ++c) {
-    T v[kPer];
-    ld_sector(qrow + c * kPer, v);
-#pragma unroll
-    for (int k = 0; k < kPer / 2; ++k) {
-      q[c * kPer / 2 + k].x = v[2 * k];
-      q[c * kPer / 2 + k].y = v[2 * k + 1];
-    }
-  }
-}
-
-template <typename T, int TT>
-__device__ __forceinline__ void had_rows(const typename Cplx<T>::type* __restrict__ Qf, int nsrc, const int (&sd)[TT],
-                                         typename Cplx<T>::type (&q)[TT][8]) {
-#pragma unroll
-  for (int u = 0; u < TT; ++u) {
+  for (int u = 0; u < kHadTT; ++u) {
     if (sd[u] >= 0) {
-      if constexpr (Q8_CHUNKED && (sizeof(T) == 4 || Q8_CHUNKED64)) {
-        // chunk c of this source: slots per*c .. per*c+per-1, one sector
-        constexpr int per = 32 / (2 * sizeof(T)), nch = 8 / per;
 #pragma unroll
-        for (int c = 0; c < nch; ++c) {
-          const T* qc = reinterpret_cast<const T*>(Qf) + ((size_t)c * nsrc + sd[u]) * 2 * per;
-          T v[2 * per];
-          ld_sector(qc, v);
+      for (int c = 0; c < 2; ++c) {
+        float v[8];
+        ld_sector(reinterpret_cast<const float*>(Qf) + ((size_t)c * nsrc + sd[u]) * 8, v);
 #pragma unroll
-          for (int k = 0; k < per; ++k) {
-            q[u][per * c + k].x = v[2 * k];
-            q[u][per * c + k].y = v[2 * k + 1];
-          }
-        }
-      } else {
-        load_row8<T>(reinterpret_cast<const T*>(Qf + (size_t)sd[u] * 8), q[u]);
+        for (int k = 0; k < 4; ++k) q[u][4 * c + k] = make_float2(v[2 * k], v[2 * k + 1]);
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) q[u][i].x = q[u][i].y = T(0);
+      for (int i = 0; i < 8; ++i) q[u][i] = make_float2(0.f, 0.f);
     }
   }
 }
 
-template <typename T, int TT>
-__device__ __forceinline__ void had_index(const int* __restrict__ tsrcT, int d, int t0, int nt, int ntar,
-                                          int (&sd)[TT]) {
+__device__ __forceinline__ void had_index(const int* __restrict__ tsrcT, int d, int t0, int ntar, int (&sd)[kHadTT]) {
 #pragma unroll
-  for (int u = 0; u < TT; ++u) {
-    const int t = t0 + u * nt;
+  for (int u = 0; u < kHadTT; ++u) {
+    const int t = t0 + u * kHadThreads;
     sd[u] = t < ntar ? tsrcT[d * ntar + t] : -1;
   }
 }
 
-template <typename T, int TT>
-__device__ __forceinline__ void had_mac(const typename Cplx<T>::type* __restrict__ g, const int (&sd)[TT],
-                                        const typename Cplx<T>::type (&q)[TT][8], T (&pr)[TT][8], T (&pi)[TT][8]) {
+// A direction's product in packed FP32x2 FMAs, the coefficients of an itar pair
+// laid (gr0, gr1, gi0, gi1) in shared memory; each output sums its FMAs in the
+// order of the sources.
+__device__ __forceinline__ void had_mac(const float4* __restrict__ g, const int (&sd)[kHadTT],
+                                        const float2 (&q)[kHadTT][8], float (&pr)[kHadTT][8], float (&pi)[kHadTT][8]) {
   bool any = false;
 #pragma unroll
-  for (int u = 0; u < TT; ++u) any |= sd[u] >= 0;
-  if (!any) return;
-#pragma unroll
-  for (int isrc = 0; isrc < 8; ++isrc)
-#pragma unroll
-    for (int itar = 0; itar < 8; itar += 2) {
-      const typename Cplx2<T>::type gv = *reinterpret_cast<const typename Cplx2<T>::type*>(g + isrc * 8 + itar);
-#pragma unroll
-      for (int u = 0; u < TT; ++u) {
-        cmad(pr[u][itar], pi[u][itar], gv.x, gv.y, q[u][isrc].x, q[u][isrc].y);
-        cmad(pr[u][itar + 1], pi[u][itar + 1], gv.z, gv.w, q[u][isrc].x, q[u][isrc].y);
-      }
-    }
-}
-
-// The same product in packed FP32x2 FMAs, with the coefficients of an itar
-// pair laid (gr0, gr1, gi0, gi1) in shared memory: per output the FMAs and
-// their order are those of cmad, so the sums are bit for bit the scalar ones.
-template <int TT>
-__device__ __forceinline__ void had_mac_f2(const float4* __restrict__ g, const int (&sd)[TT], const float2 (&q)[TT][8],
-                                           float (&pr)[TT][8], float (&pi)[TT][8]) {
-  bool any = false;
-#pragma unroll
-  for (int u = 0; u < TT; ++u) any |= sd[u] >= 0;
+  for (int u = 0; u < kHadTT; ++u) any |= sd[u] >= 0;
   if (!any) return;
 #pragma unroll
   for (int isrc = 0; isrc < 8; ++isrc) {
-    float2 qr[TT], qi[TT], nqi[TT];
+    float2 qr[kHadTT], qi[kHadTT], nqi[kHadTT];
 #pragma unroll
-    for (int u = 0; u < TT; ++u) {
+    for (int u = 0; u < kHadTT; ++u) {
       qr[u] = make_float2(q[u][isrc].x, q[u][isrc].x);
       qi[u] = make_float2(q[u][isrc].y, q[u][isrc].y);
       nqi[u] = make_float2(-q[u][isrc].y, -q[u][isrc].y);
@@ -1595,7 +1509,7 @@ __device__ __forceinline__ void had_mac_f2(const float4* __restrict__ g, const i
       const float4 gv = g[isrc * 4 + p];
       const float2 gr = make_float2(gv.x, gv.y), gi = make_float2(gv.z, gv.w);
 #pragma unroll
-      for (int u = 0; u < TT; ++u) {
+      for (int u = 0; u < kHadTT; ++u) {
         float2 re = make_float2(pr[u][2 * p], pr[u][2 * p + 1]);
         float2 im = make_float2(pi[u][2 * p], pi[u][2 * p + 1]);
         re = __ffma2_rn(gr, qr[u], re);
@@ -1611,100 +1525,77 @@ __device__ __forceinline__ void had_mac_f2(const float4* __restrict__ g, const i
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(HadCfg<T>::THREADS, HadCfg<T>::MINB)
-    k_m2l_hadamard8(const T* __restrict__ Q, const T* __restrict__ G, const int* __restrict__ tsrcT, int ntar,
-                    int nsrc, int Nf, T* __restrict__ Pk) {
-  using C2 = typename Cplx<T>::type;
-  constexpr int TT = HadCfg<T>::TT, DF = HadCfg<T>::DF, NT = HadCfg<T>::THREADS;
-  __shared__ __align__(32) C2 Gs[26 * 64];
+__global__ void __launch_bounds__(kHadThreads, kHadBlocks)
+    k_m2l_hadamard8(const float* __restrict__ Q, const float* __restrict__ G, const int* __restrict__ tsrcT, int ntar,
+                    int nsrc, float* __restrict__ Pk) {
+  constexpr int TT = kHadTT, NT = kHadThreads;
+  __shared__ __align__(32) float2 Gs[26 * 64];
   const int f = blockIdx.y;
-  const C2* Gf = reinterpret_cast<const C2*>(G) + (size_t)f * 26 * 64;
-  constexpr bool kF2 = HAD_F2 && sizeof(T) == 4;
-  if constexpr (kF2) {
-    // (gr, gi) of itar 2p, 2p+1 -> (gr0, gr1, gi0, gi1)
-    T* gs = reinterpret_cast<T*>(Gs);
-    for (int e = threadIdx.x; e < 26 * 64; e += NT) {
-      const int h = e & 1, b = (e & ~1) * 2;
-      const C2 v = Gf[e];
-      gs[b + h] = v.x;
-      gs[b + 2 + h] = v.y;
-    }
-  } else {
-    for (int e = threadIdx.x; e < 26 * 64; e += NT) Gs[e] = Gf[e];
+  const float2* Gf = reinterpret_cast<const float2*>(G) + (size_t)f * 26 * 64;
+  // (gr, gi) of itar 2p, 2p+1 -> (gr0, gr1, gi0, gi1)
+  float* gs = reinterpret_cast<float*>(Gs);
+  for (int e = threadIdx.x; e < 26 * 64; e += NT) {
+    const int h = e & 1, b = (e & ~1) * 2;
+    const float2 v = Gf[e];
+    gs[b + h] = v.x;
+    gs[b + 2 + h] = v.y;
   }
   // targets of this thread: t0 + u * NT, u < TT (coalesced tsrcT reads)
   const int t0 = blockIdx.x * NT * TT + threadIdx.x;
-  const C2* Qf = reinterpret_cast<const C2*>(Q) + (size_t)f * nsrc * 8;
+  const float2* Qf = reinterpret_cast<const float2*>(Q) + (size_t)f * nsrc * 8;
   // two-stage pipeline over directions: the source rows of direction d+1
   // are in flight while direction d is multiplied, and the row indices run
   // one direction further ahead
   int ia[TT], ib[TT];
-  C2 qa[TT][8], qb[TT][8];
+  float2 qa[TT][8], qb[TT][8];
   if (t0 < ntar) {
-    had_index<T, TT>(tsrcT, 0, t0, NT, ntar, ia);
-    had_rows<T, TT>(Qf, nsrc, ia, qa);
-    had_index<T, TT>(tsrcT, 1, t0, NT, ntar, ib);
+    had_index(tsrcT, 0, t0, ntar, ia);
+    had_rows(Qf, nsrc, ia, qa);
+    had_index(tsrcT, 1, t0, ntar, ib);
   }
   __syncthreads();
   if (t0 >= ntar) return;
-  T pr[TT][8], pi[TT][8];
+  float pr[TT][8], pi[TT][8];
 #pragma unroll
   for (int u = 0; u < TT; ++u)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) pr[u][i] = pi[u][i] = T(0);
-  // FP64 accumulators: registers, or one shared-memory column per thread
-  constexpr bool kAccS = HadCfg<T>::ACC_SMEM;
-  __shared__ double accs[kAccS ? TT * 16 : 1][NT];
-  double ar[TT][8], ai[TT][8];
+    for (int i = 0; i < 8; ++i) pr[u][i] = pi[u][i] = 0.f;
+  // FP64 accumulators: one shared-memory column per thread
+  __shared__ double accs[TT * 16][NT];
 #pragma unroll
   for (int u = 0; u < TT; ++u)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      if constexpr (kAccS) {
-        accs[u * 16 + 2 * i][threadIdx.x] = 0.0;
-        accs[u * 16 + 2 * i + 1][threadIdx.x] = 0.0;
-      } else {
-        ar[u][i] = ai[u][i] = 0.0;
-      }
+      accs[u * 16 + 2 * i][threadIdx.x] = 0.0;
+      accs[u * 16 + 2 * i + 1][threadIdx.x] = 0.0;
     }
   auto flush = [&]() {
 #pragma unroll
     for (int u = 0; u < TT; ++u)
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        if constexpr (kAccS) {
-          accs[u * 16 + 2 * i][threadIdx.x] += (double)pr[u][i];
-          accs[u * 16 + 2 * i + 1][threadIdx.x] += (double)pi[u][i];
-        } else {
-          ar[u][i] += (double)pr[u][i];
-          ai[u][i] += (double)pi[u][i];
-        }
-        pr[u][i] = pi[u][i] = T(0);
+        accs[u * 16 + 2 * i][threadIdx.x] += (double)pr[u][i];
+        accs[u * 16 + 2 * i + 1][threadIdx.x] += (double)pi[u][i];
+        pr[u][i] = pi[u][i] = 0.f;
       }
   };
-  auto MAC = [&](const C2* g, const int (&sd)[TT], const C2 (&q)[TT][8]) {
-    if constexpr (kF2) {
-      had_mac_f2<TT>(reinterpret_cast<const float4*>(g), sd, q, pr, pi);
-    } else {
-      had_mac<T, TT>(g, sd, q, pr, pi);
-    }
+  auto mac = [&](int d, const int (&sd)[TT], const float2 (&q)[TT][8]) {
+    had_mac(reinterpret_cast<const float4*>(Gs + d * 64), sd, q, pr, pi);
   };
   for (int d = 0; d < 26; d += 2) {
     int ja[TT];
-    had_rows<T, TT>(Qf, nsrc, ib, qb);
-    if (d + 2 < 26) had_index<T, TT>(tsrcT, d + 2, t0, NT, ntar, ja);
-    MAC(Gs + d * 64, ia, qa);
-    if (DF == 1 || (d + 1) % DF == 0) flush();
+    had_rows(Qf, nsrc, ib, qb);
+    if (d + 2 < 26) had_index(tsrcT, d + 2, t0, ntar, ja);
+    mac(d, ia, qa);
     if (d + 2 < 26) {
 #pragma unroll
       for (int u = 0; u < TT; ++u) ia[u] = ja[u];
-      had_rows<T, TT>(Qf, nsrc, ia, qa);
+      had_rows(Qf, nsrc, ia, qa);
     }
     int jb[TT];
-    if (d + 3 < 26) had_index<T, TT>(tsrcT, d + 3, t0, NT, ntar, jb);
-    MAC(Gs + (d + 1) * 64, ib, qb);
-    if ((d + 2) % DF == 0 || d + 2 == 26) flush();
+    if (d + 3 < 26) had_index(tsrcT, d + 3, t0, ntar, jb);
+    mac(d + 1, ib, qb);
+    if ((d + 2) % kHadDF == 0 || d + 2 == 26) flush();
     if (d + 3 < 26) {
 #pragma unroll
       for (int u = 0; u < TT; ++u) ib[u] = jb[u];
@@ -1714,19 +1605,10 @@ __global__ void __launch_bounds__(HadCfg<T>::THREADS, HadCfg<T>::MINB)
   for (int u = 0; u < TT; ++u) {
     const int t = t0 + u * NT;
     if (t >= ntar) break;
-    C2* out = reinterpret_cast<C2*>(Pk) + ((size_t)f * ntar + t) * 8;
+    float2* out = reinterpret_cast<float2*>(Pk) + ((size_t)f * ntar + t) * 8;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      C2 v;
-      if constexpr (kAccS) {
-        v.x = (T)accs[u * 16 + 2 * i][threadIdx.x];
-        v.y = (T)accs[u * 16 + 2 * i + 1][threadIdx.x];
-      } else {
-        v.x = (T)ar[u][i];
-        v.y = (T)ai[u][i];
-      }
-      out[i] = v;
-    }
+    for (int i = 0; i < 8; ++i)
+      out[i] = make_float2((float)accs[u * 16 + 2 * i][threadIdx.x], (float)accs[u * 16 + 2 * i + 1][threadIdx.x]);
   }
 }
 
@@ -2360,9 +2242,8 @@ cudaError_t launch_m2l_up(const double* q_equiv, const int* items, int nitems, c
 cudaError_t launch_m2l_hadamard8(const float* Q, const float* G, const int* tsrcT, int ntar, int nsrc, int Nf,
                                  float* Pk, cudaStream_t st) {
   if (ntar > 0) {
-    constexpr int NT = HadCfg<float>::THREADS, TT = HadCfg<float>::TT;
-    dim3 grid(cdiv(ntar, NT * TT), Nf);
-    k_m2l_hadamard8<float><<<grid, NT, 0, st>>>(Q, G, tsrcT, ntar, nsrc, Nf, Pk);
+    dim3 grid(cdiv(ntar, kHadThreads * kHadTT), Nf);
+    k_m2l_hadamard8<<<grid, kHadThreads, 0, st>>>(Q, G, tsrcT, ntar, nsrc, Pk);
   }
   return cudaGetLastError();
 }

@@ -34,9 +34,9 @@ struct P2PItem {
 // about an eighth of what each of 20 warps an SM (148 SMs) has to do, so that
 // no warp is left running alone for long, and at least 256 bodies, below which
 // a part's fixed cost shows.  Stage times: 150,001 bodies in blobs, FP64, 0.59
-// ms with halves, 0.51 with quarters, 0.47 with eighths, 0.45 with sixteenths
-// (which need twice the slots); 4 M bodies in blobs, mixed, 8.46, 8.37, 8.29,
-// 8.24 ms.  At least 64, 256, 1024 bodies: 30,011 bodies in blobs, mixed, 75,
+// ms with halves, 0.51 with quarters, 0.47 with eighths, 0.45 with sixteenths,
+// whose slots take 53 instead of 28 MB; 4 M bodies in blobs, mixed (across
+// entries), 8.46, 8.37, 8.29, 8.24 ms.  At least 64, 256, 1024 bodies: 30,011 bodies in blobs, mixed, 75,
 // 52.5, 52 us; 8192 bodies uniform, FP64, 23, 29, 47 us, where the far field's
 // chain of small kernels runs beside it and takes 150.
 #ifdef __CUDACC__
