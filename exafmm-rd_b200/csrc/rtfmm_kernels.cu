@@ -110,13 +110,15 @@ __global__ void k_body_leaf(const LeafInfo* __restrict__ leaves, int nleaf, int 
 // moved into it (x_t - offset, one rounding that all sources of the leaf
 // share, so that it cancels where their charges do; the offset added to each
 // source instead gave the potential of a lattice up to 1.4 times the error).
-// FP32 sums run over one long entry, or over 8 pairs of short ones (the
-// potential over 4) divided by the number of lane groups, and their two
-// halves go into FP64 each by itself.  Over 27 sets (uniform, blobs, lattices;
-// mean entries of 4-256 bodies) the error against FP64 is at most 1.01 times
-// that of sums over one entry each, 0.8-1.0 times for short ones; sums over 16
-// pairs across entries gave 1.0-1.9 times for the potential and up to 1.2
-// times for the gradient.
+// FP32 sums run over at most 64 bodies of one long entry, or over 8 pairs of
+// short ones (the potential over 4) divided by the number of lane groups, and
+// their two halves go into FP64 each by itself.  Over 27 sets (uniform, blobs,
+// lattices; mean entries of 4-256 bodies) the error against FP64 is at most
+// 1.01 times that of sums over one entry each, 0.4-0.8 times for entries of
+// 128 bodies and more; sums over 16 pairs across entries gave up to 1.9 times
+// for the potential and 1.2 times for the gradient.  Long entries summed
+// whole: 3.51 ms instead of 3.65 on leaves of 256 bodies (2^20); over 32
+// bodies 3.69.
 //
 // A clustered tree has leaves whose lists hold forty times the mean number of
 // bodies (a large leaf beside many small ones): such a list is cut into parts
@@ -128,9 +130,10 @@ __global__ void k_body_leaf(const LeafInfo* __restrict__ leaves, int nleaf, int 
 //
 // Measured, with one entry a tile and uncut lists -> here: 150001 bodies in
 // blobs (longest list 60593 bodies, mean 1435), FP64, 3.98 -> 0.47 ms; 30011 in
-// blobs, FP32, 0.36 -> 0.052; 10^6 in blobs, FP32, 12.8 -> 2.47; uniform 2^20,
-// FP32, ncrit = 32 1.36 -> 0.87, 64 0.68 and 0.68, 256 3.13 and 3.13, 512 3.58
-// and 3.58; FP64, ncrit = 256, 9.28 -> 7.68 (24 -> 18 FP64 operations a pair).
+// blobs, FP32, 0.36 -> 0.052; 10^6 in blobs, FP32, 11.4 -> 2.45; uniform 2^20,
+// FP32, ncrit = 32 1.36 -> 0.87, 64 0.68 and 0.70, 256 3.13 and 3.17, 512 3.58
+// and 3.65 (the whole pass 5.00 -> 4.96, P = 8); FP64, ncrit = 256, 9.28 -> 7.68
+// (24 -> 18 FP64 operations a pair).
 // FP32: bound by the register reads of the packed FMAs (3 cycles each measured,
 // 31 a pair of sources with the 2-cycle additions and products).  FP64: bound
 // by dependent operations (pipe 66% busy); 28 resident warps 7.68 ms, 20 7.94,
@@ -251,6 +254,14 @@ __device__ __forceinline__ void p2p32_run(const float4* __restrict__ s, int k0, 
 #pragma unroll kP2PUnroll
   for (int k = k0; k < npair; k += G) p2p32_pair2<MASK>(s, k, px, py, pz, p, fx, fy, fz);
 }
+// The same for a full tile of one entry that is not the target leaf: a constant
+// bound (3.65 against 3.71 ms on leaves of 256 bodies).
+template <int G>
+__device__ __forceinline__ void p2p32_full(const float4* __restrict__ s, int k0, float2 px, float2 py, float2 pz,
+                                           float2& p, float2& fx, float2& fy, float2& fz) {
+#pragma unroll kP2PUnroll
+  for (int u = 0; u < 16 / G; ++u) p2p32_pair2<false>(s, k0 + u * G, px, py, pz, p, fx, fy, fz);
+}
 // The same for a whole tile across entries, pair k of the entry with the
 // offset so[k]; FP32 sums over R pairs (the potential over RP), a lane group
 // over as many fewer as there are groups.
@@ -325,15 +336,19 @@ __device__ __forceinline__ void p2p32_item(const float4* __restrict__ body32, co
       if (cur.self)
         p2p32_run<G, true>(sw, grp, npair, make_float2(px, px), make_float2(py, py), make_float2(pz, pz), p, fx, fy,
                            fz);
+      else if (cnt == 32)
+        p2p32_full<G>(sw, grp, make_float2(px, px), make_float2(py, py), make_float2(pz, pz), p, fx, fy, fz);
       else
         p2p32_run<G, false>(sw, grp, npair, make_float2(px, px), make_float2(py, py), make_float2(pz, pz), p, fx, fy,
                             fz);
-      if (last) {
+      if (last || (c0 & 32)) {  // every 64 bodies, and at the entry's end
         P += (double)p.x + (double)p.y;
         Gx += (double)fx.x + (double)fx.y;
         Gy += (double)fy.x + (double)fy.y;
         Gz += (double)fz.x + (double)fz.y;
         p = fx = fy = fz = make_float2(0.f, 0.f);
+      }
+      if (last) {
         ++e;
         c0 = 0;
         cur = nxt;

@@ -54,7 +54,7 @@ inline int p2p_part_bodies(unsigned long long work) {
 // into FP64.  Stage times, entry by entry and across: mean 12.8 bodies (2^20
 // uniform) 1.48 and 0.87 ms, 15.6 (64,000 on a lattice) 0.049 and 0.046, 17.9
 // (100,003 uniform) 0.093 and 0.085, 24.4 0.073 and 0.081, 27.6 (150,001 in
-// blobs) 0.245 and 0.251, 32 (2^20) 0.70 and 0.76, 256 3.7 and 4.6.
+// blobs) 0.245 and 0.251, 32 (2^20) 0.70 and 0.76, 256 3.65 and 4.6.
 #ifdef __CUDACC__
 __host__ __device__
 #endif
