@@ -136,7 +136,7 @@ __global__ void k_body_leaf(const LeafInfo* __restrict__ leaves, int nleaf, int 
 // (24 -> 18 FP64 operations a pair).
 // FP32: bound by the register reads of the packed FMAs (3 cycles each measured,
 // 31 a pair of sources with the 2-cycle additions and products).  FP64: bound
-// by dependent operations (pipe 66% busy); 28 resident warps 7.68 ms, 20 7.94,
+// by dependent operations (pipe 71% busy); 28 resident warps 7.68 ms, 20 7.94,
 // 24 8.04, 32 7.76.
 // ---------------------------------------------------------------------------
 // A block is one warp: work items differ in cost several-fold, and a block of
